@@ -12,7 +12,9 @@
 // After all azimuths of a slice, dose_bev[s] += sum_phi dose / (sum_p_lastphi + 1e-4)
 // (Q2: the path sum of the last azimuth only).
 //
-// B200 design.  The reference runs one block per beamlet with one thread per
+// B200 design.  (Batches of 8 x 8, 12 x 12 and 16 x 16 maps take the
+// voxel-stationary march further down; this paragraph is about the instances
+// for the other maps.)  The reference runs one block per beamlet with one thread per
 // pixel and a block barrier after every ray step, azimuths in sequence.  Here a
 // block owns one beamlet (schedule 0: all zenith bins in turn) or one
 // (beamlet, zenith bin) (schedule 1), and each WARP owns one azimuth: its 32
@@ -43,11 +45,7 @@ namespace fd2 {
 namespace {
 
 constexpr int kStepCap = 1 << 20;  // per-slice step cap (the watchdog bound)
-// The 16x16 march is compiled for at most 8 azimuth warps, with the register
-// budget of 3 such blocks of 256 threads per SM: 80 registers, 4 blocks of
-// 192 threads (6 azimuths).  On the 4pi plan that measured faster than 48,
-// 64, 72, 96 and 126 registers (7, 5, 4, 3 and 2 blocks of 192).
-constexpr int kFx16Threads = 256;
+constexpr int kMapThreads = 256;   // the common-map instances are compiled for at most 8 azimuth warps
 
 struct RayGeom {  // per-beamlet scalars the march needs
     float hx, hy;      // fmap_size / 2
@@ -137,21 +135,6 @@ __device__ __forceinline__ bool crosses_edge(float b, float n, float ff) {
     return floorf(__fdividef(b, ff)) != floorf(__fdividef(n, ff));
 }
 
-// The same two operations for a 16-pixel map axis.  Division by 16 is exact
-// (the fast reciprocal of a power of two is exact), so b / 16 is b * 0.0625; the
-// remainder m - 16*trunc(m/16) is exact by Sterbenz's lemma and equals fmodf.
-__device__ __forceinline__ int mid_index16(float b, float n) {
-    const float m = __fmul_rn(__fadd_rn(b, n), 0.5f);
-    float r = __fsub_rn(m, __fmul_rn(16.0f, truncf(__fmul_rn(m, 0.0625f))));
-    r = r < 0.0f ? __fadd_rn(r, 16.0f) : r;
-    const int i = __float2int_rd(r);
-    return i < 16 ? i : 15;
-}
-
-__device__ __forceinline__ bool crosses16(float b, float n) {
-    return floorf(__fmul_rn(b, 0.0625f)) != floorf(__fmul_rn(n, 0.0625f));
-}
-
 // 4 bytes from global to shared memory without passing through registers
 // (PTX cp.async), committed as one group per call site; and the wait for all
 // of this thread's groups.
@@ -173,25 +156,23 @@ __device__ __forceinline__ float exp2_sfu(float x) {
 
 // Segment length sqrt(l2) as l2 * rsqrt(l2) with the SFU reciprocal square
 // root (PTX rsqrt.approx.ftz.f32); l2 > 0 for every segment the march takes.
-__device__ __forceinline__ float seg_length(float l2) {
+__device__ __forceinline__ float rsqrt_sfu(float x) {
     float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(l2));
-    return l2 * r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
+__device__ __forceinline__ float seg_length(float l2) { return l2 * rsqrt_sfu(l2); }
 
 // Block: n_phi warps.  Dynamic shared memory: float2 tr[P] (Terma, density of
 // the current slice) followed by float2 dp[n_phi][P] (per-azimuth dose and path
-// sums); for kFx16 instead float4 wb[n_phi][P] (each azimuth's copy of the
-// slice beside its sums) followed by float2 ytab[n_phi][16] (row tables).
-// RPL = rays per lane (P <= 32 * RPL); kFx16: the map is 16 x 16.
+// sums).  RPL = rays per lane (P <= 32 * RPL).
 // kCols: every map of the batch is F x F with F <= 32 -- each lane owns one
 // column (lane % F) and the rows lane / F + k j (k = 32 / F lanes per column),
 // so the x half of the voxel work is done once per lane and the y half once per
-// row and shared by shuffles (16 x 16 maps share it through the row table);
-// RPL >= ceil(F / k).
-template <int RPL, bool kFx16, bool kCols = false, bool kTab = false>
-__global__ void __launch_bounds__(kFx16 || kCols || kTab ? kFx16Threads : 768,
-                                  kFx16 ? 3 : ((kCols || kTab) && RPL <= 8 ? 4 : (kCols || kTab ? 3 : 1)))
+// row and shared by shuffles; RPL >= ceil(F / k).
+template <int RPL, bool kCols = false, bool kTab = false>
+__global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
+                                  (kCols || kTab) && RPL <= 8 ? 4 : (kCols || kTab ? 3 : 1))
     cccs_kernel(const fd2_beam_t* __restrict__ beams,
                                                    const float* const* __restrict__ terma,
                                                    const float* const* __restrict__ dens,
@@ -242,12 +223,6 @@ __global__ void __launch_bounds__(kFx16 || kCols || kTab ? kFx16Threads : 768,
     float2* dp = smem + g.P;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float2* mydp = dp + (size_t)warp * g.P;
-    // kFx16: every azimuth warp keeps its own copy of the slice beside its sums,
-    // wb[warp][v] = {Terma, density, dose, path sum}, so a ray step reads all
-    // four with one 16-byte load; behind them, each warp's 16-entry row table.
-    float4* wb = reinterpret_cast<float4*>(smem);
-    float4* mywb = wb + (size_t)warp * g.P;
-    float2* ytab = reinterpret_cast<float2*>(wb + (size_t)n_phi * g.P) + 16 * warp;
     const float* __restrict__ T = terma[bi];
     const float* __restrict__ R = dens[bi];
     float* __restrict__ D = dose[bi];
@@ -255,7 +230,7 @@ __global__ void __launch_bounds__(kFx16 || kCols || kTab ? kFx16Threads : 768,
     // per-ray constant pixel coordinates
     float fix[RPL], fiy[RPL];
     bool act[RPL];
-    if constexpr (!kFx16 && !kCols) {
+    if constexpr (!kCols) {
 #pragma unroll
         for (int j = 0; j < RPL; j++) {
             int r = j * 32 + lane;
@@ -275,7 +250,7 @@ __global__ void __launch_bounds__(kFx16 || kCols || kTab ? kFx16Threads : 768,
     // pass), copied by cp.async into s_stage (Terma, then density) during the
     // march and used only if that slice is the one taken.  Each thread copies
     // and later reads the same pixels, so no barrier stands between the two.
-    constexpr int kStageP = kFx16 ? 256 : 1024;
+    constexpr int kStageP = 1024;
     __shared__ float s_stage[2 * kStageP];
     int st_s = -1;
 
@@ -299,22 +274,11 @@ __global__ void __launch_bounds__(kFx16 || kCols || kTab ? kFx16Threads : 768,
         __syncthreads();  // the previous pass has finished; s_next is visible
         int s = *s_next;
         while (s < g.L) {
-            if constexpr (kFx16) {
-                // each pixel's pair goes to every azimuth's copy, sums cleared
-                cp_async_wait_all();  // this thread's staged pixels have landed
-                for (int v = threadIdx.x; v < g.P; v += blockDim.x) {
-                    const float2 t = s == st_s ? make_float2(s_stage[v], s_stage[kStageP + v])
-                                               : make_float2(__ldg(T + (size_t)s * pitch + v),
-                                                             __ldg(R + (size_t)s * pitch + v));
-                    for (int w = 0; w < n_phi; w++) wb[(size_t)w * g.P + v] = make_float4(t.x, t.y, 0.0f, 0.0f);
-                }
-            } else {
-                cp_async_wait_all();  // this thread's staged pixels have landed
-                for (int v = threadIdx.x; v < g.P; v += blockDim.x)
-                    tr[v] = s == st_s ? make_float2(s_stage[v], s_stage[kStageP + v])
-                                      : make_float2(__ldg(T + (size_t)s * pitch + v), __ldg(R + (size_t)s * pitch + v));
-                for (int v = lane; v < g.P; v += 32) mydp[v] = make_float2(0.0f, 0.0f);
-            }
+            cp_async_wait_all();  // this thread's staged pixels have landed
+            for (int v = threadIdx.x; v < g.P; v += blockDim.x)
+                tr[v] = s == st_s ? make_float2(s_stage[v], s_stage[kStageP + v])
+                                  : make_float2(__ldg(T + (size_t)s * pitch + v), __ldg(R + (size_t)s * pitch + v));
+            for (int v = lane; v < g.P; v += 32) mydp[v] = make_float2(0.0f, 0.0f);
             __syncthreads();
             st_s = s + 1 < g.L ? s + 1 : (t + 1 < t1 ? 0 : -1);
             if (st_s >= 0)
@@ -330,56 +294,7 @@ __global__ void __launch_bounds__(kFx16 || kCols || kTab ? kFx16Threads : 768,
                 const bool flag = next_point(c, cd, np);
                 const float fe = (np.z * g.ls + g.lim_min) * g.inv_sad;
                 const float dzp = (np.z - c.z) * g.ls;
-                if constexpr (kFx16) {
-                    // 16x16 map.  A lane's rays share their column, and the rays of
-                    // one row share their row: the voxel/edge/length work splits into
-                    // an x half per column and a y half per row, 16 of each per step.
-                    // Lanes 0-15 evaluate the x half of column `lane`, lanes 16-31 the
-                    // y half of row `lane - 16`, in the same instructions (the same
-                    // operations on the same inputs as a per-ray evaluation, done once
-                    // per column or row instead of per ray).  The half's edge
-                    // crossing travels as the sign bit of its |offset|, which enters
-                    // the length only squared.  Rows go to the warp's row table
-                    // {+-|dy|, 256 * row} (bytes into the slice copy), rows of one
-                    // parity together, so a lane reads its eight rows (of its parity)
-                    // with four 16-byte loads; lanes 16-31 take their column's x half
-                    // from lanes 0-15 by shuffle.
-                    const float lx = (float)(lane & 15);
-                    const bool yl = lane >= 16;
-                    const float hb = __fadd_rn(yl ? c.y : c.x, lx), hn = __fadd_rn(yl ? np.y : np.x, lx);
-                    const float bs = yl ? g.bsy : g.bsx;
-                    const int hi = mid_index16(hb, hn);
-                    const float hq = fabsf((hn - 8.0f) * bs * fe - (hb - 8.0f) * bs * fs);
-                    const float hs = crosses16(hb, hn) ? -hq : hq;
-                    if (yl) ytab[(lane & 1) * 8 + ((lane & 15) >> 1)] = make_float2(hs, __int_as_float(hi << 8));
-                    const int cx = __shfl_sync(0xffffffffu, hi, lane & 15);
-                    const float dxs = __shfl_sync(0xffffffffu, hs, lane & 15);
-                    const float dxz2 = dxs * dxs + dzp * dzp;
-                    const int wx = __float_as_int(dxs);
-                    const char* col = reinterpret_cast<const char*>(mywb) + (cx << 4);
-                    __syncwarp();
-                    const float4* yrow = reinterpret_cast<const float4*>(ytab) + 4 * (lane >> 4);
-                    // ray j of this lane: row (lane >> 4) + 2 j
-                    auto ray = [&](int j, float dys, int yoff) {
-                        const bool wrap = (__float_as_int(dys) | wx) < 0;
-                        const float l2 = dxz2 + dys * dys;
-                        const float len = seg_length(l2);
-                        float4* v = const_cast<float4*>(reinterpret_cast<const float4*>(col + yoff));
-                        const float4 e = *v;  // Terma, density, dose, path sum
-                        const float p = len * e.y;
-                        const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
-                        const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
-                        *reinterpret_cast<float2*>(&v->z) = make_float2(e.z + dep, e.w + p);
-                        XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - e.x, e.x);
-                        XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - e.x, e.x);
-                    };
-#pragma unroll
-                    for (int q = 0; q < RPL / 2; q++) {
-                        const float4 y2 = yrow[q];
-                        ray(2 * q, y2.x, __float_as_int(y2.y));
-                        ray(2 * q + 1, y2.z, __float_as_int(y2.w));
-                    }
-                } else if constexpr (kCols) {
+                if constexpr (kCols) {
                     const float btx = __fadd_rn(c.x, fcol), ntx = __fadd_rn(np.x, fcol);
                     const int cx = mid_index(btx, ntx, g.ffx, g.fx);
                     const bool wrapx = crosses_edge(btx, ntx, g.ffx);
@@ -506,13 +421,8 @@ __global__ void __launch_bounds__(kFx16 || kCols || kTab ? kFx16Threads : 768,
             // reduce azimuths in order; normalise by the last azimuth's path sum
             for (int v = threadIdx.x; v < g.P; v += blockDim.x) {
                 float sum = 0.0f, last_sum_p;
-                if constexpr (kFx16) {
-                    for (int w = 0; w < n_phi; w++) sum += wb[(size_t)w * g.P + v].z;
-                    last_sum_p = wb[(size_t)(n_phi - 1) * g.P + v].w;
-                } else {
-                    for (int w = 0; w < n_phi; w++) sum += dp[(size_t)w * g.P + v].x;
-                    last_sum_p = dp[(size_t)(n_phi - 1) * g.P + v].y;
-                }
+                for (int w = 0; w < n_phi; w++) sum += dp[(size_t)w * g.P + v].x;
+                last_sum_p = dp[(size_t)(n_phi - 1) * g.P + v].y;
                 const float val = sum / (last_sum_p + 1e-4f);
                 if (split)
                     split_out[(size_t)blockIdx.x * split_stride + (size_t)s * g.P + v] = val;
@@ -546,68 +456,656 @@ __global__ void cccs_split_reduce(const fd2_beam_t* __restrict__ beams, float* c
     }
 }
 
-template <int RPL, bool kFx16, bool kCols, bool kTab = false>
+// ---------------------------------------------------------------------------
+// The voxel-stationary march of common square maps (F x F, F = G * R).
+//
+// Within one step every ray of an azimuth moves by the same whole number of
+// voxels, so the map as seen by the rays is a cyclic shift of the map of
+// voxels.  A lane therefore keeps its VOXELS in registers for a whole slice --
+// lane v + F g holds column v, rows R g .. R g + R - 1: Terma, density and the
+// dose sum -- and the ray states (XA, XB) move instead: a step that enters the
+// next column rotates them by one lane (shuffles), one that enters the next row
+// by one register.  A ray step then touches no memory, and the rows of a lane
+// pair up in the packed FP32 instructions of sm_100 (fma/mul/add.rn.f32x2),
+// which take one issue slot for two rays.
+//
+// What all rays of an azimuth share does not depend on the slice data: the base
+// ray's points and when the shift changes.  One warp computes these path
+// records for all azimuths, one azimuth per lane, into shared memory: the step
+// chain of next_point is issued once per block instead of once per azimuth
+// warp, and it runs while the other warps reduce the previous slice.  Two
+// barriers per slice.
+//
+// The lateral offset and the edge crossing of a column or row are the
+// reference's own roundings, evaluated once per column and row (only the rays on
+// the first and last column and row can cross an edge).  Where rounding
+// could put a ray's segment midpoint into the neighbour of the voxel the shift
+// gives it (a midpoint within some 1e-5 of a boundary), or a segment spans
+// several voxels, the record asks for march_exact_step, which evaluates every
+// ray's voxel and crossing as the reference does (about 0.1 % of the steps).
+//
+// Bound: instruction issue, and the slowest azimuth of each slice at the
+// barrier.  CCCS time on one B200 against the march that kept the rays in place
+// and the slice in shared memory: 100-beam torso plan, 15 070 beamlets of
+// 16 x 16: 332 ms (356.9); one beam of 100 beamlets on the 64^3 slab: 1.53 ms
+// (2.15); 360 beamlets of 12 x 12, 4 azimuths: 3.3 ms (5.4); of 8 x 8, 8
+// azimuths: 2.5 ms (3.6).  Measured slower: the last azimuth's path sums in
+// shared memory instead of registers (366 ms; every slice waits for that warp),
+// a warp of its own for the paths with one barrier a slice (356 ms at 72
+// registers and 4 blocks), the edge crossings in the path records (longer
+// chain in the one warp that the others wait for).
+// ---------------------------------------------------------------------------
+constexpr int kMarchWarps = 8;   // azimuths a block may have
+constexpr int kMarchSteps = 40;  // path records of an azimuth per round; a slice with more takes several rounds
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer in the add's rounding mode
+
+// Two floats in one 64-bit register pair, and the packed operations on them.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pk(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 up(F2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// floor, ceil and round of |x| < 2^22 as adds of kMagic in the directed
+// rounding mode (FMA pipe) instead of conversions (special-function pipe).
+__device__ __forceinline__ float floor_biased(float x) { return __fadd_rd(x, kMagic); }
+__device__ __forceinline__ int biased_int(float b) { return __float_as_int(b) - __float_as_int(kMagic); }
+__device__ __forceinline__ float round_biased(float x) { return __fsub_rn(__fadd_rn(x, kMagic), kMagic); }
+
+// step_to_boundary and next_point with the roundings as biased adds: the same
+// floats for |c| < 2^22 (Reach::admits bounds the path).
+__device__ __forceinline__ float step_to_boundary_biased(float c, float s, float ra) {
+    const float up = __fsub_rn(__fadd_ru(__fmaf_rn(c, s, 1e-3f), kMagic), kMagic);
+    return __fmul_rn(__fmaf_rn(-c, s, up), ra);
+}
+__device__ __forceinline__ bool next_point_biased(float3 c, const ConeDir& k, float3& np) {
+    const float3 d = k.d;
+    const float sx = step_to_boundary_biased(c.x, k.sg.x, k.ra.x), sy = step_to_boundary_biased(c.y, k.sg.y, k.ra.y),
+                sz = step_to_boundary_biased(c.z, k.sg.z, k.ra.z);
+    const float take = fminf(fminf(sx, sy), sz);
+    np = make_float3(__fmaf_rn(take, d.x, c.x), __fmaf_rn(take, d.y, c.y), __fmaf_rn(take, d.z, c.z));
+    // (a tie rounds to even here and away from zero in roundf; the test's 1e-4 is far from a tie)
+    const bool flag = fabsf(__fsub_rn(np.z, round_biased(np.z))) < 1e-4f;
+    if (flag)
+        np = make_float3(__fmaf_rn(sz, d.x, c.x), __fmaf_rn(sz, d.y, c.y), round_biased(__fmaf_rn(sz, d.z, c.z)));
+    return flag;
+}
+
+// Bits of a path record's code.
+enum : int {
+    kRecEnd = 1,                      // the step ends the slice
+    kRecExact = 2,                    // march_exact_step
+    kRecMoveX = 4, kRecMoveY = 8,     // the shift changed by one column / row before this step
+};
+
+// Shared memory of a march block.  A map's cell (column v, row r) is at
+// v * S + r: a lane's rows are consecutive, and with S = F + 4 (F a multiple of
+// 8) eight neighbouring lanes' 16-byte accesses hit distinct banks.
+template <int F>
+struct MarchShared {
+    static constexpr int S = F + 4;
+    float4 rec[kMarchWarps][kMarchSteps];  // next point x, y; divergence factor there; (depth of the step)^2
+    int code[kMarchWarps][kMarchSteps];
+    alignas(16) float T[2][F * S];         // this slice and the one staged behind it
+    alignas(16) float R[2][F * S];
+    alignas(16) float dose[kMarchWarps][F * S];  // each azimuth's sums of the slice
+    alignas(16) float path[F * S];               // the last azimuth's path sums
+    alignas(16) float xa[kMarchWarps][F * S], xb[kMarchWarps][F * S];  // ray states in march_exact_step
+    alignas(16) float row[kMarchWarps][2][F];    // the step's lateral offset of each row
+    float3 c[kMarchWarps];                 // chain state: point, voxel shift,
+    int2 k[kMarchWarps];
+    ConeDir dir[kMarchWarps];              // direction,
+    int count[kMarchWarps];                // records of this round,
+    int next, more, abort;                 // next slice; some azimuth has more rounds; step cap hit
+};
+
+// Per-beamlet and per-pass values of a march.
+struct MarchRay {
+    float bsx, bsy, ls, lim_min, inv_sad;
+    float ka, kb, Aa, Bb;
+};
+
+__device__ __forceinline__ int pos_mod(int a, int f) {
+    const int r = a % f;
+    return r < 0 ? r + f : r;
+}
+
+// One axis of a path record: the voxel shift of the segment c..n, and whether
+// the shift may not hold for every ray.
+template <int F>
+__device__ __forceinline__ int path_axis(float c, float n, bool& exact) {
+    const float m = __fmul_rn(__fadd_rn(c, n), 0.5f);
+    const float fl = floor_biased(m);
+    // a ray's midpoint differs from the base ray's by at most 1.2e-7 of its
+    // coordinate, and the remainder by F rounds by at most 2e-6 more
+    const float eps = 4e-6f + 3e-7f * (fabsf(c) + F);
+    exact = exact || fabsf(m - __fsub_rn(fl, kMagic) - 0.5f) > 0.5f - eps || fabsf(n - c) > 1.5f;
+    return biased_int(fl);
+}
+
+// One round of every azimuth's path (lane = azimuth) from the chain state in
+// shared memory.  `open`: the lane's slice is not finished.
+template <int F>
+__device__ __forceinline__ void march_paths(MarchShared<F>& sm, const MarchRay& g, int n_phi, int s, int L, bool open) {
+    const int w = threadIdx.x & 31;
+    int n = 0;
+    if (w < n_phi && open) {
+        float3 c = sm.c[w];
+        int2 k0 = sm.k[w];
+        const ConeDir k = sm.dir[w];
+        bool flag = false;
+        while (!flag && n < kMarchSteps) {
+            float3 np;
+            flag = next_point_biased(c, k, np);
+            bool exact = false;
+            const int kx = path_axis<F>(c.x, np.x, exact), ky = path_axis<F>(c.y, np.y, exact);
+            exact = exact || abs(kx - k0.x) > 1 || abs(ky - k0.y) > 1;
+            const float fe = (np.z * g.ls + g.lim_min) * g.inv_sad;
+            const float dz = (np.z - c.z) * g.ls;
+            sm.rec[w][n] = make_float4(np.x, np.y, fe, dz * dz);
+            sm.code[w][n++] = (flag ? kRecEnd : 0) | (exact ? kRecExact : 0) | (kx != k0.x ? kRecMoveX : 0) |
+                              (ky != k0.y ? kRecMoveY : 0);
+            c = np;
+            k0 = make_int2(kx, ky);
+        }
+        sm.k[w] = k0;
+        sm.c[w] = c;
+        open = !flag;
+        if (w == 0 && flag) {
+            // the first azimuth's plane after this slice; it always lies ahead
+            const int nxt = (int)roundf(c.z);
+            sm.next = nxt > s ? nxt : L;
+        }
+    }
+    if (w < n_phi) sm.count[w] = n;
+    const bool more = __any_sync(0xffffffffu, w < n_phi && open);
+    if (w == 0) sm.more = more;
+}
+
+// A step in which some ray's voxel may not be the shifted one: every ray's
+// voxel and edge crossing as the reference computes them, from b to n.  The
+// warp's states and sums are in shared memory, each at its voxel: the states
+// come in at the old shift (ox, oy), taken modulo F, and leave at the new one,
+// which is returned.  Rays of one step can only meet in a voxel next to their
+// own, so four passes, one per parity of column and row, keep the additions
+// apart and their order fixed.
+template <int F, int G, int R>
+__device__ __noinline__ int2 march_exact_step(MarchShared<F>& sm, int buf, const MarchRay& g, float2 b, float2 n,
+                                              float fs, float fe, float dz2, int ox, int oy, bool last) {
+    constexpr int S = MarchShared<F>::S;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = lane % F, grp = lane / F;
+    const bool on = grp < G;
+    const float ff = (float)F, hh = 0.5f * F;
+    const int kx = pos_mod(biased_int(floor_biased(__fmul_rn(__fadd_rn(b.x, n.x), 0.5f))), F);
+    const int ky = pos_mod(biased_int(floor_biased(__fmul_rn(__fadd_rn(b.y, n.y), 0.5f))), F);
+    const int lx = pos_mod(v - kx, F);
+    const float bx = __fadd_rn(b.x, (float)lx), nx = __fadd_rn(n.x, (float)lx);
+    const int ix = mid_index(bx, nx, ff, F);
+    const bool wx = crosses_edge(bx, nx, ff);
+    const float dx = (nx - hh) * g.bsx * fe - (bx - hh) * g.bsx * fs;
+    const float dxz2 = dx * dx + dz2;
+    float *dose = sm.dose[warp], *xa = sm.xa[warp], *xb = sm.xb[warp];
+    float XA[R], XB[R];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const int from = pos_mod(lx + ox, F) * S + pos_mod(grp * R + j - ky + oy, F);
+        XA[j] = on ? xa[from] : 0.0f;
+        XB[j] = on ? xb[from] : 0.0f;
+    }
+    __syncwarp();
+    for (int pass = 0; pass < 4; pass++) {
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const int row = grp * R + j;
+            if (on && pass == ((v & 1) | (row & 1) << 1)) {
+                const int ly = pos_mod(row - ky, F);
+                const float by = __fadd_rn(b.y, (float)ly), ny = __fadd_rn(n.y, (float)ly);
+                const int q = ix * S + mid_index(by, ny, ff, F);
+                const float dy = (ny - hh) * g.bsy * fe - (by - hh) * g.bsy * fs;
+                const float p = seg_length(dxz2 + dy * dy) * sm.R[buf][q];
+                const float t = sm.T[buf][q];
+                dose[q] = __fmaf_rn(g.Aa * XA[j] + g.Bb * XB[j], p, dose[q]);
+                if (last) sm.path[q] += p;
+                const bool wrap = wx || crosses_edge(by, ny, ff);
+                xa[v * S + row] = wrap ? 0.0f : __fmaf_rn(exp2_sfu(g.ka * p), XA[j] - t, t);
+                xb[v * S + row] = wrap ? 0.0f : __fmaf_rn(exp2_sfu(g.kb * p), XB[j] - t, t);
+            }
+        }
+        __syncwarp();
+    }
+    return make_int2(kx, ky);
+}
+
+// A lane's R consecutive cells to and from shared memory, in pairs.
+template <int R>
+__device__ __forceinline__ void load_cells(const float* p, F2 (&o)[R / 2]) {
+    if constexpr (R % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < R / 2; q += 2) {
+            const float4 a = *reinterpret_cast<const float4*>(p + 2 * q);
+            o[q] = pk(a.x, a.y);
+            o[q + 1] = pk(a.z, a.w);
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < R / 2; q++) {
+            const float2 a = *reinterpret_cast<const float2*>(p + 2 * q);
+            o[q] = pk(a.x, a.y);
+        }
+    }
+}
+template <int R>
+__device__ __forceinline__ void store_cells(float* p, const F2 (&o)[R / 2]) {
+    if constexpr (R % 4 == 0) {
+#pragma unroll
+        for (int q = 0; q < R / 2; q += 2)
+            *reinterpret_cast<float4*>(p + 2 * q) = make_float4(up(o[q]).x, up(o[q]).y, up(o[q + 1]).x, up(o[q + 1]).y);
+    } else {
+#pragma unroll
+        for (int q = 0; q < R / 2; q++) *reinterpret_cast<float2*>(p + 2 * q) = up(o[q]);
+    }
+}
+
+// 80 registers: four blocks of 6 azimuths an SM.
+template <int F, int G, int R>
+__global__ void __launch_bounds__(32 * kMarchWarps, 3)
+    cccs_march_kernel(const fd2_beam_t* __restrict__ beams, const float* const* __restrict__ terma,
+                      const float* const* __restrict__ dens, float* const* __restrict__ dose,
+                      const float4* __restrict__ dirs,  // [beam][n_tf][n_phi]
+                      ConeParams cp, int split, float* __restrict__ split_out, size_t split_stride, DeviceStatus* status,
+                      const int* __restrict__ order) {
+    static_assert(F == G * R && G > 1 && R % 2 == 0 && F * G <= 32, "a lane holds R rows of a column in pairs");
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int P = F * F, S = MarchShared<F>::S;
+    __shared__ MarchShared<F> sm;
+    const int n_tf = cp.n_theta_fwd, n_phi = cp.n_phi;
+    // split: one block per (zenith bin, beamlet), the widest bin (most steps per
+    // slice) first; else one block per beamlet in `order` (longest first)
+    const int nb = gridDim.x / n_tf;
+    const int bi = split ? blockIdx.x % nb : (order ? order[blockIdx.x] : blockIdx.x);
+    const int t0 = split ? n_tf - 1 - blockIdx.x / nb : 0;
+    const int t1 = split ? t0 + 1 : n_tf;
+    const fd2_beam_t& bm = beams[bi];
+    const int L = (int)bm.long_dim;
+    const size_t pitch = bm.TermaBEV_pitch / sizeof(float);
+    const float* __restrict__ T = terma[bi];
+    const float* __restrict__ Rho = dens[bi];
+    float* __restrict__ D = dose[bi];
+    MarchRay g;
+    g.bsx = bm.beamlet_size[0];
+    g.bsy = bm.beamlet_size[1];
+    g.ls = bm.long_spacing;
+    g.lim_min = bm.lim_min;
+    g.inv_sad = 1.0f / bm.sad;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int v = lane % F, grp = lane / F;
+    const bool on = grp < G, last = warp == n_phi - 1;
+    const bool yl = grp == 1;  // group 0 evaluates the columns' offsets, group 1 the rows'
+    const int cell = (v * S + (on ? grp * R : 0));
+    if (threadIdx.x == 0) sm.abort = 0;
+    if (L <= 0) return;
+
+    // thread i of the block copies pixels i, i + blockDim, ... of a slice
+    auto stage = [&](int s, int buf) {
+        for (int i = threadIdx.x; i < P; i += blockDim.x) {
+            const int q = i % F * S + i / F;
+            cp_async4(&sm.T[buf][q], T + (size_t)s * pitch + i);
+            cp_async4(&sm.R[buf][q], Rho + (size_t)s * pitch + i);
+        }
+        cp_async_commit();
+    };
+    // the azimuths of slice s in order, normalised by the last one's path sum;
+    // done by the warps that compute no path (the first does)
+    const int rt0 = n_phi > 1 ? 32 : 0;
+    auto reduce = [&](int t, int s) {
+        for (int i = threadIdx.x - rt0; i < P; i += blockDim.x - rt0) {
+            const int q = i % F * S + i / F;
+            float sum = 0.0f;
+            for (int w = 0; w < n_phi; w++) sum += sm.dose[w][q];
+            const float val = sum / (sm.path[q] + 1e-4f);
+            if (split)
+                split_out[((size_t)bi * n_tf + t) * split_stride + (size_t)s * P + i] = val;
+            else
+                // this block alone owns beam bi's dose and each (s, i) stays with
+                // one thread, so a fire-and-forget add gives D + val in pass order
+                // without waiting for D's old value
+                atomicAdd(D + (size_t)s * pitch + i, val);
+        }
+    };
+
+    int buf = 0;
+    stage(0, 0);
+    int prev_s = -1, prev_t = 0;  // the slice whose sums wait to be reduced
+    for (int t = t0; t < t1; t++) {
+        g.ka = -cp.a[t] * 1.4426950408889634f;  // -k log2(e)
+        g.kb = -cp.b[t] * 1.4426950408889634f;
+        g.Aa = cp.A_a[t];
+        g.Bb = cp.B_b[t];
+        const F2 ka2 = pk(g.ka, g.ka), kb2 = pk(g.kb, g.kb), Aa2 = pk(g.Aa, g.Aa), Bb2 = pk(g.Bb, g.Bb);
+        const float4 d4 = dirs[((size_t)bi * n_tf + t) * n_phi + warp];
+        if (warp == 0 && lane < n_phi) {
+            const float4 q4 = dirs[((size_t)bi * n_tf + t) * n_phi + lane];
+            sm.dir[lane] = make_cone_dir(make_float3(q4.x, q4.y, q4.z));
+            sm.c[lane] = make_float3(0.5f, 0.5f, 0.0f);
+            sm.k[lane] = make_int2(0, 0);
+        }
+        // a move in x takes a state from lane ux, one in y the row carried over
+        // from another group's lane uy; the ray on this lane's column (group 0) or
+        // row `v` (group 1) changes by -step
+        const bool xp = d4.x >= 0.0f, yp = d4.y >= 0.0f;
+        const int ux = (xp ? (v == 0 ? F - 1 : v - 1) : (v == F - 1 ? 0 : v + 1)) + grp * F;
+        const int uy = (yp ? (grp == 0 ? G - 1 : grp - 1) : (grp + 1 >= G ? 0 : grp + 1)) * F + v;
+        const float step = (yl ? yp : xp) ? 1.0f : -1.0f;
+        const float bs = yl ? g.bsy : g.bsx;
+        float lf = (float)v;   // the ray on this lane's column or row
+        float cb = 0.5f;       // the base ray's coordinate of this lane's axis
+        F2 XA[R / 2], XB[R / 2];
+#pragma unroll
+        for (int q = 0; q < R / 2; q++) XA[q] = XB[q] = pk(0.0f, 0.0f);
+        float fs = (0.0f * g.ls + g.lim_min) * g.inv_sad;  // divergence factor at the step's start
+        // The slice of every pass is the rounded z of the first azimuth's base
+        // ray (DoseComp.cu:300): when that ray ends a slice within 1e-3 below
+        // the next plane it steps over it, and the reference skips that slice
+        // for this zenith bin; the other azimuths keep marching from wherever
+        // they stopped.
+        int s = 0, par = 0;
+        while (s < L) {
+            F2 Tv[R / 2], Rv[R / 2], Dv[R / 2], Pv[R / 2];
+            int s_next = L;
+            for (int round = 0;; round++) {
+                if (warp == 0) {
+                    bool open = true;
+                    if (round > 0) {  // azimuths still inside the slice: their last record does not end it
+                        open = lane < n_phi && sm.count[lane] > 0 && !(sm.code[lane][sm.count[lane] - 1] & kRecEnd);
+                        if ((long long)round * kMarchSteps >= kStepCap) {
+                            open = false;
+                            if (lane == 0) {
+                                atomicExch(&status->code, (int)FD2_ERR_WATCHDOG);
+                                sm.abort = 1;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    march_paths<F>(sm, g, n_phi, s, L, open);
+                }
+                if (round == 0) {
+                    if (prev_s >= 0 && (warp > 0 || n_phi == 1)) reduce(prev_t, prev_s);
+                    cp_async_wait_all();  // this thread's pixels of the slice have landed
+                }
+                __syncthreads();
+                if (sm.abort) return;  // the same for all: written before the barrier only
+                if (round == 0) {
+                    load_cells<R>(&sm.T[buf][cell], Tv);
+                    load_cells<R>(&sm.R[buf][cell], Rv);
+#pragma unroll
+                    for (int q = 0; q < R / 2; q++) {
+                        if (!on) Tv[q] = Rv[q] = pk(0.0f, 0.0f);
+                        Dv[q] = Pv[q] = pk(0.0f, 0.0f);
+                    }
+                }
+                const bool more = sm.more;
+                if (!more) {
+                    s_next = sm.next;
+                    // the next slice to come (or slice 0 of the next zenith pass)
+                    const int st = s_next < L ? s_next : (t + 1 < t1 ? 0 : -1);
+                    if (st >= 0) stage(st, buf ^ 1);
+                }
+                const int n = sm.count[warp];
+                for (int i = 0; i < n; i++) {
+                    for (; i < n; i++) {
+                        const int code = sm.code[warp][i];
+                        if (__any_sync(kAll, code & kRecExact)) break;
+                        const float4 rec = sm.rec[warp][i];
+                        const float cn = yl ? rec.y : rec.x;
+                        if (__any_sync(kAll, code & kRecMoveX)) {
+#pragma unroll
+                            for (int q = 0; q < R / 2; q++) {
+                                const float2 a = up(XA[q]), b = up(XB[q]);
+                                XA[q] = pk(__shfl_sync(kAll, a.x, ux), __shfl_sync(kAll, a.y, ux));
+                                XB[q] = pk(__shfl_sync(kAll, b.x, ux), __shfl_sync(kAll, b.y, ux));
+                            }
+                            if (!yl) lf -= step;
+                        }
+                        if (__any_sync(kAll, code & kRecMoveY)) {
+                            if (__any_sync(kAll, yp)) {
+                                const float ea = __shfl_sync(kAll, up(XA[R / 2 - 1]).y, uy);
+                                const float eb = __shfl_sync(kAll, up(XB[R / 2 - 1]).y, uy);
+#pragma unroll
+                                for (int q = R / 2 - 1; q >= 0; q--) {
+                                    XA[q] = pk(q ? up(XA[q ? q - 1 : 0]).y : ea, up(XA[q]).x);
+                                    XB[q] = pk(q ? up(XB[q ? q - 1 : 0]).y : eb, up(XB[q]).x);
+                                }
+                            } else {
+                                const float ea = __shfl_sync(kAll, up(XA[0]).x, uy);
+                                const float eb = __shfl_sync(kAll, up(XB[0]).x, uy);
+#pragma unroll
+                                for (int q = 0; q < R / 2; q++) {
+                                    const bool e = q == R / 2 - 1;
+                                    XA[q] = pk(up(XA[q]).y, e ? ea : up(XA[e ? q : q + 1]).x);
+                                    XB[q] = pk(up(XB[q]).y, e ? eb : up(XB[e ? q : q + 1]).x);
+                                }
+                            }
+                            if (yl) lf -= step;
+                        }
+                        lf = lf < 0.0f ? lf + F : (lf >= F ? lf - F : lf);
+                        // lateral offset of the ray on this lane's column or row, its edge
+                        // crossing as the sign (the offset enters the length squared)
+                        const float b = __fadd_rn(cb, lf), e = __fadd_rn(cn, lf);
+                        float d = fabsf((e - 0.5f * F) * bs * rec.z - (b - 0.5f * F) * bs * fs);
+                        d = floor_biased(__fdividef(b, (float)F)) != floor_biased(__fdividef(e, (float)F)) ? -d : d;
+                        if (yl) sm.row[warp][par][v] = d;
+                        const float dx = __shfl_sync(kAll, d, v);
+                        const float dxz2 = dx * dx + rec.w;
+                        cb = cn;
+                        fs = rec.z;
+                        __syncwarp();
+                        F2 dy[R / 2];
+                        load_cells<R>(&sm.row[warp][par][on ? grp * R : 0], dy);
+                        par ^= 1;
+                        const F2 dxz = pk(dxz2, dxz2);
+#pragma unroll
+                        for (int q = 0; q < R / 2; q++) {
+                            const F2 l2 = fma2(dy[q], dy[q], dxz);
+                            const float2 l2s = up(l2);
+                            const F2 p = mul2(mul2(l2, pk(rsqrt_sfu(l2s.x), rsqrt_sfu(l2s.y))), Rv[q]);
+                            const float2 xa = up(mul2(p, ka2)), xb = up(mul2(p, kb2));
+                            Dv[q] = fma2(fma2(Bb2, XB[q], mul2(Aa2, XA[q])), p, Dv[q]);
+                            if (last) Pv[q] = add2(Pv[q], p);
+                            XA[q] = fma2(pk(exp2_sfu(xa.x), exp2_sfu(xa.y)), sub2(XA[q], Tv[q]), Tv[q]);
+                            XB[q] = fma2(pk(exp2_sfu(xb.x), exp2_sfu(xb.y)), sub2(XB[q], Tv[q]), Tv[q]);
+                        }
+                        // rays that crossed an edge start anew
+                        const bool wx = __float_as_int(dx) < 0;
+                        if (__any_sync(kAll, wx)) {
+#pragma unroll
+                            for (int q = 0; q < R / 2; q++) {
+                                XA[q].v = wx ? 0ull : XA[q].v;
+                                XB[q].v = wx ? 0ull : XB[q].v;
+                            }
+                        }
+                        const bool w0 = __float_as_int(up(dy[0]).x) < 0, w1 = __float_as_int(up(dy[R / 2 - 1]).y) < 0;
+                        XA[0] = pk(w0 ? 0.0f : up(XA[0]).x, up(XA[0]).y);
+                        XB[0] = pk(w0 ? 0.0f : up(XB[0]).x, up(XB[0]).y);
+                        XA[R / 2 - 1] = pk(up(XA[R / 2 - 1]).x, w1 ? 0.0f : up(XA[R / 2 - 1]).y);
+                        XB[R / 2 - 1] = pk(up(XB[R / 2 - 1]).x, w1 ? 0.0f : up(XB[R / 2 - 1]).y);
+                    }
+                    if (i >= n) break;
+                    const float4 rec = sm.rec[warp][i];
+                    if (on) {
+                        store_cells<R>(&sm.dose[warp][cell], Dv);
+                        store_cells<R>(&sm.xa[warp][cell], XA);
+                        store_cells<R>(&sm.xb[warp][cell], XB);
+                        if (last) store_cells<R>(&sm.path[cell], Pv);
+                    }
+                    const int o = pos_mod(v - (int)lf, F);  // the shift: of x in group 0, of y in group 1
+                    const int2 k = march_exact_step<F, G, R>(
+                        sm, buf, g, make_float2(__shfl_sync(kAll, cb, 0), __shfl_sync(kAll, cb, F)),
+                        make_float2(rec.x, rec.y), fs, rec.z, rec.w, __shfl_sync(kAll, o, 0), __shfl_sync(kAll, o, F), last);
+                    if (on) {
+                        load_cells<R>(&sm.dose[warp][cell], Dv);
+                        load_cells<R>(&sm.xa[warp][cell], XA);
+                        load_cells<R>(&sm.xb[warp][cell], XB);
+                        if (last) load_cells<R>(&sm.path[cell], Pv);
+                    }
+                    __syncwarp();
+                    lf = (float)pos_mod(v - (yl ? k.y : k.x), F);
+                    cb = yl ? rec.y : rec.x;
+                    fs = rec.z;
+                }
+                if (!more) break;
+                __syncthreads();  // the round's records are used
+            }
+            if (on) {
+                store_cells<R>(&sm.dose[warp][cell], Dv);
+                if (last) store_cells<R>(&sm.path[cell], Pv);
+            }
+            __syncthreads();  // the slice's sums stand, its records and data are used
+            prev_s = s;
+            prev_t = t;
+            buf ^= 1;
+            s = s_next;
+        }
+    }
+    if (prev_s >= 0 && (warp > 0 || n_phi == 1)) reduce(prev_t, prev_s);
+}
+
+template <int RPL, bool kCols, bool kTab = false>
 int launch_instance(unsigned blocks, int threads, size_t shm, cudaStream_t st, const fd2_beam_t* d_beams,
                     const float* const* T, const float* const* R, float* const* D, const float4* dirs,
                     const ConeParams& cp, int split, float* planes, size_t plane_stride, DeviceStatus* status,
                     const int* order) {
-    FD2_CHECK_CUDA(cudaFuncSetAttribute(cccs_kernel<RPL, kFx16, kCols, kTab>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    FD2_CHECK_CUDA(cudaFuncSetAttribute(cccs_kernel<RPL, kCols, kTab>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)shm));
-    cccs_kernel<RPL, kFx16, kCols, kTab><<<blocks, threads, shm, st>>>(d_beams, T, R, D, dirs, cp, split, planes,
+    cccs_kernel<RPL, kCols, kTab><<<blocks, threads, shm, st>>>(d_beams, T, R, D, dirs, cp, split, planes,
                                                                  plane_stride, status, order);
     FD2_CHECK_CUDA(cudaGetLastError());
     return FD2_OK;
 }
 
+template <int F, int G, int R>
+int launch_voxel_march(unsigned blocks, int n_phi, cudaStream_t st, const fd2_beam_t* d_beams,
+                       const float* const* T, const float* const* Rho, float* const* D, const float4* dirs,
+                       const ConeParams& cp, int split, float* planes, size_t plane_stride, DeviceStatus* status,
+                       const int* order) {
+    cccs_march_kernel<F, G, R><<<blocks, 32 * n_phi, 0, st>>>(d_beams, T, Rho, D, dirs, cp, split, planes,
+                                                              plane_stride, status, order);
+    FD2_CHECK_CUDA(cudaGetLastError());
+    return FD2_OK;
+}
+
+// Lateral reach of a batch's rays in voxels: what bounds the integers and the
+// biased roundings of the voxel-stationary march.
+struct Reach {
+    double tan_x = 0, tan_y = 0;    // of the cone directions
+    double slice = 0, total = 0;    // largest lateral advance per slice, and over a beam
+    bool finite = true;
+    Reach(const ConeAngles& a) {
+        for (int t = 0; t < a.n_theta_fwd; t++)
+            for (int f = 0; f < a.n_phi; f++) {
+                const double r = std::fabs(std::tan((double)a.theta[t]));
+                tan_x = std::max(tan_x, r * std::fabs(std::cos((double)a.phi[f])));
+                tan_y = std::max(tan_y, r * std::fabs(std::sin((double)a.phi[f])));
+            }
+    }
+    void add(const fd2_beam_t& b) {
+        const double sx = std::fabs(b.long_spacing * tan_x / b.beamlet_size[0]),
+                     sy = std::fabs(b.long_spacing * tan_y / b.beamlet_size[1]);
+        if (!(sx < 1e30 && sy < 1e30)) finite = false;  // (NaN too)
+        slice = std::max({slice, sx, sy});
+        total = std::max(total, std::max(sx, sy) * b.long_dim);
+    }
+    // voxel indices fit 15 bits, and the 1e-4 slack of the slice rule moves a
+    // ray sideways by a fraction of a voxel
+    bool admits() const { return finite && slice < 500.0 && total < 15000.0; }
+};
+
 // The march for a batch.  map: the common map side F when every map of the
-// batch is F x F, else 0.  16 x 16 maps take the 16-pixel instance; other
-// common sides up to 32 the shared-column instance (both need 4..8 azimuth
-// warps); anything else the general per-ray instance.
-int launch_march(int map, int maxP, int n_phi, unsigned blocks, cudaStream_t st, const fd2_beam_t* d_beams,
+// batch is F x F, else 0; reach_ok: Reach::admits.  Common sides of 8, 12 and
+// 16 take the voxel-stationary march (1..8 azimuth warps); other common sides
+// up to 24 the half-table instance and up to 32 the shared-column instance
+// (4..8 azimuth warps); anything else the general per-ray instance.
+int launch_march(int map, bool reach_ok, int maxP, int n_phi, unsigned blocks, cudaStream_t st, const fd2_beam_t* d_beams,
                  const float* const* T, const float* const* R, float* const* D, const float4* dirs,
                  const ConeParams& cp, int split, float* planes, size_t plane_stride, DeviceStatus* status,
                  const int* order = nullptr) {
     const int threads = 32 * n_phi;
     const size_t shm = (size_t)(1 + n_phi) * maxP * sizeof(float2);
-    const bool warps_ok = threads >= 128 && threads <= kFx16Threads;
-    if (map == 16 && threads <= kFx16Threads)
-        return launch_instance<8, true, false>(blocks, threads, (size_t)n_phi * (256 * sizeof(float4) + 16 * sizeof(float2)),
-                                               st, d_beams, T, R, D, dirs, cp, split, planes, plane_stride, status, order);
+    const bool warps_ok = threads >= 128 && threads <= kMapThreads;
+    if (reach_ok && n_phi <= kMarchWarps) {
+        if (map == 16)
+            return launch_voxel_march<16, 2, 8>(blocks, n_phi, st, d_beams, T, R, D, dirs, cp, split, planes,
+                                                plane_stride, status, order);
+        if (map == 12)
+            return launch_voxel_march<12, 2, 6>(blocks, n_phi, st, d_beams, T, R, D, dirs, cp, split, planes,
+                                                plane_stride, status, order);
+        if (map == 8)
+            return launch_voxel_march<8, 4, 2>(blocks, n_phi, st, d_beams, T, R, D, dirs, cp, split, planes,
+                                               plane_stride, status, order);
+    }
     if (map > 0 && map <= 24 && warps_ok) {  // half-table instance: rays per lane = ceil(F^2 / 32)
         const int P = map * map;
         if (P <= 64)
-            return launch_instance<2, false, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
+            return launch_instance<2, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                           planes, plane_stride, status, order);
         if (P <= 160)
-            return launch_instance<5, false, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
+            return launch_instance<5, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                           planes, plane_stride, status, order);
         if (P <= 256)
-            return launch_instance<8, false, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
+            return launch_instance<8, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                           planes, plane_stride, status, order);
         if (P <= 416)
-            return launch_instance<13, false, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp,
+            return launch_instance<13, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp,
                                                            split, planes, plane_stride, status, order);
-        return launch_instance<18, false, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
+        return launch_instance<18, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                        planes, plane_stride, status, order);
     }
     if (map > 0 && map <= 32 && warps_ok) {
         const int k = 32 / map, rows = (map + k - 1) / k;  // rows per lane
         if (rows <= 8)
-            return launch_instance<8, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
+            return launch_instance<8, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                    planes, plane_stride, status, order);
         if (rows <= 20)
-            return launch_instance<20, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
+            return launch_instance<20, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                     planes, plane_stride, status, order);
         if (rows <= 24)
-            return launch_instance<24, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
+            return launch_instance<24, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                     planes, plane_stride, status, order);
-        return launch_instance<32, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
+        return launch_instance<32, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
                                                 plane_stride, status, order);
     }
     if (maxP <= 256)
-        return launch_instance<8, false, false>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
+        return launch_instance<8, false>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
                                                 plane_stride, status, order);
-    return launch_instance<32, false, false>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
+    return launch_instance<32, false>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
                                              plane_stride, status, order);
 }
 
@@ -665,7 +1163,9 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
     const unsigned blocks = (unsigned)(schedule == 1 ? n_beams * fwd.size() : n_beams);
     int map = -1;
     for (size_t i = 0; i < n_beams && map != 0; i++) map = common_map(map, h_beams[i]);
-    FD2_TRY(launch_march(map, maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp, schedule,
+    Reach reach(ang);
+    for (size_t i = 0; i < n_beams; i++) reach.add(h_beams[i]);
+    FD2_TRY(launch_march(map, reach.admits(), maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp, schedule,
                          d_planes, plane_stride, ctx->d_status, schedule == 1 ? nullptr : d_order));
     ctx->launches += 2;  // direction table + march
     if (schedule == 1) {
@@ -893,6 +1393,7 @@ extern "C" int fd2_dose_compute_static(size_t fmap_npixels, size_t n_beams, cons
     // map sizes of the batch, read back in chunks through a small stack buffer
     cudaStream_t st = (cudaStream_t)stream;
     fd2_beam_t hb[kBeamChunk];
+    Reach reach(ang);
     int maxP = 0;
     int map = -1;
     for (size_t i0 = 0; i0 < n_beams; i0 += kBeamChunk) {
@@ -904,6 +1405,7 @@ extern "C" int fd2_dose_compute_static(size_t fmap_npixels, size_t n_beams, cons
                         "dose_compute_static: Terma and density pitches differ");
             maxP = std::max(maxP, (int)(hb[i].fmap_size[0] * hb[i].fmap_size[1]));
             map = map == 0 ? 0 : common_map(map, hb[i]);
+            reach.add(hb[i]);
         }
     }
     FD2_REQUIRE(maxP > 0 && maxP <= 1024, FD2_ERR_INVALID_ARGUMENT,
@@ -917,7 +1419,7 @@ extern "C" int fd2_dose_compute_static(size_t fmap_npixels, size_t n_beams, cons
     FD2_TRY(launch_cone_dirs(d_beams, n_beams, ang, d_dirs, st));
     const float* const* T = (const float* const*)d_terma;
     const float* const* R = (const float* const*)d_density_bev;
-    FD2_TRY(launch_march(map, maxP, cp.n_phi, (unsigned)n_beams, st, d_beams, T, R, d_dose, d_dirs, cp, 0, nullptr, 0,
+    FD2_TRY(launch_march(map, reach.admits(), maxP, cp.n_phi, (unsigned)n_beams, st, d_beams, T, R, d_dose, d_dirs, cp, 0, nullptr, 0,
                          d_status));
     if (status_out)
         FD2_CHECK_CUDA(cudaMemcpyAsync(status_out, &d_status->code, sizeof(int), cudaMemcpyDefault, st));

@@ -1,0 +1,59 @@
+"""The voxel-stationary CCCS march (8x8, 12x12 and 16x16 maps) against the
+general per-ray instance, which a call with maps of two sizes takes.
+
+Both take the same discrete steps (the same float comparisons); a voxel's dose
+is a sum of at most a few hundred positive deposits in FP32, each a product of a
+few rounded factors, so the two agree to 300 * 2^-24 = 2e-5 of the voxel and,
+where the path sums nearly cancel against the 1e-4 of the normalisation, to
+1e-6 of the maximum."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from fastdose_b200 import _lib, api, phantoms
+from fastdose_b200.types import make_bundle
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(ctx, ph, side, on, dens, spec, gantry, count=6):
+    bund = make_bundle(ph.centre(), (gantry, 0.3, 0.1), sad=100.0, fluence_dim=count, beamlet_size=0.5,
+                       sub_fluence_dim=side, sub_fluence_on=on, long_spacing=0.25)
+    flags = np.zeros(count * count, np.uint8)
+    flags[:: max(1, count * count // count)] = 1  # distinct beamlet sizes: distinct ray paths
+    b = api.BEVBatch(api.bundle_beamlets(bund, flags, ph.volume))
+    api.TermaComputeCollective(ctx, b, api.beamlet_fluence(bund), dens, spec)
+    return b
+
+
+@pytest.mark.parametrize("n_phi", [1, 4, 6, 8])
+@pytest.mark.parametrize("side,on", [(8, 2), (12, 4), (16, 4)])
+def test_march_matches_the_per_ray_instance(ctx, side, on, n_phi):
+    import torch
+
+    ph = phantoms.torso_phantom(seed=side + n_phi, dim=(72, 64, 56))
+    dens = api.Density(ctx, ph.density, ph.volume)
+    spec = api.Spectrum(ctx, phantoms.synthetic_spectrum())
+    kern = api.Kernel(ctx, phantoms.synthetic_kernel(n_phi=n_phi))
+    b = _batch(ctx, ph, side, on, dens, spec, 0.7)
+    api.DoseComputeCollective(ctx, b, kern)  # one map size: the march
+    # the same beams beside one of another map size: the general instance
+    other = _batch(ctx, ph, 10, 2, dens, spec, 1.9, count=1)
+    dose = [torch.zeros_like(b.dose), torch.zeros_like(other.dose)]
+    beams = torch.cat([b.d_beams, other.d_beams])
+    ptrs = {}
+    for name in ("terma", "dens"):
+        ptrs[name] = torch.cat([b._ptrs[name], other._ptrs[name]])
+    off = [dose[0].data_ptr() + 4 * int(o) for o in b.offsets[:-1]] + [dose[1].data_ptr()]
+    ptrs["dose"] = torch.from_numpy(np.array(off, np.uint64).view(np.int64)).cuda()
+    n = len(b.beams) + 1
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(ctx.lib.fd2_dose_compute(ctx.h, side * side, n, p(beams), p(ptrs["terma"]), p(ptrs["dens"]),
+                                        p(ptrs["dose"]), kern.h, C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+               "dose_compute")
+    torch.cuda.synchronize()
+    got, ref = b.dose.double(), dose[0].double()
+    assert float(ref.max()) > 0
+    assert torch.all((got == 0) == (ref == 0))
+    assert torch.all((got - ref).abs() <= 2e-5 * ref + 1e-6 * ref.max())
