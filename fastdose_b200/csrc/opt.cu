@@ -233,7 +233,7 @@ __global__ void ptv_column_sums(const int64_t* __restrict__ off, ColView col,
     double s = 0;
     for (int64_t k = off[r] + lane; k < off[r + 1]; k += 32) {
         if (col.at(k) >= n_ptv) break;
-        s += (double)as_float(val[slot(k)]);
+        s += (double)as_float(val[col.at_slot(k)]);
     }
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) out[r] = s * (row_scale ? (double)row_scale[r] : 1.0);

@@ -14,14 +14,17 @@ namespace fd2 {
 constexpr int kChunk = 256;           // nonzeros per SpMV chunk (32 lanes x 8)
 constexpr int kChunkWords = kChunk / 32;
 
-// Storage position of logical nonzero k.  Inside a chunk, logical element
+// Storage position of logical nonzero k.  A matrix of long rows whose x is
+// gathered from global memory is interleaved inside a chunk: logical element
 // 32 i + l is stored at 8 l + i, so that lane l's two 16-byte loads bring it
-// elements l, l + 32, ..., l + 224: each of the warp's x-gathers then covers 32
-// consecutive nonzeros of the row instead of 32 elements 8 apart.
-__host__ __device__ __forceinline__ int64_t slot(int64_t k) {
+// elements l, l + 32, ..., l + 224, and each of the warp's x-gathers covers 32
+// consecutive nonzeros of the row instead of 32 elements 8 apart.  In the other
+// matrices lane l holds elements 8 l .. 8 l + 7, rotated by l / 4: a gather of
+// consecutive columns from shared memory then meets every bank once.
+__host__ __device__ __forceinline__ int64_t slot(int64_t k, bool interleaved) {
     const int64_t c = k / kChunk;
     const int e = (int)(k % kChunk);
-    return c * kChunk + (e % 32) * 8 + e / 32;
+    return c * kChunk + (interleaved ? (e % 32) * 8 + e / 32 : (e & ~7) + ((e - (e >> 5)) & 7));
 }
 
 // Column index of logical nonzero k in either index format (after finalize).
@@ -30,8 +33,10 @@ struct ColView {
     const uint16_t* col16;  // PACKED16: [nnz_pad] offset from the chunk base, storage order
     const int32_t* cbase;   // PACKED16: per chunk base, or -(1 + exception slot)
     const int32_t* exc;     // PACKED16: [slots * kChunk] columns of exception chunks, storage order
+    bool interleaved;       // storage order: slot()
+    __device__ __forceinline__ int64_t at_slot(int64_t k) const { return slot(k, interleaved); }
     __device__ __forceinline__ int at(int64_t k) const {
-        const int64_t q = slot(k);
+        const int64_t q = at_slot(k);
         if (col) return col[q];
         const int32_t b = cbase[k / kChunk];
         return b >= 0 ? b + (int)col16[q] : exc[(int64_t)(-1 - b) * kChunk + (q % kChunk)];
@@ -62,19 +67,21 @@ struct fd2_matrix {
     // stream SpMV plan
     int64_t n_chunks = 0;          // nnz_pad / kChunk
     uint32_t* d_head = nullptr;    // [n_chunks * kChunkWords] row starts: per chunk 32 bytes, one per
-                                   // lane; bit i of byte l: element 32 i + l starts its row
+                                   // lane; bit i of byte l: the lane's element i starts its row
     int32_t* d_chunk_h = nullptr;  // [n_chunks] row starts before the chunk
     int32_t* d_chunk_row0 = nullptr;  // [n_chunks] first row starting in the chunk if its starts are
                                       // consecutive rows, else -1 - d_chunk_h[c]
     int32_t* d_nzrow = nullptr;    // [n_nzrows] rows with nonzeros, in order
     int64_t n_nzrows = 0;
-    int n_warps = 0;               // SpMV warps (contiguous chunk ranges)
+    int n_warps = 0;               // SpMV warps
+    int n_ranges = 0;              // contiguous chunk ranges, n_warps or a multiple of it
     bool x_in_smem = false;        // SpMV instance: x staged in shared memory (cols small enough)
-    int64_t* d_carry_row = nullptr;  // [n_warps] row open at each warp's range end
-    float* d_carry_val = nullptr;    // [n_warps] its partial sum
+    bool interleaved = true;       // storage order inside a chunk (slot())
+    int64_t* d_carry_row = nullptr;  // [n_ranges] row open at each range's end
+    float* d_carry_val = nullptr;    // [n_ranges] its partial sum
     float* d_xs = nullptr;           // [cols] x times the column scale
 
-    fd2::ColView cols_view() const { return fd2::ColView{d_col, d_col16, d_cbase, d_exc}; }
+    fd2::ColView cols_view() const { return fd2::ColView{d_col, d_col16, d_cbase, d_exc, interleaved}; }
 };
 
 namespace fd2 {

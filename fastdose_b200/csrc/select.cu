@@ -38,7 +38,7 @@ __global__ void select_rows_kernel(const int64_t* __restrict__ src_off, ColView 
             const int c = cv.at(a + i);
             if (c < l || c >= h) atomicAdd(bad, 1);
             dst_col[d + i] = c + sh;
-            dst_val[d + i] = src_val[slot(a + i)];
+            dst_val[d + i] = src_val[cv.at_slot(a + i)];
         }
     }
 }

@@ -9,15 +9,18 @@
 //    a contiguous range of chunks, so every warp streams the same number of
 //    matrix bytes whatever the row lengths (VOI rows of a few hundred
 //    nonzeros, beamlet rows of tens of thousands, empty rows);
-//  * inside a chunk the nonzeros are stored lane-major (slot()), so a lane's
-//    two 16-byte streaming loads (`ld.global.cs`: the matrix is read once, x
-//    stays in the 126 MB L2) bring its 8 elements l, l+32, ..., l+224, and each
-//    x-gather of the warp covers 32 consecutive nonzeros;
+//  * a lane's two 16-byte streaming loads (`ld.global.cs`: the matrix is read
+//    once, x stays in the 126 MB L2) bring 8 elements of a chunk;
 //  * rows are found from a row-start bitmap (1 bit per nonzero) and a per-chunk
-//    count of row starts: a 32-element slice without a row start is one FMA
-//    per lane into the open row; a slice with row starts closes the open row
-//    with a warp sum and sums the rows inside it with a segmented warp-shuffle
-//    scan -- no shared memory, no block barrier;
+//    count of row starts; a chunk without row starts is one FMA per lane and
+//    element into the open row;
+//  * storage order and summation come in two forms.  Where x is in shared
+//    memory, and for short rows, a lane's elements are consecutive: a chunk
+//    with row starts is summed per lane up to and after its row start, and one
+//    segmented warp scan over the lanes closes all its rows.  For long rows
+//    with x in global memory the chunk is interleaved (slot()), so that each
+//    x-gather of the warp covers 32 consecutive nonzeros, and the rare slices
+//    of 32 elements with row starts are scanned one by one;
 //  * the row open at the end of a warp's range is carried; a second kernel
 //    adds carries in warp order.
 //
@@ -41,7 +44,13 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kStreamThreads = 256;
 constexpr int kMaxStreamWarps = 148 * 64;  // one full wave of 64 warps per SM
 constexpr int kSmemThreads = 1024;          // x-in-shared-memory variant: one block per SM
-constexpr int64_t kSmemXMaxBytes = 200 * 1024;
+// Ranges of chunks per warp and the least chunks in one.  Rows of few nonzeros
+// lie together (the edge of the dose), and their chunks cost several times the
+// others: with four ranges spread over the matrix, no warp owns only such.
+// 250k x 10k, 200 nonzeros a row: 87 us with one range, 83 with 2 and 4, 85
+// with 8; long interleaved rows only lose prefetch (54 us with one, 58 with 4).
+constexpr int kRangesPerWarp = 4, kMinRange = 8;
+constexpr int64_t kSmemXMaxBytes = 200 * 1024, kSmemXSmall = 32 * 1024;
 
 struct StreamArgs {
     const void* val;
@@ -52,7 +61,7 @@ struct StreamArgs {
     const int32_t* nzrow;
     const float* row_scale;
     int64_t n_chunks;
-    int n_warps;
+    int n_warps, n_ranges;
     int64_t rows;
     int64_t* carry_row;
     float* carry_val;
@@ -144,19 +153,31 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// One warp per contiguous range of chunks.  In a chunk, slice i holds logical
-// elements 32 i .. 32 i + 31 (one per lane); bit i of lane l's row-start byte
-// flags element 32 i + l.  A slice without row starts only adds to the open
+// One warp per contiguous range of chunks.
+//
+// kInter: in a chunk, slice i holds logical elements 32 i .. 32 i + 31 (one per
+// lane); bit i of lane l's row-start byte flags element 32 i + l.  A slice without row starts only adds to the open
 // row (one FMA per lane); a slice with row starts closes the open row (warp
 // sum), sums the rows that start and end inside it with a segmented warp scan,
 // and leaves its last row open.
+//
+// Otherwise lane l holds elements 8 l .. 8 l + 7 of the chunk, rotated by l / 4
+// (register i: element (i + l / 4) mod 8; the row-start byte is in element
+// order).  Products are
+// summed inside the lane up to its first row start and after its last one (and
+// rows inside the lane are written), then one segmented scan over the lanes
+// closes every row of the chunk.  The slice form costs a dependent chain of
+// shuffles per slice, up to eight a chunk: on a VOI matrix of 250k x 10k and 200
+// nonzeros a row, whose sparse ends hold rows of a few nonzeros, the warps there
+// ran three times as long as the others (176 us a product in 16 bits, 81 in this
+// form; 172 and 83 in 32 bits).
 //
 // kSmemX: x is copied to shared memory first (one block of kSmemThreads per
 // SM) and the gathers read it there: 32 lanes reading 32 scattered columns
 // cost a few bank cycles instead of up to 32 L1 tag lookups.  With 16-bit
 // values a warp loads ahead: the next chunk while it sums the current one (x
 // in shared memory), or two chunks at a time (x in global memory).
-template <typename T, bool kPacked, bool kSmemX>
+template <typename T, bool kPacked, bool kSmemX, bool kInter>
 __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX ? 1 : 4)
     spmv_stream_kernel(StreamArgs a, const float* __restrict__ x, float* __restrict__ y) {
     extern __shared__ float xs[];
@@ -167,14 +188,10 @@ __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     if (w >= a.n_warps) return;  // uniform per warp
-    const int64_t c0 = (int64_t)w * a.n_chunks / a.n_warps, c1 = (int64_t)(w + 1) * a.n_chunks / a.n_warps;
-    float oacc = 0.0f;        // this lane's share of the open row (the row in progress), this warp's part
-    bool open_valid = false;  // the warp has met an element of the open row
+    float oacc = 0.0f, open = 0.0f;  // the open row (the row in progress): this lane's share, and (!kInter) its sum so far
+    bool shares = false;      // !kInter: some lane's share is not zero
+    bool open_valid = false;  // the range has met an element of the open row
     int open_row = 0;
-    if (c0 < c1) {
-        const int hb0 = __ldg(a.chunk_h + c0);
-        if (hb0 > 0 && !(__ldg(a.head + c0 * kChunkWords) & 1u)) open_row = __ldg(a.nzrow + hb0 - 1);
-    }
     auto xv = [&](int col) -> float {
         if constexpr (kSmemX)
             return xs[col];
@@ -185,6 +202,94 @@ __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX
     auto row_at = [&](const RawChunk<T, kPacked>& r, int j) -> int {
         return r.row0 >= 0 ? r.row0 + j : __ldg(a.nzrow + (-1 - r.row0) + j);
     };
+    auto body_lanes = [&](const RawChunk<T, kPacked>& r, const float (&v)[8], const int (&col)[8]) {
+        if (!__any_sync(kFull, r.h != 0u)) {  // no row starts: all of it is the open row
+#pragma unroll
+            for (int i = 0; i < 8; i++) oacc = fmaf(v[i], xv(col[i]), oacc);
+            open_valid = shares = true;
+            return;
+        }
+        float p[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) p[i] = v[i] * xv(col[i]);
+        const uint32_t hm = __ballot_sync(kFull, r.h != 0u);
+        float pre = 0.0f, suf = 0.0f;  // before the lane's first row start (all, without one), from its last on
+        int before, total;             // row starts in earlier lanes, and in the chunk
+        if (!__any_sync(kFull, (r.h & (r.h - 1u)) != 0u)) {  // at most one row start a lane
+            const uint32_t h1 = (r.h - 1u) & 0xffu;          // bits before the row start; all without one
+            const uint32_t below = h1 >> (lane >> 2) | h1 << (8 - (lane >> 2));
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (below >> i & 1u)
+                    pre += p[i];
+                else
+                    suf += p[i];
+            }
+            before = __popc(hm & ((1u << lane) - 1u));
+            total = __popc(hm);
+        } else {
+            const int nh = __popc(r.h);
+            int inc = nh;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(kFull, inc, o);
+                if (lane >= o) inc += t;
+            }
+            before = inc - nh;
+            total = __shfl_sync(kFull, inc, 31);
+#pragma unroll
+            for (int b = 1; b < 8; b <<= 1) {  // products back to element order
+                float q[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) q[i] = (lane >> 2) & b ? p[(i - b) & 7] : p[i];
+#pragma unroll
+                for (int i = 0; i < 8; i++) p[i] = q[i];
+            }
+            int k = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (r.h >> i & 1u) {
+                    if (k == 0)
+                        pre = suf;
+                    else
+                        put(y, a.row_scale, row_at(r, before + k - 1), suf);
+                    suf = 0.0f;
+                    k++;
+                }
+                suf += p[i];
+            }
+            if (k == 0) {
+                pre = suf;
+                suf = 0.0f;
+            }
+        }
+        // sums since the last row start at or before each lane
+        float s = r.h ? suf : pre;
+        const uint32_t le = hm & (0xffffffffu >> (31 - lane));
+        const int start = le ? 31 - __clz(le) : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(kFull, s, o);
+            if (lane - o >= start) s += t;
+        }
+        float prev = __shfl_up_sync(kFull, s, 1);
+        if (lane == 0) prev = 0.0f;
+        if (shares) {
+            open += warp_sum(oacc);
+            oacc = 0.0f;
+            shares = false;
+        }
+        if (r.h) {
+            const float closing = prev + pre;
+            if (before > 0)
+                put(y, a.row_scale, row_at(r, before - 1), closing);
+            else if (open_valid || lane > 0 || !(r.h & 1u))
+                put(y, a.row_scale, open_row, open + closing);
+        }
+        open = __shfl_sync(kFull, s, 31);
+        open_row = row_at(r, total - 1);
+        open_valid = true;
+    };
     auto body = [&](const RawChunk<T, kPacked>& r, int64_t c) {
         float v[8];
         int col[8];
@@ -193,6 +298,10 @@ __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX
         else
             unpack_vals<T>(r.v, v);
         unpack_cols<T, kPacked>(r, a.cols, c, lane, col);
+        if constexpr (!kInter) {
+            body_lanes(r, v, col);
+            return;
+        }
         if (!__any_sync(kFull, r.h != 0u)) {  // no row starts: all of it is the open row
 #pragma unroll
             for (int i = 0; i < 8; i++) oacc = fmaf(v[i], xv(col[i]), oacc);
@@ -242,55 +351,65 @@ __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX
             open_valid = true;
         }
     };
-    if constexpr (sizeof(T) == 2 && kSmemX) {
-        // 16-bit values, x in shared memory: the next chunk's loads are issued
-        // before this chunk is summed, so a warp keeps a chunk in flight while
-        // it computes
-        RawChunk<T, kPacked> r;
-        if (c0 < c1) load_raw(a, c0, lane, r);
-        for (int64_t c = c0; c < c1; c++) {
-            RawChunk<T, kPacked> rn;
-            const bool more = c + 1 < c1;  // uniform per warp
-            if (more) load_raw(a, c + 1, lane, rn);
-            body(r, c);
-            if (more) r = rn;
+    for (int range = w; range < a.n_ranges; range += a.n_warps) {
+        const int64_t c0 = (int64_t)range * a.n_chunks / a.n_ranges, c1 = (int64_t)(range + 1) * a.n_chunks / a.n_ranges;
+        oacc = open = 0.0f;
+        shares = open_valid = false;
+        open_row = 0;
+        if (c0 < c1) {
+            const int hb0 = __ldg(a.chunk_h + c0);
+            if (hb0 > 0 && !(__ldg(a.head + c0 * kChunkWords) & 1u)) open_row = __ldg(a.nzrow + hb0 - 1);
         }
-    } else if constexpr (sizeof(T) == 2) {
-        // 16-bit values, x gathered from global memory: two chunks' loads are
-        // issued together (fewer registers held than the rolling form)
-        for (int64_t c = c0; c < c1; c += 2) {
-            RawChunk<T, kPacked> r0, r1;
-            load_raw(a, c, lane, r0);
-            const bool two = c + 1 < c1;  // uniform per warp
-            if (two) load_raw(a, c + 1, lane, r1);
-            body(r0, c);
-            if (two) body(r1, c + 1);
-        }
-    } else {
-        for (int64_t c = c0; c < c1; c++) {
+        if constexpr (sizeof(T) == 2 && kSmemX) {
+            // 16-bit values, x in shared memory: the next chunk's loads are issued
+            // before this chunk is summed, so a warp keeps a chunk in flight while
+            // it computes
             RawChunk<T, kPacked> r;
-            load_raw(a, c, lane, r);
-            body(r, c);
+            if (c0 < c1) load_raw(a, c0, lane, r);
+            for (int64_t c = c0; c < c1; c++) {
+                RawChunk<T, kPacked> rn;
+                const bool more = c + 1 < c1;  // uniform per warp
+                if (more) load_raw(a, c + 1, lane, rn);
+                body(r, c);
+                if (more) r = rn;
+            }
+        } else if constexpr (sizeof(T) == 2) {
+            // 16-bit values, x gathered from global memory: two chunks' loads are
+            // issued together (fewer registers held than the rolling form)
+            for (int64_t c = c0; c < c1; c += 2) {
+                RawChunk<T, kPacked> r0, r1;
+                load_raw(a, c, lane, r0);
+                const bool two = c + 1 < c1;  // uniform per warp
+                if (two) load_raw(a, c + 1, lane, r1);
+                body(r0, c);
+                if (two) body(r1, c + 1);
+            }
+        } else {
+            for (int64_t c = c0; c < c1; c++) {
+                RawChunk<T, kPacked> r;
+                load_raw(a, c, lane, r);
+                body(r, c);
+            }
         }
-    }
-    const float part = warp_sum(oacc);
-    if (lane == 0) {
-        a.carry_row[w] = open_valid ? (int64_t)open_row : a.rows;
-        a.carry_val[w] = part;
+        const float part = open + warp_sum(oacc);
+        if (lane == 0) {
+            a.carry_row[range] = open_valid ? (int64_t)open_row : a.rows;
+            a.carry_val[range] = part;
+        }
     }
 }
 
-// Adds the carries of rows that cross warp ranges: the first warp of each run
-// of equal carry rows sums the run in warp order.
-__global__ void spmv_fixup_kernel(int n_warps, const int64_t* __restrict__ carry_row,
+// Adds the carries of rows that cross ranges: the first range of each run of
+// equal carry rows sums the run in range order.
+__global__ void spmv_fixup_kernel(int n_ranges, const int64_t* __restrict__ carry_row,
                                   const float* __restrict__ carry_val, const float* __restrict__ row_scale,
                                   int64_t rows, float* __restrict__ y) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_warps) return;
+    if (t >= n_ranges) return;
     const int64_t r = carry_row[t];
     if (r >= rows || (t > 0 && carry_row[t - 1] == r)) return;
     float s = 0.0f;
-    for (int u = t; u < n_warps && carry_row[u] == r; u++) s += carry_val[u];
+    for (int u = t; u < n_ranges && carry_row[u] == r; u++) s += carry_val[u];
     y[r] += row_scale ? row_scale[r] * s : s;
 }
 
@@ -307,16 +426,18 @@ unsigned grid_for(int64_t n, int threads = 256) {
 
 // the row-start bit of off[r] for every row with nonzeros (rows own distinct
 // bits; atomicOr makes the word updates safe).  Layout: a chunk has 32 bytes,
-// one per lane; bit i of byte l flags logical element 32 i + l.
-__global__ void mark_row_starts(const int64_t* __restrict__ off, int64_t rows, uint32_t* __restrict__ head,
-                                int32_t* __restrict__ nonempty) {
+// one per lane; bit i of byte l flags the lane's element i: logical element
+// 32 i + l of an interleaved chunk, 8 l + i otherwise.
+__global__ void mark_row_starts(const int64_t* __restrict__ off, int64_t rows, bool interleaved,
+                                uint32_t* __restrict__ head, int32_t* __restrict__ nonempty) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
         const bool ne = off[r + 1] > off[r];
         nonempty[r] = ne;
-        if (ne) {  // element e of chunk c: lane e % 32's byte, bit e / 32
+        if (ne) {
             const int64_t c = off[r] / kChunk;
-            const int e = (int)(off[r] % kChunk), l = e & 31;
-            atomicOr(head + c * kChunkWords + (l >> 2), 1u << ((l & 3) * 8 + (e >> 5)));
+            const int e = (int)(off[r] % kChunk);
+            const int l = interleaved ? e & 31 : e >> 3, i = interleaved ? e >> 5 : e & 7;
+            atomicOr(head + c * kChunkWords + (l >> 2), 1u << ((l & 3) * 8 + i));
         }
     }
 }
@@ -383,10 +504,11 @@ __global__ void chunk_span(const int32_t* __restrict__ col, int64_t nnz, int64_t
 // from logical-order columns into storage order
 __global__ void pack_columns(const int32_t* __restrict__ col, int64_t nnz, int64_t n_chunks,
                              const int32_t* __restrict__ wide, const int32_t* __restrict__ exc_slot,
-                             int32_t* __restrict__ base, uint16_t* __restrict__ col16, int32_t* __restrict__ exc) {
+                             int32_t* __restrict__ base, uint16_t* __restrict__ col16, int32_t* __restrict__ exc,
+                             bool interleaved) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n_chunks * kChunk;
          k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = k / kChunk, q = slot(k);
+        const int64_t c = k / kChunk, q = slot(k, interleaved);
         const int cv = k < nnz ? col[k] : 0;
         if (wide[c]) {
             exc[(int64_t)exc_slot[c] * kChunk + q % kChunk] = cv;
@@ -399,9 +521,9 @@ __global__ void pack_columns(const int32_t* __restrict__ col, int64_t nnz, int64
 
 // logical order -> storage order
 template <typename E>
-__global__ void to_storage_order(const E* __restrict__ src, E* __restrict__ dst, int64_t n) {
+__global__ void to_storage_order(const E* __restrict__ src, E* __restrict__ dst, int64_t n, bool interleaved) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-        dst[slot(k)] = src[k];
+        dst[slot(k, interleaved)] = src[k];
 }
 
 __global__ void mark_wide_bases(const int32_t* __restrict__ wide, const int32_t* __restrict__ slot, int64_t n_chunks,
@@ -477,7 +599,7 @@ __global__ void unpack_entries(const int64_t* __restrict__ off, int64_t rows, Co
                                float* __restrict__ val_out) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
         const int c = cv.at(k);
-        float v = to_float(val[slot(k)]);
+        float v = to_float(val[cv.at_slot(k)]);
         if (axis == FD2_SCALE_COLS)
             v *= s[c];
         else if (axis == FD2_SCALE_ROWS)
@@ -508,19 +630,19 @@ __global__ void offsets_from_sorted(const int32_t* __restrict__ keys, int64_t nn
 
 template <typename T>
 __global__ void gather_transposed(const int64_t* __restrict__ off, int64_t rows, const int64_t* __restrict__ perm,
-                                  const T* __restrict__ val, int64_t nnz, int32_t* __restrict__ col_out,
-                                  T* __restrict__ val_out) {
+                                  const T* __restrict__ val, bool interleaved, int64_t nnz,
+                                  int32_t* __restrict__ col_out, T* __restrict__ val_out) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
         const int64_t src = perm[k];
         col_out[k] = (int32_t)row_of(off, rows, src);
-        val_out[k] = val[slot(src)];
+        val_out[k] = val[slot(src, interleaved)];
     }
 }
 
 // The x-in-shared-memory instance of the stream kernel, allowed the largest x.
 template <typename T, bool kPacked>
 cudaError_t allow_smem_x() {
-    return cudaFuncSetAttribute(spmv_stream_kernel<T, kPacked, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(spmv_stream_kernel<T, kPacked, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kSmemXMaxBytes);
 }
 
@@ -528,10 +650,14 @@ template <typename T, bool kPacked>
 int launch_stream_fmt(const fd2_matrix* m, const StreamArgs& a, const float* x, float* y, cudaStream_t st) {
     if (m->x_in_smem) {  // the shared-memory limit was raised when the matrix was finalized
         const unsigned blocks = (unsigned)(((int64_t)m->n_warps * 32 + kSmemThreads - 1) / kSmemThreads);
-        spmv_stream_kernel<T, kPacked, true><<<blocks, kSmemThreads, (size_t)m->cols * sizeof(float), st>>>(a, x, y);
+        spmv_stream_kernel<T, kPacked, true, false>
+            <<<blocks, kSmemThreads, (size_t)m->cols * sizeof(float), st>>>(a, x, y);
     } else {
         const unsigned blocks = (unsigned)(((int64_t)m->n_warps * 32 + kStreamThreads - 1) / kStreamThreads);
-        spmv_stream_kernel<T, kPacked, false><<<blocks, kStreamThreads, 0, st>>>(a, x, y);
+        if (m->interleaved)
+            spmv_stream_kernel<T, kPacked, false, true><<<blocks, kStreamThreads, 0, st>>>(a, x, y);
+        else
+            spmv_stream_kernel<T, kPacked, false, false><<<blocks, kStreamThreads, 0, st>>>(a, x, y);
     }
     FD2_CHECK_CUDA(cudaGetLastError());
     return FD2_OK;
@@ -540,13 +666,14 @@ int launch_stream_fmt(const fd2_matrix* m, const StreamArgs& a, const float* x, 
 template <typename T>
 int launch_stream(const fd2_matrix* m, const float* x, float* y, cudaStream_t st) {
     StreamArgs a{m->d_val, m->cols_view(), m->d_head, m->d_chunk_h, m->d_chunk_row0, m->d_nzrow,
-                 m->scale_axis == FD2_SCALE_ROWS ? m->d_scale : nullptr, m->n_chunks, m->n_warps, m->rows,
+                 m->scale_axis == FD2_SCALE_ROWS ? m->d_scale : nullptr, m->n_chunks, m->n_warps,
+                 m->n_ranges, m->rows,
                  m->d_carry_row, m->d_carry_val, (int)m->cols};
     if (m->index_format == FD2_INDEX_PACKED16)
         FD2_TRY((launch_stream_fmt<T, true>(m, a, x, y, st)));
     else
         FD2_TRY((launch_stream_fmt<T, false>(m, a, x, y, st)));
-    spmv_fixup_kernel<<<(m->n_warps + 255) / 256, 256, 0, st>>>(m->n_warps, m->d_carry_row, m->d_carry_val,
+    spmv_fixup_kernel<<<(m->n_ranges + 255) / 256, 256, 0, st>>>(m->n_ranges, m->d_carry_row, m->d_carry_val,
                                                                a.row_scale, m->rows, y);
     FD2_CHECK_CUDA(cudaGetLastError());
     return FD2_OK;
@@ -581,8 +708,8 @@ int transpose_typed(const fd2_matrix* m, fd2_matrix* t, cudaStream_t st) {
     }
     if (e == cudaSuccess) {
         offsets_from_sorted<<<grid_for(t->rows + 1), 256, 0, st>>>(keys_out, nnz, t->rows, t->d_off);
-        gather_transposed<T><<<grid_for(nnz), 256, 0, st>>>(m->d_off, m->rows, perm_out, (const T*)m->d_val, nnz,
-                                                            t->d_col, (T*)t->d_val);
+        gather_transposed<T><<<grid_for(nnz), 256, 0, st>>>(m->d_off, m->rows, perm_out, (const T*)m->d_val,
+                                                            m->interleaved, nnz, t->d_col, (T*)t->d_val);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -635,26 +762,34 @@ void matrix_free(fd2_matrix* m) {
     m->d_carry_val = m->d_xs = nullptr;
 }
 
-// Warps of one full wave of the stream kernel for this matrix's instance: every
-// warp owns one contiguous range, so there is no second, partial wave.  A
-// matrix whose x fits in shared memory (cols x 4 bytes <= kSmemXMaxBytes) uses
-// the x-in-shared-memory instance, one block of kSmemThreads per SM.
+// Warps of one full wave of the stream kernel for this matrix's instance, so
+// that there is no second, partial wave.  A matrix whose x fits in shared memory
+// (cols x 4 bytes <= kSmemXMaxBytes) uses the x-in-shared-memory instance, one
+// block of kSmemThreads per SM, unless x is large and the matrix small: every SM
+// copies all of x, which above kSmemXSmall costs more than it saves on a matrix
+// of fewer bytes than those copies (48k columns, 2.8e6 nonzeros in 16 bits: 28 MB
+// of copies for 11 MB of matrix).
 template <typename T, bool kPacked>
 int resident_warps(fd2_matrix* m, int sm_count) {
     int per_sm = 0;
     const int64_t xb = m->cols * (int64_t)sizeof(float);
     m->x_in_smem = false;
-    if (xb > 0 && xb <= kSmemXMaxBytes && allow_smem_x<T, kPacked>() == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmv_stream_kernel<T, kPacked, true>, kSmemThreads,
+    const int64_t entry = (int64_t)sizeof(T) + (kPacked ? 2 : 4);
+    const bool worth = xb <= kSmemXSmall || m->nnz * entry >= xb * sm_count;
+    if (xb > 0 && xb <= kSmemXMaxBytes && worth && allow_smem_x<T, kPacked>() == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmv_stream_kernel<T, kPacked, true, false>, kSmemThreads,
                                                       (size_t)xb) == cudaSuccess &&
         per_sm >= 1) {
         m->x_in_smem = true;
+        m->interleaved = false;
         return per_sm * sm_count * (kSmemThreads / 32);
     }
     cudaGetLastError();  // a refused attribute or query leaves the global-gather instance
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmv_stream_kernel<T, kPacked, false>, kStreamThreads,
-                                                      0) != cudaSuccess ||
-        per_sm < 1)
+    // rows shorter than a quarter chunk: most slices of an interleaved chunk would
+    // hold row starts
+    m->interleaved = m->nnz >= (kChunk / 4) * m->rows;
+    auto kernel = m->interleaved ? spmv_stream_kernel<T, kPacked, false, true> : spmv_stream_kernel<T, kPacked, false, false>;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kStreamThreads, 0) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     return per_sm * sm_count * (kStreamThreads / 32);
 }
@@ -678,11 +813,14 @@ int stream_warps(fd2_matrix* m) {
 int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     m->n_chunks = round_chunk(m->nnz) / kChunk;
     m->n_warps = (int)std::max<int64_t>(1, std::min<int64_t>(m->n_chunks, stream_warps(m)));
+    m->n_ranges = m->n_warps;
+    if (!m->interleaved)
+        m->n_ranges *= (int)std::max<int64_t>(1, std::min<int64_t>(kRangesPerWarp, m->n_chunks / ((int64_t)m->n_warps * kMinRange)));
     FD2_CHECK_CUDA(cudaMalloc(&m->d_head, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t)));
     FD2_CHECK_CUDA(cudaMalloc(&m->d_chunk_h, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t)));
     FD2_CHECK_CUDA(cudaMalloc(&m->d_chunk_row0, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_row, m->n_warps * sizeof(int64_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_val, m->n_warps * sizeof(float)));
+    FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_row, m->n_ranges * sizeof(int64_t)));
+    FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_val, m->n_ranges * sizeof(float)));
     if (m->scale_axis == FD2_SCALE_COLS)
         FD2_CHECK_CUDA(cudaMalloc(&m->d_xs, std::max<int64_t>(m->cols, 1) * sizeof(float)));
     FD2_CHECK_CUDA(cudaMemsetAsync(m->d_head, 0, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t),
@@ -702,7 +840,7 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
         return FD2_ERR_OUT_OF_MEMORY;
     }
     int rc = FD2_OK;
-    if (m->rows) mark_row_starts<<<grid_for(m->rows), 256, 0, st>>>(m->d_off, m->rows, m->d_head, ne);
+    if (m->rows) mark_row_starts<<<grid_for(m->rows), 256, 0, st>>>(m->d_off, m->rows, m->interleaved, m->d_head, ne);
     if (m->rows) rc = exclusive_scan(ne, pos, m->rows, st);
     int32_t last_ne = 0, last_pos = 0;
     if (!rc && m->rows) {
@@ -744,7 +882,7 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             rc = FD2_ERR_OUT_OF_MEMORY;
         if (!rc) {
             pack_columns<<<grid_for(m->n_chunks * kChunk), 256, 0, st>>>(m->d_col, m->nnz, m->n_chunks, wide, eslot,
-                                                                        m->d_cbase, m->d_col16, m->d_exc);
+                                                                        m->d_cbase, m->d_col16, m->d_exc, m->interleaved);
             mark_wide_bases<<<grid_for(m->n_chunks), 256, 0, st>>>(wide, eslot, m->n_chunks, m->d_cbase);
             if (cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
         }
@@ -773,9 +911,9 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             rc = FD2_ERR_OUT_OF_MEMORY;
         } else {
             if (vs == 4)
-                to_storage_order<uint32_t><<<grid_for(pad), 256, 0, st>>>((const uint32_t*)m->d_val, (uint32_t*)tmp, pad);
+                to_storage_order<uint32_t><<<grid_for(pad), 256, 0, st>>>((const uint32_t*)m->d_val, (uint32_t*)tmp, pad, m->interleaved);
             else
-                to_storage_order<uint16_t><<<grid_for(pad), 256, 0, st>>>((const uint16_t*)m->d_val, (uint16_t*)tmp, pad);
+                to_storage_order<uint16_t><<<grid_for(pad), 256, 0, st>>>((const uint16_t*)m->d_val, (uint16_t*)tmp, pad, m->interleaved);
             if (cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
             cudaFree(m->d_val);
             m->d_val = tmp;
@@ -785,7 +923,7 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             if (cudaMalloc(&tc, pad * sizeof(int32_t)) != cudaSuccess) {
                 rc = FD2_ERR_OUT_OF_MEMORY;
             } else {
-                to_storage_order<int32_t><<<grid_for(pad), 256, 0, st>>>(m->d_col, tc, pad);
+                to_storage_order<int32_t><<<grid_for(pad), 256, 0, st>>>(m->d_col, tc, pad, m->interleaved);
                 if (cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
                 cudaFree(m->d_col);
                 m->d_col = tc;

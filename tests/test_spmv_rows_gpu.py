@@ -1,0 +1,50 @@
+"""Products over rows of a constant length around the lane (8), slice (32) and
+chunk (256 nonzeros) sizes of the stream kernel, with runs of empty rows, in the
+forms a matrix is stored in: x in shared memory, and x in global memory with
+short rows (a lane's elements consecutive) or long ones (interleaved).
+
+Tolerance: a row of n nonzeros is a sum in FP32 of n products in some order, so
+it is within (n + 2) 2^-24 of its |A||x| sum."""
+import numpy as np
+import pytest
+
+from fastdose_b200 import optimize
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cols", [900, 60000])
+@pytest.mark.parametrize("length", [1, 2, 7, 8, 9, 31, 33, 63, 64, 65, 255, 256, 257, 700])
+def test_rows_of_one_length(ctx, cols, length):
+    import torch
+
+    rng = np.random.default_rng(length)
+    rows = max(40, 40000 // length) + 3
+    counts = np.full(rows, length, np.int64)
+    counts[rng.random(rows) < 0.2] = 0
+    counts[:2] = 0
+    counts[-1] = 0
+    counts[rows // 2] = min(cols, 5 * length + 3)
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    # ascending columns: a random start and random gaps that stay inside
+    col = np.concatenate([np.sort(rng.choice(cols, c, replace=False)) for c in counts]).astype(np.int64)
+    val = (rng.random(len(col)) - 0.3).astype(np.float32)
+    x = rng.standard_normal(cols).astype(np.float32)
+    row = np.repeat(np.arange(rows), counts)
+    for vt, fmt in (("f32", "i32"), ("f32", "packed16"), ("f16", "packed16"), ("bf16", "i32")):
+        M = optimize.Matrix.from_csr(ctx, off, col, val, cols, value_type=vt, index_format=fmt)
+        o, c, v = M.to_host()
+        np.testing.assert_array_equal(o, off)
+        np.testing.assert_array_equal(c, col)
+        y = M.spmv(torch.from_numpy(x).cuda()).cpu().numpy()
+        p = v.astype(np.float64) * x[col]
+        ref = np.bincount(row, p, rows)
+        bound = np.bincount(row, np.abs(p), rows)
+        # 16-bit values: x is scaled by the column's scale, one more rounding each
+        assert np.all(np.abs(y - ref) <= (counts + 4) * 2.0 ** -24 * bound)
+        assert np.all(y[counts == 0] == 0)
+        T = M.transpose()
+        yt = T.spmv(torch.from_numpy(rng.standard_normal(rows).astype(np.float32)).cuda())
+        assert yt.shape == (cols,) and bool(torch.isfinite(yt).all())
+        for a, b in zip(T.transpose().to_host(), (o, c, v)):
+            np.testing.assert_array_equal(a, b)
