@@ -30,6 +30,7 @@
 // correctly rounded float operations in the order the reference writes them,
 // starting from cone directions computed on the host; the CPU oracle performs
 // the identical operations, so both march the same segments bit for bit.
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <algorithm>
@@ -45,7 +46,9 @@ namespace fd2 {
 namespace {
 
 constexpr int kStepCap = 1 << 20;  // per-slice step cap (the watchdog bound)
-constexpr int kMapThreads = 256;   // the common-map instances are compiled for at most 8 azimuth warps
+constexpr int kMapThreads = 256;     // the common-map instances are compiled for at most 8 azimuth warps
+constexpr int kSpreadThreads = 768;  // and the spread ones (kWpa > 1) for blocks of up to 24 warps
+constexpr int kMaxCluster = 4;       // blocks of a spread cluster
 
 struct RayGeom {  // per-beamlet scalars the march needs
     float hx, hy;      // fmap_size / 2
@@ -163,16 +166,38 @@ __device__ __forceinline__ float rsqrt_sfu(float x) {
 }
 __device__ __forceinline__ float seg_length(float l2) { return l2 * rsqrt_sfu(l2); }
 
-// Block: n_phi warps.  Dynamic shared memory: float2 tr[P] (Terma, density of
+// Could the midpoints of the segment c..n of two rays of a step, whole voxels
+// apart, round to the same voxel?  (The base ray's midpoint close to a boundary;
+// margins as in path_axis.)
+__device__ __forceinline__ bool may_meet(float c, float n, float ff) {
+    const float m = __fmul_rn(__fadd_rn(c, n), 0.5f);
+    const float eps = 4e-6f + 3e-7f * (fabsf(c) + ff);
+    return !(fabsf(m - floorf(m) - 0.5f) < 0.5f - eps);
+}
+
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Block: n_phi warps (kWpa per azimuth of the block).  Dynamic shared memory: float2 tr[P] (Terma, density of
 // the current slice) followed by float2 dp[n_phi][P] (per-azimuth dose and path
 // sums).  RPL = rays per lane (P <= 32 * RPL).
 // kCols: every map of the batch is F x F with F <= 32 -- each lane owns one
 // column (lane % F) and the rows lane / F + k j (k = 32 / F lanes per column),
 // so the x half of the voxel work is done once per lane and the y half once per
 // row and shared by shuffles; RPL >= ceil(F / k).
-template <int RPL, bool kCols = false, bool kTab = false>
-__global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
-                                  (kCols || kTab) && RPL <= 8 ? 4 : (kCols || kTab ? 3 : 1))
+//
+// kWpa > 1 spreads a (beamlet, zenith bin) that would leave most of the device
+// idle: kWpa warps share an azimuth's rays, RPL each, and the azimuths are
+// divided over the blocks of a cluster, which reduce them through each other's
+// shared memory.  The rays of a step deposit into distinct voxels, whichever
+// warp marches them, so one barrier of the azimuth's warps per step keeps the
+// deposits of a voxel in step order, as with one warp; where rounding could let
+// two rays of a step meet (a midpoint within some 1e-5 of a boundary), the warps
+// deposit in turn.  The dose is the same bit for bit.
+template <int RPL, bool kCols = false, bool kTab = false, int kWpa = 1>
+__global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? kMapThreads : 768),
+                                  kWpa > 1 ? 1 : ((kCols || kTab) && RPL <= 8 ? 4 : (kCols || kTab ? 3 : 1)))
     cccs_kernel(const fd2_beam_t* __restrict__ beams,
                                                    const float* const* __restrict__ terma,
                                                    const float* const* __restrict__ dens,
@@ -189,8 +214,12 @@ __global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
     const int n_tf = cp.n_theta_fwd, n_phi = cp.n_phi;
     // order (optional, one block per beamlet only): the beamlet each block
     // marches, longest first, so the launch ends on short blocks
-    const int bi = split ? blockIdx.x / n_tf : (order ? order[blockIdx.x] : blockIdx.x);
-    const int t0 = split ? blockIdx.x % n_tf : 0;
+    namespace cg = cooperative_groups;
+    const int n_cl = kWpa > 1 ? (int)cg::this_cluster().num_blocks() : 1;
+    const int rank = kWpa > 1 ? (int)cg::this_cluster().block_rank() : 0;
+    const int unit = blockIdx.x / n_cl;
+    const int bi = split ? unit / n_tf : (order ? order[unit] : unit);
+    const int t0 = split ? unit % n_tf : 0;
     const int t1 = split ? t0 + 1 : n_tf;
     const fd2_beam_t& b = beams[bi];
     RayGeom g;
@@ -212,17 +241,20 @@ __global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
     // kTab: per block, the (column, row) table entries of ray j of each lane
     // (x entry = column, y entry = F + row; all ones past the map), and per
     // azimuth warp the step's 2F halves
-    __shared__ uint32_t s_pairs[kTab ? RPL * 32 : 1];
-    __shared__ float2 s_htab[kTab ? 8 * 64 : 1];
+    __shared__ uint32_t s_pairs[kTab ? kWpa * RPL * 32 : 1];
+    __shared__ float2 s_htab[kTab ? (kWpa > 1 ? kSpreadThreads / 32 : 8) * 64 : 1];
     if constexpr (kTab) {
-        for (int i = threadIdx.x; i < RPL * 32; i += blockDim.x)  // ray i / 32 of lane i % 32 is cell i
+        for (int i = threadIdx.x; i < kWpa * RPL * 32; i += blockDim.x)  // ray i / 32 of lane i % 32 is cell i
             s_pairs[i] = i < g.P ? (uint32_t)(i % g.fx) | (uint32_t)(g.fx + i / g.fx) << 16 : 0xffffffffu;
     }  // visible after the first slice's barrier
 
     float2* tr = smem;
     float2* dp = smem + g.P;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float2* mydp = dp + (size_t)warp * g.P;
+    // this warp's azimuth in its block and its share of that azimuth's rays
+    const int az = warp / kWpa, sub = warp % kWpa;
+    const int n_az = n_phi / n_cl, phi = rank * n_az + az;
+    float2* mydp = dp + (size_t)az * g.P;
     const float* __restrict__ T = terma[bi];
     const float* __restrict__ R = dens[bi];
     float* __restrict__ D = dose[bi];
@@ -257,7 +289,7 @@ __global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
     for (int t = t0; t < t1; t++) {
         const float Aa = cp.A_a[t], Bb = cp.B_b[t];
         const float ka = -cp.a[t] * 1.4426950408889634f, kb = -cp.b[t] * 1.4426950408889634f;  // -k log2(e)
-        const float4 d4 = dirs[((size_t)bi * n_tf + t) * n_phi + warp];
+        const float4 d4 = dirs[((size_t)bi * n_tf + t) * n_phi + phi];
         const ConeDir cd = make_cone_dir(make_float3(d4.x, d4.y, d4.z));
         float3 c = make_float3(0.5f, 0.5f, 0.0f);
         float fs = (c.z * g.ls + g.lim_min) * g.inv_sad;  // divergence factor at c, carried step to step
@@ -278,7 +310,7 @@ __global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
             for (int v = threadIdx.x; v < g.P; v += blockDim.x)
                 tr[v] = s == st_s ? make_float2(s_stage[v], s_stage[kStageP + v])
                                   : make_float2(__ldg(T + (size_t)s * pitch + v), __ldg(R + (size_t)s * pitch + v));
-            for (int v = lane; v < g.P; v += 32) mydp[v] = make_float2(0.0f, 0.0f);
+            for (int v = 32 * sub + lane; v < g.P; v += 32 * kWpa) mydp[v] = make_float2(0.0f, 0.0f);
             __syncthreads();
             st_s = s + 1 < g.L ? s + 1 : (t + 1 < t1 ? 0 : -1);
             if (st_s >= 0)
@@ -294,110 +326,118 @@ __global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
                 const bool flag = next_point(c, cd, np);
                 const float fe = (np.z * g.ls + g.lim_min) * g.inv_sad;
                 const float dzp = (np.z - c.z) * g.ls;
-                if constexpr (kCols) {
-                    const float btx = __fadd_rn(c.x, fcol), ntx = __fadd_rn(np.x, fcol);
-                    const int cx = mid_index(btx, ntx, g.ffx, g.fx);
-                    const bool wrapx = crosses_edge(btx, ntx, g.ffx);
-                    const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
-                    const float dxz2 = dxp * dxp + dzp * dzp;
-                    const float bty = __fadd_rn(c.y, frow), nty = __fadd_rn(np.y, frow);
-                    const int ycode = mid_index(bty, nty, g.ffy, g.fy) | (crosses_edge(bty, nty, g.ffy) ? 64 : 0);
-                    const float dyq = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
+                // the azimuth's warps in turn when two of its rays might meet in a voxel
+                const bool turns = kWpa > 1 && (may_meet(c.x, np.x, g.ffx) || may_meet(c.y, np.y, g.ffy));
+                for (int turn = turns ? 0 : sub;; turn++) {
+                    if (turn == sub) {
+                        if constexpr (kCols) {
+                            const float btx = __fadd_rn(c.x, fcol), ntx = __fadd_rn(np.x, fcol);
+                            const int cx = mid_index(btx, ntx, g.ffx, g.fx);
+                            const bool wrapx = crosses_edge(btx, ntx, g.ffx);
+                            const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
+                            const float dxz2 = dxp * dxp + dzp * dzp;
+                            const float bty = __fadd_rn(c.y, frow), nty = __fadd_rn(np.y, frow);
+                            const int ycode = mid_index(bty, nty, g.ffy, g.fy) | (crosses_edge(bty, nty, g.ffy) ? 64 : 0);
+                            const float dyq = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
 #pragma unroll
-                    for (int j = 0; j < RPL; j++) {
-                        const int y = cgrp + kgrp * j;
-                        const bool on = clane && y < g.fy;
-                        const int yc = __shfl_sync(0xffffffffu, ycode, on ? y : 0);
-                        const float dyp = __shfl_sync(0xffffffffu, dyq, on ? y : 0);
-                        const int mi = on ? cx + g.fx * (yc & 63) : 0;
-                        const bool wrap = wrapx || (yc & 64);
-                        const float l2 = dxz2 + dyp * dyp;
-                        const float len = seg_length(l2);
-                        const float2 trv = tr[mi];
-                        const float p = len * trv.y;
-                        const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
-                        const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
-                        if (on) {
-                            float2 acc = mydp[mi];
-                            acc.x += dep;
-                            acc.y += p;
-                            mydp[mi] = acc;
+                            for (int j = 0; j < RPL; j++) {
+                                const int y = cgrp + kgrp * (kWpa > 1 ? sub * RPL + j : j);
+                                const bool on = clane && y < g.fy;
+                                const int yc = __shfl_sync(0xffffffffu, ycode, on ? y : 0);
+                                const float dyp = __shfl_sync(0xffffffffu, dyq, on ? y : 0);
+                                const int mi = on ? cx + g.fx * (yc & 63) : 0;
+                                const bool wrap = wrapx || (yc & 64);
+                                const float l2 = dxz2 + dyp * dyp;
+                                const float len = seg_length(l2);
+                                const float2 trv = tr[mi];
+                                const float p = len * trv.y;
+                                const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
+                                const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
+                                if (on) {
+                                    float2 acc = mydp[mi];
+                                    acc.x += dep;
+                                    acc.y += p;
+                                    mydp[mi] = acc;
+                                }
+                                XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
+                                XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
+                            }
+                        } else if constexpr (kTab) {
+                            // F x F map, F <= 24: the rays of lane l are the cells l + 32 j,
+                            // so all 32 lanes carry rays whatever F.  The step's 2F halves
+                            // (x of each column, y of each row) are evaluated once, one per
+                            // lane and round, into the warp's half table {+-|offset|,
+                            // bytes into the slice}, the edge crossing as the sign bit;
+                            // each ray then reads its column's and its row's entry.
+                            float2* ht = s_htab + 64 * warp;
+                            for (int h = lane; h < 2 * g.fx; h += 32) {
+                                const bool yh = h >= g.fx;
+                                const float off = (float)(yh ? h - g.fx : h);
+                                const float hb = __fadd_rn(yh ? c.y : c.x, off), hn = __fadd_rn(yh ? np.y : np.x, off);
+                                const float ff = yh ? g.ffy : g.ffx, hh = yh ? g.hy : g.hx, bs = yh ? g.bsy : g.bsx;
+                                const int hi = mid_index(hb, hn, ff, yh ? g.fy : g.fx);
+                                const float hq = fabsf((hn - hh) * bs * fe - (hb - hh) * bs * fs);
+                                const float hs = crosses_edge(hb, hn, ff) ? -hq : hq;
+                                const int bytes = (int)sizeof(float2) * (yh ? hi * g.fx : hi);
+                                ht[h] = make_float2(hs, __int_as_float(bytes));
+                            }
+                            __syncwarp();
+                            const float dz2 = dzp * dzp;
+#pragma unroll
+                            for (int j = 0; j < RPL; j++) {
+                                const uint32_t pr = s_pairs[32 * (kWpa > 1 ? sub * RPL + j : j) + lane];
+                                const bool on = pr != 0xffffffffu;
+                                const float2 xe = ht[on ? (pr & 0xffffu) : 0], ye = ht[on ? (pr >> 16) : 0];
+                                const bool wrap = (__float_as_int(xe.x) | __float_as_int(ye.x)) < 0;
+                                const int mb = __float_as_int(xe.y) + __float_as_int(ye.y);
+                                const float dxz2 = xe.x * xe.x + dz2;
+                                const float l2 = dxz2 + ye.x * ye.x;
+                                const float len = seg_length(l2);
+                                const float2 trv = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(tr) + mb);
+                                const float p = len * trv.y;
+                                const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
+                                const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
+                                if (on) {
+                                    float2* acc_p = reinterpret_cast<float2*>(reinterpret_cast<char*>(mydp) + mb);
+                                    float2 acc = *acc_p;
+                                    acc.x += dep;
+                                    acc.y += p;
+                                    *acc_p = acc;
+                                }
+                                XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
+                                XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
+                            }
+                        } else {
+#pragma unroll
+                        for (int j = 0; j < RPL; j++) {
+                            const float btx = __fadd_rn(c.x, fix[j]), ntx = __fadd_rn(np.x, fix[j]);
+                            const float bty = __fadd_rn(c.y, fiy[j]), nty = __fadd_rn(np.y, fiy[j]);
+                            const int cx = mid_index(btx, ntx, g.ffx, g.fx);
+                            const int cy = mid_index(bty, nty, g.ffy, g.fy);
+                            const int mi = cx + cy * g.fx;
+                            const bool wrap = crosses_edge(btx, ntx, g.ffx) || crosses_edge(bty, nty, g.ffy);
+                            // physical segment length (d_calcLineSeg, DoseComp.cu:114-144)
+                            const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
+                            const float dyp = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
+                            const float l2 = dxp * dxp + dyp * dyp + dzp * dzp;
+                            const float len = seg_length(l2);
+                            const float2 trv = tr[act[j] ? mi : 0];
+                            const float p = len * trv.y;
+                            const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
+                            const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
+                            if (act[j]) {
+                                float2 acc = mydp[mi];
+                                acc.x += dep;
+                                acc.y += p;
+                                mydp[mi] = acc;
+                            }
+                            XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
+                            XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
                         }
-                        XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
-                        XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
-                    }
-                } else if constexpr (kTab) {
-                    // F x F map, F <= 24: the rays of lane l are the cells l + 32 j,
-                    // so all 32 lanes carry rays whatever F.  The step's 2F halves
-                    // (x of each column, y of each row) are evaluated once, one per
-                    // lane and round, into the warp's half table {+-|offset|,
-                    // bytes into the slice}, the edge crossing as the sign bit;
-                    // each ray then reads its column's and its row's entry.
-                    float2* ht = s_htab + 64 * warp;
-                    for (int h = lane; h < 2 * g.fx; h += 32) {
-                        const bool yh = h >= g.fx;
-                        const float off = (float)(yh ? h - g.fx : h);
-                        const float hb = __fadd_rn(yh ? c.y : c.x, off), hn = __fadd_rn(yh ? np.y : np.x, off);
-                        const float ff = yh ? g.ffy : g.ffx, hh = yh ? g.hy : g.hx, bs = yh ? g.bsy : g.bsx;
-                        const int hi = mid_index(hb, hn, ff, yh ? g.fy : g.fx);
-                        const float hq = fabsf((hn - hh) * bs * fe - (hb - hh) * bs * fs);
-                        const float hs = crosses_edge(hb, hn, ff) ? -hq : hq;
-                        const int bytes = (int)sizeof(float2) * (yh ? hi * g.fx : hi);
-                        ht[h] = make_float2(hs, __int_as_float(bytes));
-                    }
-                    __syncwarp();
-                    const float dz2 = dzp * dzp;
-#pragma unroll
-                    for (int j = 0; j < RPL; j++) {
-                        const uint32_t pr = s_pairs[32 * j + lane];
-                        const bool on = pr != 0xffffffffu;
-                        const float2 xe = ht[on ? (pr & 0xffffu) : 0], ye = ht[on ? (pr >> 16) : 0];
-                        const bool wrap = (__float_as_int(xe.x) | __float_as_int(ye.x)) < 0;
-                        const int mb = __float_as_int(xe.y) + __float_as_int(ye.y);
-                        const float dxz2 = xe.x * xe.x + dz2;
-                        const float l2 = dxz2 + ye.x * ye.x;
-                        const float len = seg_length(l2);
-                        const float2 trv = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(tr) + mb);
-                        const float p = len * trv.y;
-                        const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
-                        const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
-                        if (on) {
-                            float2* acc_p = reinterpret_cast<float2*>(reinterpret_cast<char*>(mydp) + mb);
-                            float2 acc = *acc_p;
-                            acc.x += dep;
-                            acc.y += p;
-                            *acc_p = acc;
                         }
-                        XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
-                        XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
                     }
-                } else {
-#pragma unroll
-                for (int j = 0; j < RPL; j++) {
-                    const float btx = __fadd_rn(c.x, fix[j]), ntx = __fadd_rn(np.x, fix[j]);
-                    const float bty = __fadd_rn(c.y, fiy[j]), nty = __fadd_rn(np.y, fiy[j]);
-                    const int cx = mid_index(btx, ntx, g.ffx, g.fx);
-                    const int cy = mid_index(bty, nty, g.ffy, g.fy);
-                    const int mi = cx + cy * g.fx;
-                    const bool wrap = crosses_edge(btx, ntx, g.ffx) || crosses_edge(bty, nty, g.ffy);
-                    // physical segment length (d_calcLineSeg, DoseComp.cu:114-144)
-                    const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
-                    const float dyp = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
-                    const float l2 = dxp * dxp + dyp * dyp + dzp * dzp;
-                    const float len = seg_length(l2);
-                    const float2 trv = tr[act[j] ? mi : 0];
-                    const float p = len * trv.y;
-                    const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
-                    const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
-                    if (act[j]) {
-                        float2 acc = mydp[mi];
-                        acc.x += dep;
-                        acc.y += p;
-                        mydp[mi] = acc;
-                    }
-                    XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
-                    XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
-                }
+                    if constexpr (kWpa > 1) named_barrier(1 + az, 32 * kWpa);
+                    if (!turns || turn == kWpa - 1) break;
                 }
                 c = np;
                 fs = fe;
@@ -406,18 +446,47 @@ __global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
                 if (++guard >= kStepCap) {
                     if (lane == 0) {
                         atomicExch(&status->code, (int)FD2_ERR_WATCHDOG);
-                        *s_abort = 1;
+                        if constexpr (kWpa > 1)
+                            *cg::this_cluster().map_shared_rank(s_abort, 0) = 1;
+                        else
+                            *s_abort = 1;
                     }
                     break;
                 }
             }
-            if (threadIdx.x == 0) {
+            if (threadIdx.x == 0 && rank == 0) {
                 // the first azimuth's plane after this slice; it always lies ahead
                 const int nxt = (int)roundf(c.z);
                 *s_next = nxt > s ? nxt : g.L;
             }
+            int s_new;
+            if constexpr (kWpa > 1) {
+                cg::this_cluster().sync();
+                const int* ctrl = cg::this_cluster().map_shared_rank(s_ctrl, 0);
+                s_new = ctrl[1] ? g.L : ctrl[0];
+                // this block's share of the pixels, over all blocks' azimuths in order
+                const float2* part[kMaxCluster];
+#pragma unroll
+                for (int r = 0; r < kMaxCluster; r++)
+                    part[r] = cg::this_cluster().map_shared_rank(dp, r < n_cl ? r : 0);
+                for (int v = rank * blockDim.x + threadIdx.x; v < g.P; v += n_cl * blockDim.x) {
+                    float sum = 0.0f, last_sum_p = 0.0f;
+#pragma unroll
+                    for (int r = 0; r < kMaxCluster; r++)
+                        if (r < n_cl)
+                            for (int w = 0; w < n_az; w++) {
+                                const float2 d = part[r][(size_t)w * g.P + v];
+                                sum += d.x;
+                                last_sum_p = d.y;
+                            }
+                    split_out[(size_t)unit * split_stride + (size_t)s * g.P + v] = sum / (last_sum_p + 1e-4f);
+                }
+                cg::this_cluster().sync();  // every block's sums and rank 0's s_next are read
+                s = s_new;
+                continue;
+            }
             __syncthreads();
-            const int s_new = *s_abort ? g.L : *s_next;
+            s_new = *s_abort ? g.L : *s_next;
             // reduce azimuths in order; normalise by the last azimuth's path sum
             for (int v = threadIdx.x; v < g.P; v += blockDim.x) {
                 float sum = 0.0f, last_sum_p;
@@ -425,7 +494,7 @@ __global__ void __launch_bounds__(kCols || kTab ? kMapThreads : 768,
                 last_sum_p = dp[(size_t)(n_phi - 1) * g.P + v].y;
                 const float val = sum / (last_sum_p + 1e-4f);
                 if (split)
-                    split_out[(size_t)blockIdx.x * split_stride + (size_t)s * g.P + v] = val;
+                    split_out[(size_t)unit * split_stride + (size_t)s * g.P + v] = val;
                 else
                     // this block alone owns beam bi's dose and each (s, v) stays with
                     // one thread, so a fire-and-forget add gives D + val in pass order
@@ -1088,25 +1157,49 @@ int launch_march(int map, bool reach_ok, int maxP, int n_phi, unsigned blocks, c
         return launch_instance<18, false, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
                                                        planes, plane_stride, status, order);
     }
-    if (map > 0 && map <= 32 && warps_ok) {
-        const int k = 32 / map, rows = (map + k - 1) / k;  // rows per lane
-        if (rows <= 8)
-            return launch_instance<8, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
-                                                   planes, plane_stride, status, order);
-        if (rows <= 20)
-            return launch_instance<20, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
-                                                    planes, plane_stride, status, order);
-        if (rows <= 24)
-            return launch_instance<24, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split,
-                                                    planes, plane_stride, status, order);
+    if (map > 0 && map <= 32 && warps_ok)  // 25 to 32: one lane per column, up to 32 rows each
         return launch_instance<32, true>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
-                                                plane_stride, status, order);
-    }
+                                         plane_stride, status, order);
     if (maxP <= 256)
         return launch_instance<8, false>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
                                                 plane_stride, status, order);
     return launch_instance<32, false>(blocks, threads, shm, st, d_beams, T, R, D, dirs, cp, split, planes,
                                              plane_stride, status, order);
+}
+
+// The spread march: 17 x 17 to 32 x 32 maps, where an azimuth's rays keep a warp
+// busy for hundreds of instructions a step, in a batch under schedule 1 whose
+// (beamlet, zenith bin) pairs leave SMs without a block.
+template <int RPL, bool kCols, bool kTab, int kWpa>
+int launch_spread(unsigned blocks, int cluster, int n_phi, size_t maxP, cudaStream_t st, const fd2_beam_t* d_beams,
+                  const float* const* T, const float* const* R, float* const* D, const float4* dirs,
+                  const ConeParams& cp, float* planes, size_t plane_stride, DeviceStatus* status) {
+    const size_t shm = (size_t)(1 + n_phi / cluster) * maxP * sizeof(float2);
+    FD2_CHECK_CUDA(cudaFuncSetAttribute(cccs_kernel<RPL, kCols, kTab, kWpa>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)shm));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks * cluster);
+    cfg.blockDim = dim3(32 * kWpa * (n_phi / cluster));
+    cfg.dynamicSmemBytes = shm;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    FD2_CHECK_CUDA(cudaLaunchKernelEx(&cfg, cccs_kernel<RPL, kCols, kTab, kWpa>, d_beams, T, R, D, dirs, cp, 1, planes,
+                                      plane_stride, status, (const int*)nullptr));
+    return FD2_OK;
+}
+
+// Blocks per cluster of the spread march: the azimuths are divided evenly and
+// the clusters stay within two blocks an SM; 0 when it is not taken.
+int spread_cluster(int map, int n_phi, unsigned blocks, int sm_count) {
+    if (map < 17 || map > 32 || n_phi < 4 || n_phi > 8) return 0;
+    for (int c : {kMaxCluster, 2})
+        if (n_phi % c == 0 && blocks * (unsigned)c <= 2u * (unsigned)sm_count) return c;
+    return 0;
 }
 
 // common map side of a batch (F when every map is F x F), else 0
@@ -1165,8 +1258,19 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
     for (size_t i = 0; i < n_beams && map != 0; i++) map = common_map(map, h_beams[i]);
     Reach reach(ang);
     for (size_t i = 0; i < n_beams; i++) reach.add(h_beams[i]);
-    FD2_TRY(launch_march(map, reach.admits(), maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp, schedule,
-                         d_planes, plane_stride, ctx->d_status, schedule == 1 ? nullptr : d_order));
+    const int cluster = schedule == 1 ? spread_cluster(map, k->n_phi, blocks, ctx->sm_count) : 0;
+    if (cluster && map <= 24)
+        FD2_TRY((launch_spread<5, false, true, 4>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
+                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
+    else if (cluster && k->n_phi / cluster <= 3)
+        FD2_TRY((launch_spread<4, true, false, 8>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
+                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
+    else if (cluster)
+        FD2_TRY((launch_spread<8, true, false, 4>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
+                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
+    else
+        FD2_TRY(launch_march(map, reach.admits(), maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp, schedule,
+                             d_planes, plane_stride, ctx->d_status, schedule == 1 ? nullptr : d_order));
     ctx->launches += 2;  // direction table + march
     if (schedule == 1) {
         dim3 grid(std::max(1, std::min(64, (int)((plane_stride + 255) / 256))), (unsigned)n_beams);

@@ -57,3 +57,37 @@ def test_march_matches_the_per_ray_instance(ctx, side, on, n_phi):
     assert float(ref.max()) > 0
     assert torch.all((got == 0) == (ref == 0))
     assert torch.all((got - ref).abs() <= 2e-5 * ref + 1e-6 * ref.max())
+
+
+@pytest.mark.parametrize("n_phi", [4, 6, 8])
+@pytest.mark.parametrize("side", [17, 20, 24, 25, 32])
+def test_spread_march_is_the_march_of_a_large_batch(ctx, side, n_phi):
+    """One beam of a wide map is spread over clusters of blocks with several
+    warps an azimuth; 24 copies of it are not.  The same dose, bit for bit."""
+    import torch
+
+    from fastdose_b200.types import BEAM_DTYPE
+
+    ph = phantoms.torso_phantom(seed=side, dim=(64, 56, 48))
+    dens = api.Density(ctx, ph.density, ph.volume)
+    spec = api.Spectrum(ctx, phantoms.synthetic_spectrum())
+    kern = api.Kernel(ctx, phantoms.synthetic_kernel(n_phi=n_phi))
+    b = np.zeros((), BEAM_DTYPE)
+    b["isocenter"] = ph.centre()
+    b["beamlet_size"] = (0.23, 0.31)
+    b["fmap_size"] = (side, side)
+    b["sad"] = 100.0
+    b["angles"] = (1.1, 0.4, 0.2)
+    b["long_spacing"] = 0.25
+    b = api.calc_range(b, ph.volume)
+    fl = torch.rand(side * side, device="cuda", generator=torch.Generator(device="cuda").manual_seed(side))
+    doses = []
+    for n in (1, 24):
+        batch = api.BEVBatch(np.array([b] * n, BEAM_DTYPE))
+        api.TermaComputeCollective(ctx, batch, fl, dens, spec)
+        api.DoseComputeCollective(ctx, batch, kern)
+        doses += [batch.get("dose", 0).clone(), batch.get("dose", n - 1).clone()]
+    torch.cuda.synchronize()
+    assert float(doses[0].max()) > 0
+    for d in doses[1:]:
+        assert torch.equal(doses[0], d)
