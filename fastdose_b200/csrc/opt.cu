@@ -23,8 +23,6 @@
 #include <type_traits>
 #include <vector>
 
-#include <cub/block/block_reduce.cuh>
-
 #include "opt_internal.cuh"
 
 namespace fd2 {
@@ -39,26 +37,85 @@ constexpr float kEps = 1e-4f;  // eps_fastdose, FastDoseLib/include/macros.h:21
 // slots of the reduced scalars
 enum Slot { S_G = 0, S_GY = 1, S_GX = 2, S_DXY = 3, S_NXY = 4, S_TERMS = 8, S_COUNT = 16 };
 
+// Sums of K values over the block, in a fixed order; valid in thread 0.
 template <int K>
-__device__ __forceinline__ void block_partials(double (&v)[K], double* __restrict__ part) {
-    typedef cub::BlockReduce<double, kRedThreads> R;
-    __shared__ typename R::TempStorage tmp;
+__device__ __forceinline__ void block_sums(double (&v)[K]) {
+    __shared__ double s_part[kRedThreads / 32][K];
 #pragma unroll
-    for (int q = 0; q < K; q++) {
-        const double s = R(tmp).Sum(v[q]);
-        if (threadIdx.x == 0) part[(size_t)blockIdx.x * K + q] = s;
-        __syncthreads();
-    }
+    for (int q = 0; q < K; q++)
+#pragma unroll
+        for (int o = 16; o; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int q = 0; q < K; q++) s_part[threadIdx.x >> 5][q] = v[q];
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            v[q] = s_part[0][q];
+            for (int w = 1; w < kRedThreads / 32; w++) v[q] += s_part[w][q];
+        }
+    __syncthreads();  // s_part may be used again
 }
+
+// Sums of K values over the grid: the blocks' partial sums in block order, by
+// the last block to finish.  True in that block, whose thread 0 then holds the
+// sums in v; *done counts the blocks and is left at zero.
+template <int K>
+__device__ __forceinline__ bool grid_sums(double (&v)[K], double* __restrict__ part, unsigned* __restrict__ done) {
+    __shared__ bool s_last;
+    block_sums<K>(v);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < K; q++) part[(size_t)blockIdx.x * K + q] = v[q];
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < K; q++) v[q] = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kRedThreads)
+#pragma unroll
+        for (int q = 0; q < K; q++) v[q] += __ldcg(part + (size_t)b * K + q);
+    block_sums<K>(v);
+    if (threadIdx.x == 0) *done = 0u;
+    return true;
+}
+
+__device__ __forceinline__ double objective_of(const double* terms, float gamma, float eta) {
+    return 0.5 * (terms[0] + terms[1] + terms[2]) + (double)eta * (terms[3] + 0.5 / (double)gamma * terms[4]);
+}
+
+// What the host reads after a call: the reduced scalars and the group norms,
+// copied to pinned memory by the kernel that completes them (h_red null: not
+// yet).  One kernel of a trial writes host memory, which delays its end.
+struct Publish {
+    const double* red;
+    double* h_red;
+    const float* nrm;
+    float* h_nrm;
+    int64_t n_groups;
+    __device__ __forceinline__ void operator()() const {  // by a whole block
+        if (!h_red) return;
+        __syncthreads();
+        for (int i = threadIdx.x; i < S_COUNT; i += blockDim.x) h_red[i] = __ldcg(red + i);
+        for (int64_t i = threadIdx.x; i < n_groups; i += blockDim.x) h_nrm[i] = __ldcg(nrm + i);
+    }
+};
 
 // Objective terms over the VOI rows (s1, s2, s3) and the D rows (s4, s5);
 // optionally the gradient inputs g1 [nv] and g2 [m] (FP32, as the reference's
-// d_calc_grad_term1_input / d_calc_grad_term2_input).
+// d_calc_grad_term1_input / d_calc_grad_term2_input).  The last block sums the
+// terms into terms_out and, unless they are still to be summed over ranks, the
+// objective's value into out, and publishes the results.
 __global__ void __launch_bounds__(kRedThreads) objective_terms(
     const float* __restrict__ Ax, const float* __restrict__ Dx, int64_t n_ptv, int64_t nv, int64_t m,
     const float* __restrict__ max_dose, const float* __restrict__ max_w, const float* __restrict__ min_dose,
     const float* __restrict__ min_w, const float* __restrict__ oar_w, float gamma, float eta,
-    float* __restrict__ g1, float* __restrict__ g2, double* __restrict__ part) {
+    float* __restrict__ g1, float* __restrict__ g2, double* __restrict__ part, unsigned* __restrict__ done,
+    double* __restrict__ terms_out, double* out, Publish publish) {
     double s[kTerms] = {0, 0, 0, 0, 0};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nv; i += stride) {
@@ -93,30 +150,20 @@ __global__ void __launch_bounds__(kRedThreads) objective_terms(
             g2[i] = __fmul_rn(__fsub_rn(t4, pr4), eg);
         }
     }
-    block_partials<kTerms>(s, part);
-}
-
-// Sums the per-block partials of K terms in block order.
-template <int K>
-__global__ void __launch_bounds__(kRedThreads) finish_sums(const double* __restrict__ part, int n_blocks,
-                                                           double* __restrict__ out) {
-    typedef cub::BlockReduce<double, kRedThreads> R;
-    __shared__ typename R::TempStorage tmp;
-    for (int q = 0; q < K; q++) {
-        double s = 0;
-        for (int b = threadIdx.x; b < n_blocks; b += kRedThreads) s += part[(size_t)b * K + q];
-        s = R(tmp).Sum(s);
-        if (threadIdx.x == 0) out[q] = s;
-        __syncthreads();
+    if (grid_sums<kTerms>(s, part, done)) {
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int q = 0; q < kTerms; q++) terms_out[q] = s[q];
+            if (out) *out = objective_of(s, gamma, eta);
+        }
+        publish();
     }
 }
 
-// objective value from the five terms into out[slot]
-__global__ void objective_value(const double* __restrict__ terms, float gamma, float eta, double* __restrict__ out,
-                                int slot) {
-    if (threadIdx.x == 0 && blockIdx.x == 0)
-        out[slot] = 0.5 * (terms[0] + terms[1] + terms[2]) +
-                    (double)eta * (terms[3] + 0.5 / (double)gamma * terms[4]);
+// objective value from terms summed over the ranks
+__global__ void objective_value(const double* terms, float gamma, float eta, double* out, Publish publish) {
+    if (threadIdx.x == 0) *out = objective_of(terms, gamma, eta);
+    publish();
 }
 
 __global__ void add_vectors(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
@@ -125,13 +172,19 @@ __global__ void add_vectors(const float* __restrict__ a, const float* __restrict
         out[i] = __fadd_rn(a[i], b[i]);  // d_elementWiseAdd
 }
 
-// y = (1 - theta) x + theta v when step[2] != 0, else y = x; theta = step[0]
-// (the trial's scalars come from device memory, so one captured graph serves
-// every trial)
-__global__ void extrapolate(const float* __restrict__ x, const float* __restrict__ v, const float* __restrict__ step,
+// A trial's scalars: theta and t of the step, and whether y is extrapolated.
+struct Step {
+    float theta, t;
+    int extrapolated;
+};
+
+// y = (1 - theta) x + theta v when extrapolated, else y = x; t is left in device
+// memory for the kernels after this one.
+__global__ void extrapolate(const float* __restrict__ x, const float* __restrict__ v, Step step, float* __restrict__ d_t,
                             float* __restrict__ y, int64_t n) {
-    const float theta = step[0], a = 1.0f - theta;
-    const bool ex = step[2] != 0.0f;
+    const float theta = step.theta, a = 1.0f - theta;
+    const bool ex = step.extrapolated != 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *d_t = step.t;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = ex ? __fadd_rn(__fmul_rn(a, x[i]), __fmul_rn(theta, v[i])) : x[i];
 }
@@ -147,12 +200,15 @@ __global__ void momentum(const float* __restrict__ x, float iot, float* __restri
     }
 }
 
-// x = max(y - t g, 0)   (the polish projection), t = *t_dev
-__global__ void project_step(const float* __restrict__ y, const float* __restrict__ g, const float* __restrict__ t_dev,
-                             float* __restrict__ x, int64_t n) {
+// g = o1 + o2, x = max(y - t g, 0)   (the polish projection), t = *t_dev
+__global__ void project_step(const float* __restrict__ y, const float* __restrict__ o1, const float* __restrict__ o2,
+                             const float* __restrict__ t_dev, float* __restrict__ g, float* __restrict__ x, int64_t n) {
     const float t = *t_dev;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] = fmaxf(__fadd_rn(y[i], __fmul_rn(-t, g[i])), 0.0f);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float gi = __fadd_rn(o1[i], o2[i]);
+        g[i] = gi;
+        x[i] = fmaxf(__fadd_rn(y[i], __fmul_rn(-t, gi)), 0.0f);
+    }
 }
 
 // d_proxL2Onehalf_calc_tHat (IMRTOptimize_var1.cu:544-570) in FP32, the
@@ -168,50 +224,57 @@ __device__ __forceinline__ float t_hat(float nrm2, float tau) {
     return s * s;
 }
 
-// One block per group: in = max(y - t g, 0) (or y itself when g is null),
-// prox = tHat(||in||^2, tau) in, nrm = ||prox||, with FP64 norm sums.
-// tau = tau[r] when given, else w[r] * t; t = *t_dev when t_dev is given.
+// One block per group: in = max(y - t g, 0) with g = o1 + o2, kept in g (or y
+// itself when o1 is null), prox = tHat(||in||^2, tau) in, nrm = ||prox||, with
+// FP64 norm sums.  tau = tau[r] when given, else w[r] * t, t = *t_dev.
 __global__ void __launch_bounds__(kRedThreads) group_prox(const int64_t* __restrict__ go, const float* __restrict__ y,
-                                                          const float* __restrict__ g, float t,
-                                                          const float* __restrict__ t_dev,
+                                                          const float* __restrict__ o1, const float* __restrict__ o2,
+                                                          float* __restrict__ g, const float* __restrict__ t_dev,
                                                           const float* __restrict__ w, const float* __restrict__ tau,
                                                           float* __restrict__ x, float* __restrict__ nrm) {
-    if (t_dev) t = *t_dev;
-    typedef cub::BlockReduce<double, kRedThreads> R;
-    __shared__ typename R::TempStorage tmp;
+    const float t = t_dev ? *t_dev : 0.0f;
     __shared__ float s_th;
     const int64_t r = blockIdx.x, a = go[r], b = go[r + 1];
-    double n2 = 0;
+    double n2[1] = {0};
     for (int64_t i = a + threadIdx.x; i < b; i += kRedThreads) {
-        const float in = g ? fmaxf(__fadd_rn(y[i], __fmul_rn(-t, g[i])), 0.0f) : y[i];
-        n2 += (double)in * in;
+        float in = y[i];
+        if (o1) {
+            const float gi = __fadd_rn(o1[i], o2[i]);
+            g[i] = gi;
+            in = fmaxf(__fadd_rn(in, __fmul_rn(-t, gi)), 0.0f);
+        }
+        x[i] = in;
+        n2[0] += (double)in * in;
     }
-    n2 = R(tmp).Sum(n2);
-    if (threadIdx.x == 0) s_th = t_hat((float)n2, tau ? tau[r] : __fmul_rn(w[r], t));
+    block_sums<1>(n2);
+    if (threadIdx.x == 0) s_th = t_hat((float)n2[0], tau ? tau[r] : __fmul_rn(w[r], t));
     __syncthreads();
     const float th = s_th;
-    double m2 = 0;
-    for (int64_t i = a + threadIdx.x; i < b; i += kRedThreads) {
-        const float in = g ? fmaxf(__fadd_rn(y[i], __fmul_rn(-t, g[i])), 0.0f) : y[i];
-        const float p = __fmul_rn(th, in);
+    double m2[1] = {0};
+    for (int64_t i = a + threadIdx.x; i < b; i += kRedThreads) {  // the same thread wrote x[i]
+        const float p = __fmul_rn(th, x[i]);
         x[i] = p;
-        m2 += (double)p * p;
+        m2[0] += (double)p * p;
     }
-    m2 = R(tmp).Sum(m2);
-    if (threadIdx.x == 0) nrm[r] = sqrtf((float)m2);
+    block_sums<1>(m2);
+    if (threadIdx.x == 0) nrm[r] = sqrtf((float)m2[0]);
 }
 
 // line-search terms: sum g (x - y), sum (x - y)^2
 __global__ void __launch_bounds__(kRedThreads) step_terms(const float* __restrict__ g, const float* __restrict__ x,
                                                           const float* __restrict__ y, int64_t n,
-                                                          double* __restrict__ part) {
+                                                          double* __restrict__ part, unsigned* __restrict__ done,
+                                                          double* __restrict__ out) {
     double s[2] = {0, 0};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float d = __fsub_rn(x[i], y[i]);
         s[0] += (double)g[i] * d;
         s[1] += (double)d * d;
     }
-    block_partials<2>(s, part);
+    if (grid_sums<2>(s, part, done) && threadIdx.x == 0) {
+        out[0] = s[0];
+        out[1] = s[1];
+    }
 }
 
 template <typename T>
@@ -239,6 +302,10 @@ __global__ void ptv_column_sums(const int64_t* __restrict__ off, ColView col,
     if (lane == 0) out[r] = s * (row_scale ? (double)row_scale[r] : 1.0);
 }
 
+// blocks of a reduction over n elements: a fixed shape for a size
+unsigned red_blocks(int64_t n) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + kRedThreads - 1) / kRedThreads, kRedBlocks));
+}
 unsigned vec_blocks(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8)); }
 
 }  // namespace
@@ -252,12 +319,16 @@ struct fd2_opt_problem {
     float *d_max_dose = nullptr, *d_max_w = nullptr, *d_min_dose = nullptr, *d_min_w = nullptr, *d_oar_w = nullptr;
     float *d_Ax = nullptr, *d_Dx = nullptr, *d_g1 = nullptr, *d_g2 = nullptr, *d_o1 = nullptr, *d_o2 = nullptr;
     float *d_y = nullptr, *d_g = nullptr, *d_x = nullptr;
-    double *d_part = nullptr, *d_red = nullptr;
+    double *d_part = nullptr, *d_part2 = nullptr, *d_red = nullptr;
+    unsigned* d_done = nullptr;  // [2] block counters of the two reductions
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     double* h_red = nullptr;  // pinned [S_COUNT]
-    // the trial's scalars (theta, t, extrapolated) in pinned host memory and
-    // on the device, and the trial captured as a CUDA graph
-    float* h_step = nullptr;  // pinned [4]
-    float* d_step = nullptr;  // [4]
+    // the trial's step size on the device, and the trial captured as a CUDA graph,
+    // whose extrapolate node takes the trial's scalars as its argument
+    float* d_t = nullptr;
+    fd2::Step step{};
+    cudaGraph_t trial_graph = nullptr;
+    cudaGraphNode_t step_node = nullptr;
     bool use_graph = true;
     // row-sharded problems: the caller's sum over ranks of a device FP64 buffer
     fd2_reduce_fn reducer = nullptr;
@@ -318,43 +389,63 @@ int reduce_partials(fd2_opt_problem* p, bool with_grad) {
     return FD2_OK;
 }
 
-// objective of x into d_red[slot]; with grad: the gradient into grad
-int objective(fd2_opt_problem* p, const float* x, float* grad, int slot) {
-    cudaStream_t st = p->ctx->stream;
-    FD2_TRY(matrix_spmv(p->A, x, p->d_Ax, st));
-    if (p->m) FD2_TRY(matrix_spmv(p->D, x, p->d_Dx, st));
-    objective_terms<<<kRedBlocks, kRedThreads, 0, st>>>(p->d_Ax, p->d_Dx, p->n_ptv, p->nv, p->m, p->d_max_dose,
-                                                        p->d_max_w, p->d_min_dose, p->d_min_w, p->d_oar_w, p->gamma,
-                                                        p->eta, grad ? p->d_g1 : nullptr, grad ? p->d_g2 : nullptr,
-                                                        p->d_part);
-    finish_sums<kTerms><<<1, kRedThreads, 0, st>>>(p->d_part, kRedBlocks, p->d_red + S_TERMS);
-    FD2_CHECK_CUDA(cudaGetLastError());
-    p->ctx->launches += 2;
-    if (grad) {
-        if (p->m) {
-            FD2_TRY(matrix_spmv(p->DT, p->d_g2, p->d_o2, st));
-        } else {
-            FD2_CHECK_CUDA(cudaMemsetAsync(p->d_o2, 0, p->n * sizeof(float), st));
-        }
-        FD2_TRY(matrix_spmv(p->AT, p->d_g1, p->d_o1, st));
-    }
-    if (p->reducer) FD2_TRY(reduce_partials(p, grad != nullptr));
-    objective_value<<<1, 32, 0, st>>>(p->d_red + S_TERMS, p->gamma, p->eta, p->d_red, slot);
-    p->ctx->launches += 1;
-    if (grad) {
-        add_vectors<<<vec_blocks(p->n), 256, 0, st>>>(p->d_o1, p->d_o2, grad, p->n);
-        p->ctx->launches += 1;
-    }
-    FD2_CHECK_CUDA(cudaGetLastError());
+// The context's second stream, for the small fluence-gradient products beside
+// the VOI ones: forked from and joined to the work stream by events.
+int fork_side(fd2_opt_problem* p, cudaStream_t* side) {
+    fd2_context* c = p->ctx;
+    if (!c->aux_stream) FD2_CHECK_CUDA(cudaStreamCreateWithFlags(&c->aux_stream, cudaStreamNonBlocking));
+    FD2_CHECK_CUDA(cudaEventRecord(p->ev_fork, c->stream));
+    FD2_CHECK_CUDA(cudaStreamWaitEvent(c->aux_stream, p->ev_fork, 0));
+    *side = c->aux_stream;
+    return FD2_OK;
+}
+int join_side(fd2_opt_problem* p) {
+    FD2_CHECK_CUDA(cudaEventRecord(p->ev_join, p->ctx->aux_stream));
+    FD2_CHECK_CUDA(cudaStreamWaitEvent(p->ctx->stream, p->ev_join, 0));
     return FD2_OK;
 }
 
-int read_scalars(fd2_opt_problem* p, int64_t n_groups) {
-    cudaStream_t st = p->ctx->stream;
-    FD2_CHECK_CUDA(cudaMemcpyAsync(p->h_red, p->d_red, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (n_groups > 0)
-        FD2_CHECK_CUDA(cudaMemcpyAsync(p->h_nrm, p->d_nrm, n_groups * sizeof(float), cudaMemcpyDeviceToHost, st));
-    FD2_CHECK_CUDA(cudaStreamSynchronize(st));
+// objective of x into d_red[slot]; with_grad: the gradient's two parts into
+// d_o1 and d_o2; step: the line-search terms of d_x, d_y and d_g too.  The D
+// products and the line-search terms run beside the A products.  n_groups >= 0:
+// the results, with that many group norms, go to the host.
+int objective(fd2_opt_problem* p, const float* x, bool with_grad, int slot, int64_t n_groups, bool step = false) {
+    cudaStream_t st = p->ctx->stream, side = st;
+    const bool fork = p->m > 0 || step;
+    if (fork) FD2_TRY(fork_side(p, &side));
+    FD2_TRY(matrix_spmv(p->A, x, p->d_Ax, st));
+    if (p->m) FD2_TRY(matrix_spmv(p->D, x, p->d_Dx, side));
+    if (step) {
+        step_terms<<<red_blocks(p->n), kRedThreads, 0, side>>>(p->d_g, p->d_x, p->d_y, p->n, p->d_part2, p->d_done + 1,
+                                                              p->d_red + S_DXY);
+        FD2_CHECK_CUDA(cudaGetLastError());
+        p->ctx->launches += 1;
+    }
+    if (fork) FD2_TRY(join_side(p));
+    const Publish publish{p->d_red, n_groups >= 0 ? p->h_red : nullptr, p->d_nrm, p->h_nrm, n_groups};
+    const Publish later{};
+    objective_terms<<<red_blocks(std::max(p->nv, p->m)), kRedThreads, 0, st>>>(
+        p->d_Ax, p->d_Dx, p->n_ptv, p->nv, p->m, p->d_max_dose, p->d_max_w, p->d_min_dose, p->d_min_w, p->d_oar_w,
+        p->gamma, p->eta, with_grad ? p->d_g1 : nullptr, with_grad ? p->d_g2 : nullptr, p->d_part, p->d_done,
+        p->d_red + S_TERMS, p->reducer ? nullptr : p->d_red + slot, p->reducer ? later : publish);
+    FD2_CHECK_CUDA(cudaGetLastError());
+    p->ctx->launches += 1;
+    if (with_grad) {
+        if (p->m) FD2_TRY(fork_side(p, &side));
+        FD2_TRY(matrix_spmv(p->AT, p->d_g1, p->d_o1, st));
+        if (p->m) {
+            FD2_TRY(matrix_spmv(p->DT, p->d_g2, p->d_o2, side));
+            FD2_TRY(join_side(p));
+        } else {
+            FD2_CHECK_CUDA(cudaMemsetAsync(p->d_o2, 0, p->n * sizeof(float), st));
+        }
+    }
+    if (p->reducer) {
+        FD2_TRY(reduce_partials(p, with_grad));
+        objective_value<<<1, 128, 0, st>>>(p->d_red + S_TERMS, p->gamma, p->eta, p->d_red + slot, publish);
+        FD2_CHECK_CUDA(cudaGetLastError());
+        p->ctx->launches += 1;
+    }
     return FD2_OK;
 }
 
@@ -376,38 +467,39 @@ int ensure_groups(fd2_opt_problem* p, int64_t n_groups) {
 // One line-search trial at step t: y from (theta, xkm1, vkm1); x = prox or
 // projection of y - t grad g(y); leaves gx, gy, <grad, x - y>, ||x - y||^2 in h_red.
 // The work of one trial, enqueued on the context's stream without a host
-// wait: the scalars' upload, the products and reductions, the read-back of
-// the four scalars and the group norms into pinned memory.
+// wait; the last kernel leaves the four results and the group norms in pinned
+// memory.  On a problem of a few million
+// nonzeros a trial is a chain of short kernels, so their number counts: the
+// products are one launch each, every sum is finished by the last block of the
+// kernel that starts it, the gradient's parts are added where they are used, and
+// the D products run beside the A products.  20 steps on 48k x 1944 in 16 bits:
+// 3.8 ms with some 34 graph nodes a trial in a row, 2.5 ms with 14.
 int trial_enqueue(fd2_opt_problem* p, const fd2_opt_state_t* st, int64_t n_groups) {
     cudaStream_t s = p->ctx->stream;
     const int64_t n = p->n;
-    FD2_CHECK_CUDA(cudaMemcpyAsync(p->d_step, p->h_step, 4 * sizeof(float), cudaMemcpyHostToDevice, s));
-    extrapolate<<<vec_blocks(n), 256, 0, s>>>(st->d_xkm1, st->d_vkm1, p->d_step, p->d_y, n);
-    FD2_TRY(objective(p, p->d_y, p->d_g, S_GY));
+    extrapolate<<<vec_blocks(n), 256, 0, s>>>(st->d_xkm1, st->d_vkm1, p->step, p->d_t, p->d_y, n);
+    FD2_TRY(objective(p, p->d_y, true, S_GY, -1));
     if (n_groups > 0)
-        group_prox<<<(unsigned)n_groups, kRedThreads, 0, s>>>(p->d_go, p->d_y, p->d_g, 0.0f, p->d_step + 1, p->d_w,
+        group_prox<<<(unsigned)n_groups, kRedThreads, 0, s>>>(p->d_go, p->d_y, p->d_o1, p->d_o2, p->d_g, p->d_t, p->d_w,
                                                               nullptr, p->d_x, p->d_nrm);
     else
-        project_step<<<vec_blocks(n), 256, 0, s>>>(p->d_y, p->d_g, p->d_step + 1, p->d_x, n);
-    FD2_TRY(objective(p, p->d_x, nullptr, S_GX));
-    step_terms<<<kRedBlocks, kRedThreads, 0, s>>>(p->d_g, p->d_x, p->d_y, n, p->d_part);
-    finish_sums<2><<<1, kRedThreads, 0, s>>>(p->d_part, kRedBlocks, p->d_red + S_DXY);
+        project_step<<<vec_blocks(n), 256, 0, s>>>(p->d_y, p->d_o1, p->d_o2, p->d_t, p->d_g, p->d_x, n);
     FD2_CHECK_CUDA(cudaGetLastError());
-    p->ctx->launches += 5;
-    FD2_CHECK_CUDA(cudaMemcpyAsync(p->h_red, p->d_red, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
-    if (n_groups > 0)
-        FD2_CHECK_CUDA(cudaMemcpyAsync(p->h_nrm, p->d_nrm, n_groups * sizeof(float), cudaMemcpyDeviceToHost, s));
-    return FD2_OK;
+    p->ctx->launches += 2;
+    return objective(p, p->d_x, false, S_GX, n_groups, true);
 }
 
 void drop_graph(fd2_opt_problem* p) {
     if (p->trial_exec) cudaGraphExecDestroy(p->trial_exec);
+    if (p->trial_graph) cudaGraphDestroy(p->trial_graph);
     p->trial_exec = nullptr;
+    p->trial_graph = nullptr;
+    p->step_node = nullptr;
     p->graph_groups = -1;
 }
 
 // The trial's launches as one CUDA graph, captured for this state's vectors and
-// group count; replays read the scalars from p->h_step at execution.
+// group count; each replay sets the scalars of its extrapolate node.
 int capture_trial(fd2_opt_problem* p, const fd2_opt_state_t* st, int64_t n_groups) {
     drop_graph(p);
     cudaStream_t s = p->ctx->stream;
@@ -421,9 +513,22 @@ int capture_trial(fd2_opt_problem* p, const fd2_opt_state_t* st, int64_t n_group
         if (!rc) FD2_CHECK_CUDA(e);
         return rc;
     }
-    const cudaError_t ei = cudaGraphInstantiate(&p->trial_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    FD2_CHECK_CUDA(ei);
+    p->trial_graph = graph;
+    FD2_CHECK_CUDA(cudaGraphInstantiate(&p->trial_exec, graph, 0));
+    // the node that takes the trial's scalars
+    size_t n_nodes = 0;
+    FD2_CHECK_CUDA(cudaGraphGetNodes(graph, nullptr, &n_nodes));
+    std::vector<cudaGraphNode_t> nodes(n_nodes);
+    FD2_CHECK_CUDA(cudaGraphGetNodes(graph, nodes.data(), &n_nodes));
+    for (cudaGraphNode_t node : nodes) {
+        cudaGraphNodeType type;
+        cudaKernelNodeParams prm{};
+        FD2_CHECK_CUDA(cudaGraphNodeGetType(node, &type));
+        if (type != cudaGraphNodeTypeKernel) continue;
+        FD2_CHECK_CUDA(cudaGraphKernelNodeGetParams(node, &prm));
+        if (prm.func == (void*)extrapolate) p->step_node = node;
+    }
+    FD2_REQUIRE(p->step_node, FD2_ERR_CUDA, "optimizer: the captured trial has no extrapolate node");
     p->graph_xkm1 = st->d_xkm1;
     p->graph_vkm1 = st->d_vkm1;
     p->graph_groups = n_groups;
@@ -434,13 +539,20 @@ int capture_trial(fd2_opt_problem* p, const fd2_opt_state_t* st, int64_t n_group
 
 int trial(fd2_opt_problem* p, const fd2_opt_state_t* st, float theta, bool extrapolated, float t, int64_t n_groups) {
     cudaStream_t s = p->ctx->stream;
-    p->h_step[0] = theta;
-    p->h_step[1] = t;
-    p->h_step[2] = extrapolated ? 1.0f : 0.0f;
+    p->step = Step{theta, t, extrapolated ? 1 : 0};
     if (p->use_graph) {
         if (!p->trial_exec || p->graph_xkm1 != st->d_xkm1 || p->graph_vkm1 != st->d_vkm1 ||
             p->graph_groups != n_groups)
             FD2_TRY(capture_trial(p, st, n_groups));
+        const float *x = st->d_xkm1, *v = st->d_vkm1;
+        int64_t n = p->n;
+        void* args[] = {&x, &v, &p->step, &p->d_t, &p->d_y, &n};
+        cudaKernelNodeParams prm{};
+        prm.func = (void*)extrapolate;
+        prm.gridDim = dim3(vec_blocks(n));
+        prm.blockDim = dim3(256);
+        prm.kernelParams = args;
+        FD2_CHECK_CUDA(cudaGraphExecKernelNodeSetParams(p->trial_exec, p->step_node, &prm));
         FD2_CHECK_CUDA(cudaGraphLaunch(p->trial_exec, s));
         p->ctx->launches += p->graph_kernels;
     } else {
@@ -581,10 +693,14 @@ int fd2_opt_problem_create(fd2_context* ctx, const fd2_matrix* A, const fd2_matr
     for (const auto& q : bufs)
         if (!rc) rc = palloc(p, (void**)q.first, q.second * sizeof(float));
     if (!rc) rc = palloc(p, (void**)&p->d_part, (size_t)kRedBlocks * kTerms * sizeof(double));
+    if (!rc) rc = palloc(p, (void**)&p->d_part2, (size_t)kRedBlocks * 2 * sizeof(double));
+    if (!rc) rc = palloc(p, (void**)&p->d_done, 2 * sizeof(unsigned));
+    if (!rc && cudaMemsetAsync(p->d_done, 0, 2 * sizeof(unsigned), st) != cudaSuccess) rc = FD2_ERR_CUDA;
+    for (cudaEvent_t* ev : {&p->ev_fork, &p->ev_join})
+        if (!rc && cudaEventCreateWithFlags(ev, cudaEventDisableTiming) != cudaSuccess) rc = FD2_ERR_CUDA;
     if (!rc) rc = palloc(p, (void**)&p->d_red, S_COUNT * sizeof(double));
     if (!rc && cudaMallocHost(&p->h_red, S_COUNT * sizeof(double)) != cudaSuccess) rc = FD2_ERR_OUT_OF_MEMORY;
-    if (!rc && cudaMallocHost(&p->h_step, 4 * sizeof(float)) != cudaSuccess) rc = FD2_ERR_OUT_OF_MEMORY;
-    if (!rc) rc = palloc(p, (void**)&p->d_step, 4 * sizeof(float));
+    if (!rc) rc = palloc(p, (void**)&p->d_t, sizeof(float));
     if (!rc && cudaMemsetAsync(p->d_red, 0, S_COUNT * sizeof(double), st) != cudaSuccess) rc = FD2_ERR_CUDA;
     if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
     if (rc) {
@@ -600,8 +716,9 @@ int fd2_opt_problem_destroy(fd2_opt_problem* p) {
     drop_graph(p);
     for (void* q : p->owned) cudaFree(q);
     if (p->h_red) cudaFreeHost(p->h_red);
-    if (p->h_step) cudaFreeHost(p->h_step);
     if (p->h_nrm) cudaFreeHost(p->h_nrm);
+    for (cudaEvent_t ev : {p->ev_fork, p->ev_join})
+        if (ev) cudaEventDestroy(ev);
     delete p;
     return FD2_OK;
 }
@@ -627,16 +744,19 @@ int fd2_opt_problem_set_reducer(fd2_opt_problem* p, fd2_reduce_fn fn, void* user
 
 int fd2_eval_g(fd2_opt_problem* p, const float* d_x, double* h_value) {
     FD2_REQUIRE(p && d_x && h_value, FD2_ERR_INVALID_ARGUMENT, "eval_g: null argument");
-    FD2_TRY(objective(p, d_x, nullptr, S_G));
-    FD2_TRY(read_scalars(p, 0));
+    FD2_TRY(objective(p, d_x, false, S_G, 0));
+    FD2_CHECK_CUDA(cudaStreamSynchronize(p->ctx->stream));
     *h_value = p->h_red[S_G];
     return FD2_OK;
 }
 
 int fd2_eval_grad(fd2_opt_problem* p, const float* d_x, float* d_grad, double* h_value) {
     FD2_REQUIRE(p && d_x && d_grad && h_value, FD2_ERR_INVALID_ARGUMENT, "eval_grad: null argument");
-    FD2_TRY(objective(p, d_x, d_grad, S_G));
-    FD2_TRY(read_scalars(p, 0));
+    FD2_TRY(objective(p, d_x, true, S_G, 0));
+    add_vectors<<<vec_blocks(p->n), 256, 0, p->ctx->stream>>>(p->d_o1, p->d_o2, d_grad, p->n);
+    FD2_CHECK_CUDA(cudaGetLastError());
+    p->ctx->launches += 1;
+    FD2_CHECK_CUDA(cudaStreamSynchronize(p->ctx->stream));
     *h_value = p->h_red[S_G];
     return FD2_OK;
 }
@@ -646,8 +766,8 @@ int fd2_prox_l2onehalf(fd2_context* ctx, int64_t n_groups, const int64_t* d_go, 
     FD2_REQUIRE(ctx && d_go && d_g0 && d_tau && d_prox && d_nrm, FD2_ERR_INVALID_ARGUMENT,
                 "prox_l2onehalf: null argument");
     if (n_groups <= 0) return FD2_OK;
-    group_prox<<<(unsigned)n_groups, kRedThreads, 0, (cudaStream_t)stream>>>(d_go, d_g0, nullptr, 0.0f, nullptr,
-                                                                             nullptr, d_tau, d_prox, d_nrm);
+    group_prox<<<(unsigned)n_groups, kRedThreads, 0, (cudaStream_t)stream>>>(
+        d_go, d_g0, nullptr, nullptr, nullptr, nullptr, nullptr, d_tau, d_prox, d_nrm);
     FD2_CHECK_CUDA(cudaGetLastError());
     ctx->launches += 1;
     return FD2_OK;

@@ -80,6 +80,8 @@ struct fd2_matrix {
     int64_t* d_carry_row = nullptr;  // [n_ranges] row open at each range's end
     float* d_carry_val = nullptr;    // [n_ranges] its partial sum
     float* d_xs = nullptr;           // [cols] x times the column scale
+    int32_t* d_zrow = nullptr;       // rows the product itself does not write: empty, or only in carries
+    int* d_nz = nullptr;             // number of those rows
 
     fd2::ColView cols_view() const { return fd2::ColView{d_col, d_col16, d_cbase, d_exc, interleaved}; }
 };

@@ -21,8 +21,9 @@
 //    with x in global memory the chunk is interleaved (slot()), so that each
 //    x-gather of the warp covers 32 consecutive nonzeros, and the rare slices
 //    of 32 elements with row starts are scanned one by one;
-//  * the row open at the end of a warp's range is carried; a second kernel
-//    adds carries in warp order.
+//  * the row open at the end of a range is carried; a second kernel adds the
+//    carries in range order.  The rows that no range closes are listed with the
+//    matrix and set to zero by the product itself.
 //
 // Summation order depends only on the matrix and the launch shape, so products
 // are reproducible run to run.  A pass is HBM-bound: it reads nnz x (value +
@@ -66,6 +67,9 @@ struct StreamArgs {
     int64_t* carry_row;
     float* carry_val;
     int x_len;  // kSmemX: floats of x staged in shared memory
+    const float* col_scale;  // kSmemX: factor of each x, or null
+    const int32_t* zrow;
+    const int* n_zrow;
 };
 
 // A lane's share of one chunk as loaded, values and columns still packed, so
@@ -182,12 +186,17 @@ __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX
     spmv_stream_kernel(StreamArgs a, const float* __restrict__ x, float* __restrict__ y) {
     extern __shared__ float xs[];
     if constexpr (kSmemX) {
-        for (int i = threadIdx.x; i < a.x_len; i += blockDim.x) xs[i] = __ldg(x + i);
+        if (a.col_scale)
+            for (int i = threadIdx.x; i < a.x_len; i += blockDim.x) xs[i] = __ldg(a.col_scale + i) * __ldg(x + i);
+        else
+            for (int i = threadIdx.x; i < a.x_len; i += blockDim.x) xs[i] = __ldg(x + i);
         __syncthreads();
     }
+    // rows no range closes start at zero
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < __ldg(a.n_zrow); i += gridDim.x * blockDim.x)
+        y[__ldg(a.zrow + i)] = 0.0f;
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    if (w >= a.n_warps) return;  // uniform per warp
     float oacc = 0.0f, open = 0.0f;  // the open row (the row in progress): this lane's share, and (!kInter) its sum so far
     bool shares = false;      // !kInter: some lane's share is not zero
     bool open_valid = false;  // the range has met an element of the open row
@@ -351,7 +360,7 @@ __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX
             open_valid = true;
         }
     };
-    for (int range = w; range < a.n_ranges; range += a.n_warps) {
+    for (int range = w < a.n_warps ? w : a.n_ranges; range < a.n_ranges; range += a.n_warps) {
         const int64_t c0 = (int64_t)range * a.n_chunks / a.n_ranges, c1 = (int64_t)(range + 1) * a.n_chunks / a.n_ranges;
         oacc = open = 0.0f;
         shares = open_valid = false;
@@ -400,7 +409,8 @@ __global__ void __launch_bounds__(kSmemX ? kSmemThreads : kStreamThreads, kSmemX
 }
 
 // Adds the carries of rows that cross ranges: the first range of each run of
-// equal carry rows sums the run in range order.
+// equal carry rows sums the run in range order.  A launch of its own: done by the
+// product's last block, one block's walk over some 5000 to 19000 carries took 20 us.
 __global__ void spmv_fixup_kernel(int n_ranges, const int64_t* __restrict__ carry_row,
                                   const float* __restrict__ carry_val, const float* __restrict__ row_scale,
                                   int64_t rows, float* __restrict__ y) {
@@ -516,6 +526,22 @@ __global__ void pack_columns(const int32_t* __restrict__ col, int64_t nnz, int64
         } else {
             col16[q] = (uint16_t)(k < nnz ? cv - base[c] : 0);
         }
+    }
+}
+
+// Rows that the product's ranges do not write: empty ones, and those that end
+// where a range does (the next row starts the next range, or the matrix ends),
+// whose sum is only in carries.  In any order: they are set to zero.
+__global__ void list_unwritten_rows(const int64_t* __restrict__ off, int64_t rows, int64_t nnz, int64_t n_chunks,
+                                    int64_t n_ranges, int32_t* __restrict__ zrow, int* __restrict__ count) {
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t end = off[r + 1];
+        bool un = off[r] == end || end == nnz;
+        if (!un && end % kChunk == 0) {
+            const int64_t c = end / kChunk, range = (c * n_ranges + n_chunks - 1) / n_chunks;
+            un = range < n_ranges && range * n_chunks / n_ranges == c;
+        }
+        if (un) zrow[atomicAdd(count, 1)] = (int32_t)r;
     }
 }
 
@@ -668,13 +694,14 @@ int launch_stream(const fd2_matrix* m, const float* x, float* y, cudaStream_t st
     StreamArgs a{m->d_val, m->cols_view(), m->d_head, m->d_chunk_h, m->d_chunk_row0, m->d_nzrow,
                  m->scale_axis == FD2_SCALE_ROWS ? m->d_scale : nullptr, m->n_chunks, m->n_warps,
                  m->n_ranges, m->rows,
-                 m->d_carry_row, m->d_carry_val, (int)m->cols};
+                 m->d_carry_row, m->d_carry_val, (int)m->cols,
+                 m->scale_axis == FD2_SCALE_COLS && m->x_in_smem ? m->d_scale : nullptr, m->d_zrow, m->d_nz};
     if (m->index_format == FD2_INDEX_PACKED16)
         FD2_TRY((launch_stream_fmt<T, true>(m, a, x, y, st)));
     else
         FD2_TRY((launch_stream_fmt<T, false>(m, a, x, y, st)));
-    spmv_fixup_kernel<<<(m->n_ranges + 255) / 256, 256, 0, st>>>(m->n_ranges, m->d_carry_row, m->d_carry_val,
-                                                               a.row_scale, m->rows, y);
+    spmv_fixup_kernel<<<(m->n_ranges + 127) / 128, 128, 0, st>>>(m->n_ranges, m->d_carry_row, m->d_carry_val,
+                                                                 a.row_scale, m->rows, y);
     FD2_CHECK_CUDA(cudaGetLastError());
     return FD2_OK;
 }
@@ -748,7 +775,7 @@ int matrix_alloc_entries(fd2_matrix* m, cudaStream_t st) {
 void matrix_free(fd2_matrix* m) {
     for (void* p : {(void*)m->d_off, (void*)m->d_col, (void*)m->d_col16, (void*)m->d_cbase, (void*)m->d_exc, m->d_val,
                     (void*)m->d_scale, (void*)m->d_head, (void*)m->d_chunk_h, (void*)m->d_chunk_row0, (void*)m->d_nzrow,
-                    (void*)m->d_carry_row, (void*)m->d_carry_val, (void*)m->d_xs})
+                    (void*)m->d_carry_row, (void*)m->d_carry_val, (void*)m->d_xs, (void*)m->d_zrow, (void*)m->d_nz})
         if (p) cudaFree(p);
     m->d_off = nullptr;
     m->d_col = nullptr;
@@ -760,6 +787,8 @@ void matrix_free(fd2_matrix* m) {
     m->d_chunk_h = m->d_chunk_row0 = m->d_nzrow = nullptr;
     m->d_carry_row = nullptr;
     m->d_carry_val = m->d_xs = nullptr;
+    m->d_zrow = nullptr;
+    m->d_nz = nullptr;
 }
 
 // Warps of one full wave of the stream kernel for this matrix's instance, so
@@ -821,7 +850,10 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     FD2_CHECK_CUDA(cudaMalloc(&m->d_chunk_row0, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t)));
     FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_row, m->n_ranges * sizeof(int64_t)));
     FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_val, m->n_ranges * sizeof(float)));
-    if (m->scale_axis == FD2_SCALE_COLS)
+    FD2_CHECK_CUDA(cudaMalloc(&m->d_zrow, std::max<int64_t>(m->rows, 1) * sizeof(int32_t)));
+    FD2_CHECK_CUDA(cudaMalloc(&m->d_nz, sizeof(int)));
+    FD2_CHECK_CUDA(cudaMemsetAsync(m->d_nz, 0, sizeof(int), st));
+    if (m->scale_axis == FD2_SCALE_COLS && !m->x_in_smem)
         FD2_CHECK_CUDA(cudaMalloc(&m->d_xs, std::max<int64_t>(m->cols, 1) * sizeof(float)));
     FD2_CHECK_CUDA(cudaMemsetAsync(m->d_head, 0, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t),
                                    st));
@@ -851,6 +883,9 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     m->n_nzrows = (int64_t)last_pos + last_ne;
     if (!rc && cudaMalloc(&m->d_nzrow, std::max<int64_t>(m->n_nzrows, 1) * sizeof(int32_t)) != cudaSuccess)
         rc = FD2_ERR_OUT_OF_MEMORY;
+    if (!rc && m->rows && m->n_chunks)
+        list_unwritten_rows<<<grid_for(m->rows), 256, 0, st>>>(m->d_off, m->rows, m->nnz, m->n_chunks, m->n_ranges, m->d_zrow,
+                                                              m->d_nz);
     if (!rc && m->rows) scatter_rows<<<grid_for(m->rows), 256, 0, st>>>(ne, pos, m->rows, m->d_nzrow);
     if (!rc && m->n_chunks) {
         chunk_head_counts<<<grid_for(m->n_chunks), 256, 0, st>>>(m->d_head, m->n_chunks, cnt);
@@ -938,9 +973,11 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
 
 int matrix_spmv(const fd2_matrix* m, const float* x, float* y, cudaStream_t st) {
     if (m->rows == 0) return FD2_OK;
-    FD2_CHECK_CUDA(cudaMemsetAsync(y, 0, m->rows * sizeof(float), st));  // empty rows, and rows only carries reach
-    if (m->n_chunks == 0) return FD2_OK;
-    if (m->scale_axis == FD2_SCALE_COLS) {
+    if (m->n_chunks == 0) {
+        FD2_CHECK_CUDA(cudaMemsetAsync(y, 0, m->rows * sizeof(float), st));
+        return FD2_OK;
+    }
+    if (m->scale_axis == FD2_SCALE_COLS && !m->x_in_smem) {
         scale_vector_kernel<<<grid_for(m->cols), 256, 0, st>>>(m->d_scale, x, m->d_xs, m->cols);
         FD2_CHECK_CUDA(cudaGetLastError());
         x = m->d_xs;
