@@ -41,13 +41,12 @@ void ctx_graphs_free(fd2_context* ctx) {
     }
 }
 
-// One pool per device for the densities of fd2_density_create: created on
-// first use and kept until the process ends, so a density may be freed after
-// the context it was made with; freed memory is kept for the next density.
-int density_pool(int device, cudaMemPool_t* out) {
+// One pool per device, created on first use and kept until the process ends, so
+// that what it holds may be freed after the context it was made with.  keep:
+// bytes of freed memory it holds on to.
+static int device_pool(cudaMemPool_t* pools, int device, uint64_t keep, const char* what, cudaMemPool_t* out) {
     static std::mutex mu;
-    static cudaMemPool_t pools[kMaxDevices] = {};
-    FD2_REQUIRE(device >= 0 && device < kMaxDevices, FD2_ERR_INVALID_ARGUMENT, "density pool: device %d", device);
+    FD2_REQUIRE(device >= 0 && device < kMaxDevices, FD2_ERR_INVALID_ARGUMENT, "%s pool: device %d", what, device);
     std::lock_guard<std::mutex> lock(mu);
     if (!pools[device]) {
         cudaMemPoolProps pp = {};
@@ -55,18 +54,28 @@ int density_pool(int device, cudaMemPool_t* out) {
         pp.handleTypes = cudaMemHandleTypeNone;
         pp.location.type = cudaMemLocationTypeDevice;
         pp.location.id = device;
-        const uint64_t keep = ~0ull;
         cudaMemPool_t p = nullptr;
         FD2_CHECK_CUDA(cudaMemPoolCreate(&p, &pp));
         if (cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, (void*)&keep) != cudaSuccess) {
             cudaMemPoolDestroy(p);
-            fd2::set_error("density pool: cannot set its release threshold");
+            fd2::set_error("%s pool: cannot set its release threshold", what);
             return FD2_ERR_CUDA;
         }
         pools[device] = p;
     }
     *out = pools[device];
     return FD2_OK;
+}
+
+// The densities of fd2_density_create: freed memory is kept for the next one.
+int density_pool(int device, cudaMemPool_t* out) {
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    return device_pool(pools, device, ~0ull, "density", out);
+}
+
+int matrix_pool(int device, cudaMemPool_t* out) {
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    return device_pool(pools, device, 1ull << 30, "matrix", out);
 }
 
 int density_create_pooled(fd2_context* ctx, const float* host_density, const fd2_volume_t* volume,
@@ -168,6 +177,9 @@ int fd2_context_release(fd2_context* c) {
     }
     FD2_CHECK_CUDA(cudaStreamSynchronize(c->stream));
     FD2_CHECK_CUDA(cudaMemPoolTrimTo(c->pool, 0));
+    cudaMemPool_t mats = nullptr;
+    FD2_TRY(fd2::matrix_pool(c->device, &mats));
+    FD2_CHECK_CUDA(cudaMemPoolTrimTo(mats, 0));
     return FD2_OK;
 }
 

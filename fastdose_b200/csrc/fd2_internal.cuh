@@ -163,6 +163,7 @@ inline int ctx_scratch(fd2_context* ctx, size_t bytes, cudaStream_t st, void** o
 // service worker's requests); the public fd2_density_create allocates plainly.
 constexpr int kMaxDevices = 64;
 int density_pool(int device, cudaMemPool_t* out);
+int matrix_pool(int device, cudaMemPool_t* out);  // optimizer matrices and problems
 int density_create_pooled(fd2_context* ctx, const float* host_density, const fd2_volume_t* volume,
                           fd2_density** out);
 

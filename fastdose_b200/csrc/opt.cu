@@ -350,7 +350,7 @@ namespace fd2 {
 namespace {
 
 int palloc(fd2_opt_problem* p, void** ptr, size_t bytes) {
-    FD2_CHECK_CUDA(cudaMalloc(ptr, std::max<size_t>(bytes, 16)));
+    FD2_CHECK_CUDA(mat_malloc(ptr, std::max<size_t>(bytes, 16), p->ctx->stream));
     p->owned.push_back(*ptr);
     return FD2_OK;
 }
@@ -714,7 +714,8 @@ int fd2_opt_problem_create(fd2_context* ctx, const fd2_matrix* A, const fd2_matr
 int fd2_opt_problem_destroy(fd2_opt_problem* p) {
     if (!p) return FD2_OK;
     drop_graph(p);
-    for (void* q : p->owned) cudaFree(q);
+    cudaDeviceSynchronize();  // a caller may still read what the problem wrote
+    for (void* q : p->owned) mat_free(q, nullptr);
     if (p->h_red) cudaFreeHost(p->h_red);
     if (p->h_nrm) cudaFreeHost(p->h_nrm);
     for (cudaEvent_t ev : {p->ev_fork, p->ev_join})
@@ -780,7 +781,7 @@ int fd2_beam_weights_init(fd2_opt_problem* p, int64_t n_groups, const int64_t* h
     const fd2_matrix* at = p->AT;
     cudaStream_t st = p->ctx->stream;
     double* d_s = nullptr;  // [rows] PTV sums, then this problem's PTV row count (summed over ranks)
-    FD2_CHECK_CUDA(cudaMalloc(&d_s, (at->rows + 1) * sizeof(double)));
+    FD2_CHECK_CUDA(mat_malloc(&d_s, (at->rows + 1) * sizeof(double), st));
     const float* rs = at->scale_axis == FD2_SCALE_ROWS ? at->d_scale : nullptr;
     const unsigned blocks = (unsigned)((at->rows * 32 + 255) / 256);
     if (at->rows) {
@@ -806,7 +807,7 @@ int fd2_beam_weights_init(fd2_opt_problem* p, int64_t n_groups, const int64_t* h
     if (e == cudaSuccess && p->reducer) {  // the PTV rows are spread over the ranks
         e = cudaStreamSynchronize(st);
         if (e == cudaSuccess && p->reducer(p->reducer_user, d_s, at->rows + 1, st) != 0) {
-            cudaFree(d_s);
+            mat_free(d_s, st);
             set_error("beam_weights_init: the rank reduction failed");
             return FD2_ERR_CUDA;
         }
@@ -814,7 +815,7 @@ int fd2_beam_weights_init(fd2_opt_problem* p, int64_t n_groups, const int64_t* h
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(s.data(), d_s, (at->rows + 1) * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_s);
+    mat_free(d_s, st);
     FD2_CHECK_CUDA(e);
     const double n_ptv = s[at->rows];  // all ranks' PTV rows
     FD2_REQUIRE(n_ptv > 0, FD2_ERR_INVALID_ARGUMENT, "beam_weights_init: no PTV rows");
@@ -880,10 +881,10 @@ int fd2_beam_orientation_optimization(fd2_context* ctx, const fd2_matrix* AT, co
     float *xb[2] = {nullptr, nullptr}, *vb[2] = {nullptr, nullptr};
     auto release = [&]() {
         for (float* q : {xb[0], xb[1], vb[0], vb[1]})
-            if (q) cudaFree(q);
+            mat_free(q, s);
     };
     for (float** q : {&xb[0], &xb[1], &vb[0], &vb[1]})
-        if (cudaMalloc(q, std::max<int64_t>(n_all, 1) * sizeof(float)) != cudaSuccess) {
+        if (mat_malloc(q, std::max<int64_t>(n_all, 1) * sizeof(float), s) != cudaSuccess) {
             release();
             set_error("beam_orientation_optimization: out of device memory");
             return FD2_ERR_OUT_OF_MEMORY;

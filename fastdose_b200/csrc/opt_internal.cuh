@@ -88,6 +88,19 @@ struct fd2_matrix {
 
 namespace fd2 {
 
+// Device memory of matrices and problems and of what builds them, in the order
+// of a stream, from a pool the library keeps per device (as densities are): a
+// matrix makes some thirty allocations, and cudaMalloc and cudaFree, which wait
+// for the device, took most of the time of the orientation loop's phases.  The
+// pool keeps at most 1 GiB of freed memory; fd2_context_release empties it.
+cudaError_t mat_malloc_bytes(void** p, size_t bytes, cudaStream_t stream);
+template <typename T>
+cudaError_t mat_malloc(T** p, size_t bytes, cudaStream_t stream) {
+    return mat_malloc_bytes((void**)p, bytes, stream);
+}
+// Returns memory whose last use is before this point of the stream.
+void mat_free(void* p, cudaStream_t stream);
+
 // Allocates d_off (rows + 1), d_col (int32, nnz padded to kChunk), d_val
 // (padded, zeroed past nnz) and d_scale for the sizes in m.
 int matrix_alloc(fd2_matrix* m, cudaStream_t stream);
@@ -97,6 +110,8 @@ int matrix_alloc_entries(fd2_matrix* m, cudaStream_t stream);
 // warp partition) from d_off, and packs the columns when m->index_format is
 // PACKED16.  Call once the offsets, columns and values are written.
 int matrix_finalize(fd2_matrix* m, cudaStream_t stream);
+// Frees what m holds, after all work of the device (a product may run on any
+// stream, and the matrix may outlive its context).
 void matrix_free(fd2_matrix* m);
 // Transpose into a matrix of the given index format.
 int matrix_transpose_fmt(const fd2_matrix* m, int index_format, fd2_matrix** out);

@@ -124,7 +124,7 @@ int matrix_select_blocks(const fd2_matrix* m, int64_t n_blocks, const int64_t* h
     int* d_bad = nullptr;
     auto dev = [&](void** p, const void* h, size_t bytes) {
         if (rc) return;
-        if (cudaMalloc(p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+        if (mat_malloc(p, std::max<size_t>(bytes, 16), st) != cudaSuccess) {
             rc = FD2_ERR_OUT_OF_MEMORY;
             return;
         }
@@ -182,7 +182,7 @@ int matrix_select_blocks(const fd2_matrix* m, int64_t n_blocks, const int64_t* h
                 cudaStreamSynchronize(st) != cudaSuccess))
         rc = FD2_ERR_CUDA;
     for (void* p : {(void*)d_map, (void*)d_mapc, (void*)d_shift, (void*)d_lo, (void*)d_hi, (void*)d_bad})
-        if (p) cudaFree(p);
+        mat_free(p, st);
     if (!rc && bad) {
         set_error("matrix_select_blocks: %d entries lie outside their column block (not block-diagonal)", bad);
         rc = FD2_ERR_INVALID_ARGUMENT;

@@ -565,10 +565,10 @@ int exclusive_scan(const T* in, T* out, int64_t n, cudaStream_t st) {
     size_t tb = 0;
     FD2_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, in, out, n, st));
     void* tmp = nullptr;
-    FD2_CHECK_CUDA(cudaMalloc(&tmp, std::max<size_t>(tb, 16)));
+    FD2_CHECK_CUDA(mat_malloc(&tmp, std::max<size_t>(tb, 16), st));
     cudaError_t e = cub::DeviceScan::ExclusiveSum(tmp, tb, in, out, n, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(tmp);
+    mat_free(tmp, st);
     FD2_CHECK_CUDA(e);
     return FD2_OK;
 }
@@ -716,17 +716,17 @@ int transpose_typed(const fd2_matrix* m, fd2_matrix* t, cudaStream_t st) {
     int end_bit = 1;
     while (end_bit < 31 && ((int64_t)1 << end_bit) < m->cols) end_bit++;
     int rc = FD2_OK;
-    cudaError_t e = cudaMalloc(&keys_in, nnz * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&keys_out, nnz * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&perm_in, nnz * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&perm_out, nnz * sizeof(int64_t));
+    cudaError_t e = mat_malloc(&keys_in, nnz * sizeof(int32_t), st);
+    if (e == cudaSuccess) e = mat_malloc(&keys_out, nnz * sizeof(int32_t), st);
+    if (e == cudaSuccess) e = mat_malloc(&perm_in, nnz * sizeof(int64_t), st);
+    if (e == cudaSuccess) e = mat_malloc(&perm_out, nnz * sizeof(int64_t), st);
     if (e == cudaSuccess) {
         unpack_entries<T><<<grid_for(nnz), 256, 0, st>>>(m->d_off, m->rows, m->cols_view(), (const T*)m->d_val,
                                                          nullptr, FD2_SCALE_NONE, nnz, keys_in, nullptr);
         e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys_in, keys_out, perm_in, perm_out, nnz, 0, end_bit,
                                             st);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, std::max<size_t>(tmp_bytes, 16));
+    if (e == cudaSuccess) e = mat_malloc(&tmp, std::max<size_t>(tmp_bytes, 16), st);
     if (e == cudaSuccess) {
         // stable sort by column: within a new row, entries keep ascending old-row order
         iota64<<<grid_for(nnz), 256, 0, st>>>(perm_in, nnz);
@@ -745,21 +745,34 @@ int transpose_typed(const fd2_matrix* m, fd2_matrix* t, cudaStream_t st) {
         rc = e == cudaErrorMemoryAllocation ? FD2_ERR_OUT_OF_MEMORY : FD2_ERR_CUDA;
     }
     for (void* p : {(void*)keys_in, (void*)keys_out, (void*)perm_in, (void*)perm_out, tmp})
-        if (p) cudaFree(p);
+        mat_free(p, st);
     return rc;
 }
 
 }  // namespace
 
+cudaError_t mat_malloc_bytes(void** p, size_t bytes, cudaStream_t stream) {
+    *p = nullptr;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    cudaMemPool_t pool = nullptr;
+    if (e == cudaSuccess && matrix_pool(device, &pool) != FD2_OK) e = cudaErrorMemoryAllocation;
+    return e == cudaSuccess ? cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, stream) : e;
+}
+
+void mat_free(void* p, cudaStream_t stream) {
+    if (p) cudaFreeAsync(p, stream);
+}
+
 int matrix_alloc(fd2_matrix* m, cudaStream_t st) {
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_off, (m->rows + 1) * sizeof(int64_t)));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_off, (m->rows + 1) * sizeof(int64_t), st));
     return matrix_alloc_entries(m, st);
 }
 
 int matrix_alloc_entries(fd2_matrix* m, cudaStream_t st) {
     const int64_t pad = round_chunk(m->nnz);
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_col, std::max<int64_t>(pad, 1) * sizeof(int32_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_val, std::max<int64_t>(pad, 1) * value_size(m->value_type)));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_col, std::max<int64_t>(pad, 1) * sizeof(int32_t), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_val, std::max<int64_t>(pad, 1) * value_size(m->value_type), st));
     if (pad > m->nnz) {  // the last chunk's padding: column 0, value 0
         FD2_CHECK_CUDA(cudaMemsetAsync(m->d_col + m->nnz, 0, (pad - m->nnz) * sizeof(int32_t), st));
         FD2_CHECK_CUDA(cudaMemsetAsync((char*)m->d_val + m->nnz * value_size(m->value_type), 0,
@@ -767,16 +780,17 @@ int matrix_alloc_entries(fd2_matrix* m, cudaStream_t st) {
     }
     if (m->scale_axis != FD2_SCALE_NONE) {
         const int64_t n = m->scale_axis == FD2_SCALE_ROWS ? m->rows : m->cols;
-        FD2_CHECK_CUDA(cudaMalloc(&m->d_scale, std::max<int64_t>(n, 1) * sizeof(float)));
+        FD2_CHECK_CUDA(mat_malloc(&m->d_scale, std::max<int64_t>(n, 1) * sizeof(float), st));
     }
     return FD2_OK;
 }
 
 void matrix_free(fd2_matrix* m) {
+    cudaDeviceSynchronize();
     for (void* p : {(void*)m->d_off, (void*)m->d_col, (void*)m->d_col16, (void*)m->d_cbase, (void*)m->d_exc, m->d_val,
                     (void*)m->d_scale, (void*)m->d_head, (void*)m->d_chunk_h, (void*)m->d_chunk_row0, (void*)m->d_nzrow,
                     (void*)m->d_carry_row, (void*)m->d_carry_val, (void*)m->d_xs, (void*)m->d_zrow, (void*)m->d_nz})
-        if (p) cudaFree(p);
+        mat_free(p, nullptr);
     m->d_off = nullptr;
     m->d_col = nullptr;
     m->d_col16 = nullptr;
@@ -845,28 +859,28 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     m->n_ranges = m->n_warps;
     if (!m->interleaved)
         m->n_ranges *= (int)std::max<int64_t>(1, std::min<int64_t>(kRangesPerWarp, m->n_chunks / ((int64_t)m->n_warps * kMinRange)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_head, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_chunk_h, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_chunk_row0, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_row, m->n_ranges * sizeof(int64_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_carry_val, m->n_ranges * sizeof(float)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_zrow, std::max<int64_t>(m->rows, 1) * sizeof(int32_t)));
-    FD2_CHECK_CUDA(cudaMalloc(&m->d_nz, sizeof(int)));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_head, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_chunk_h, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_chunk_row0, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_carry_row, m->n_ranges * sizeof(int64_t), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_carry_val, m->n_ranges * sizeof(float), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_zrow, std::max<int64_t>(m->rows, 1) * sizeof(int32_t), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_nz, sizeof(int), st));
     FD2_CHECK_CUDA(cudaMemsetAsync(m->d_nz, 0, sizeof(int), st));
     if (m->scale_axis == FD2_SCALE_COLS && !m->x_in_smem)
-        FD2_CHECK_CUDA(cudaMalloc(&m->d_xs, std::max<int64_t>(m->cols, 1) * sizeof(float)));
+        FD2_CHECK_CUDA(mat_malloc(&m->d_xs, std::max<int64_t>(m->cols, 1) * sizeof(float), st));
     FD2_CHECK_CUDA(cudaMemsetAsync(m->d_head, 0, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t),
                                    st));
     // row starts, non-empty rows, row starts before each chunk
     int32_t *ne = nullptr, *pos = nullptr, *cnt = nullptr;
     auto cleanup = [&]() {
         for (void* p : {(void*)ne, (void*)pos, (void*)cnt})
-            if (p) cudaFree(p);
+            mat_free(p, st);
     };
     const int64_t rows1 = std::max<int64_t>(m->rows, 1);
-    if (cudaMalloc(&ne, rows1 * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&pos, rows1 * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&cnt, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t)) != cudaSuccess) {
+    if (mat_malloc(&ne, rows1 * sizeof(int32_t), st) != cudaSuccess ||
+        mat_malloc(&pos, rows1 * sizeof(int32_t), st) != cudaSuccess ||
+        mat_malloc(&cnt, std::max<int64_t>(m->n_chunks, 1) * sizeof(int32_t), st) != cudaSuccess) {
         cleanup();
         set_error("matrix_finalize: out of device memory");
         return FD2_ERR_OUT_OF_MEMORY;
@@ -881,7 +895,7 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             rc = FD2_ERR_CUDA;
     }
     m->n_nzrows = (int64_t)last_pos + last_ne;
-    if (!rc && cudaMalloc(&m->d_nzrow, std::max<int64_t>(m->n_nzrows, 1) * sizeof(int32_t)) != cudaSuccess)
+    if (!rc && mat_malloc(&m->d_nzrow, std::max<int64_t>(m->n_nzrows, 1) * sizeof(int32_t), st) != cudaSuccess)
         rc = FD2_ERR_OUT_OF_MEMORY;
     if (!rc && m->rows && m->n_chunks)
         list_unwritten_rows<<<grid_for(m->rows), 256, 0, st>>>(m->d_off, m->rows, m->nnz, m->n_chunks, m->n_ranges, m->d_zrow,
@@ -898,10 +912,10 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     if (!rc && m->index_format == FD2_INDEX_PACKED16 && m->n_chunks) {
         int32_t *wide = ne, *eslot = pos;  // reuse when large enough
         bool own = m->n_chunks > rows1;
-        if (own && (cudaMalloc(&wide, m->n_chunks * sizeof(int32_t)) != cudaSuccess ||
-                    cudaMalloc(&eslot, m->n_chunks * sizeof(int32_t)) != cudaSuccess))
+        if (own && (mat_malloc(&wide, m->n_chunks * sizeof(int32_t), st) != cudaSuccess ||
+                    mat_malloc(&eslot, m->n_chunks * sizeof(int32_t), st) != cudaSuccess))
             rc = FD2_ERR_OUT_OF_MEMORY;
-        if (!rc && cudaMalloc(&m->d_cbase, m->n_chunks * sizeof(int32_t)) != cudaSuccess) rc = FD2_ERR_OUT_OF_MEMORY;
+        if (!rc && mat_malloc(&m->d_cbase, m->n_chunks * sizeof(int32_t), st) != cudaSuccess) rc = FD2_ERR_OUT_OF_MEMORY;
         if (!rc) {
             chunk_span<<<(unsigned)((m->n_chunks * 32 + 255) / 256), 256, 0, st>>>(m->d_col, m->nnz, m->n_chunks,
                                                                                  m->d_cbase, wide);
@@ -912,8 +926,8 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
                     cudaMemcpy(&ls, eslot + m->n_chunks - 1, 4, cudaMemcpyDeviceToHost) != cudaSuccess))
             rc = FD2_ERR_CUDA;
         m->n_exc = (int64_t)lw + ls;
-        if (!rc && (cudaMalloc(&m->d_col16, m->n_chunks * kChunk * sizeof(uint16_t)) != cudaSuccess ||
-                    cudaMalloc(&m->d_exc, std::max<int64_t>(m->n_exc, 1) * kChunk * sizeof(int32_t)) != cudaSuccess))
+        if (!rc && (mat_malloc(&m->d_col16, m->n_chunks * kChunk * sizeof(uint16_t), st) != cudaSuccess ||
+                    mat_malloc(&m->d_exc, std::max<int64_t>(m->n_exc, 1) * kChunk * sizeof(int32_t), st) != cudaSuccess))
             rc = FD2_ERR_OUT_OF_MEMORY;
         if (!rc) {
             pack_columns<<<grid_for(m->n_chunks * kChunk), 256, 0, st>>>(m->d_col, m->nnz, m->n_chunks, wide, eslot,
@@ -922,19 +936,19 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             if (cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
         }
         if (own) {
-            if (wide) cudaFree(wide);
-            if (eslot) cudaFree(eslot);
+            mat_free(wide, st);
+            mat_free(eslot, st);
         }
         if (!rc) {  // the int32 columns are no longer needed
-            cudaFree(m->d_col);
+            mat_free(m->d_col, st);
             m->d_col = nullptr;
         }
     } else if (!rc && m->index_format == FD2_INDEX_PACKED16) {
-        cudaFree(m->d_col);  // empty matrix: nothing to pack
+        mat_free(m->d_col, st);  // empty matrix: nothing to pack
         m->d_col = nullptr;
-        if (cudaMalloc(&m->d_cbase, sizeof(int32_t)) != cudaSuccess ||
-            cudaMalloc(&m->d_col16, kChunk * sizeof(uint16_t)) != cudaSuccess ||
-            cudaMalloc(&m->d_exc, kChunk * sizeof(int32_t)) != cudaSuccess)
+        if (mat_malloc(&m->d_cbase, sizeof(int32_t), st) != cudaSuccess ||
+            mat_malloc(&m->d_col16, kChunk * sizeof(uint16_t), st) != cudaSuccess ||
+            mat_malloc(&m->d_exc, kChunk * sizeof(int32_t), st) != cudaSuccess)
             rc = FD2_ERR_OUT_OF_MEMORY;
     }
     // values (and int32 columns) to storage order
@@ -942,7 +956,7 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
         const int64_t pad = m->n_chunks * kChunk;
         const size_t vs = value_size(m->value_type);
         void* tmp = nullptr;
-        if (cudaMalloc(&tmp, pad * vs) != cudaSuccess) {
+        if (mat_malloc(&tmp, pad * vs, st) != cudaSuccess) {
             rc = FD2_ERR_OUT_OF_MEMORY;
         } else {
             if (vs == 4)
@@ -950,17 +964,17 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             else
                 to_storage_order<uint16_t><<<grid_for(pad), 256, 0, st>>>((const uint16_t*)m->d_val, (uint16_t*)tmp, pad, m->interleaved);
             if (cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
-            cudaFree(m->d_val);
+            mat_free(m->d_val, st);
             m->d_val = tmp;
         }
         if (!rc && m->d_col) {
             int32_t* tc = nullptr;
-            if (cudaMalloc(&tc, pad * sizeof(int32_t)) != cudaSuccess) {
+            if (mat_malloc(&tc, pad * sizeof(int32_t), st) != cudaSuccess) {
                 rc = FD2_ERR_OUT_OF_MEMORY;
             } else {
                 to_storage_order<int32_t><<<grid_for(pad), 256, 0, st>>>(m->d_col, tc, pad, m->interleaved);
                 if (cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
-                cudaFree(m->d_col);
+                mat_free(m->d_col, st);
                 m->d_col = tc;
             }
         }
@@ -1032,8 +1046,8 @@ int fd2_matrix_create(fd2_context* ctx, int64_t rows, int64_t cols, int64_t nnz,
     float* d_f = nullptr;
     unsigned* d_mx = nullptr;
     auto fail = [&](int rc) {
-        if (d_f) cudaFree(d_f);
-        if (d_mx) cudaFree(d_mx);
+        mat_free(d_f, st);
+        mat_free(d_mx, st);
         matrix_free(m);
         delete m;
         return rc;
@@ -1047,10 +1061,10 @@ int fd2_matrix_create(fd2_context* ctx, int64_t rows, int64_t cols, int64_t nnz,
         if (nnz) e = cudaMemcpyAsync(m->d_val, h_val, nnz * sizeof(float), cudaMemcpyHostToDevice, st);
     } else if (e == cudaSuccess) {
         const int64_t nc = std::max<int64_t>(cols, 1);
-        e = cudaMalloc(&d_mx, nc * sizeof(unsigned));
+        e = mat_malloc(&d_mx, nc * sizeof(unsigned), st);
         if (e == cudaSuccess) e = cudaMemsetAsync(d_mx, 0, nc * sizeof(unsigned), st);
         if (e == cudaSuccess && nnz) {
-            e = cudaMalloc(&d_f, nnz * sizeof(float));
+            e = mat_malloc(&d_f, nnz * sizeof(float), st);
             if (e == cudaSuccess) e = cudaMemcpyAsync(d_f, h_val, nnz * sizeof(float), cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess) abs_max_by_column<<<grid_for(nnz), 256, 0, st>>>(m->d_col, d_f, nnz, d_mx);
         }
@@ -1072,8 +1086,8 @@ int fd2_matrix_create(fd2_context* ctx, int64_t rows, int64_t cols, int64_t nnz,
     }
     rc = matrix_finalize(m, st);
     if (rc) return fail(rc);
-    if (d_f) cudaFree(d_f);
-    if (d_mx) cudaFree(d_mx);
+    mat_free(d_f, st);
+    mat_free(d_mx, st);
     *out = m;
     return FD2_OK;
 }
@@ -1112,8 +1126,8 @@ int fd2_matrix_to_host(const fd2_matrix* m, int64_t* h_off, int32_t* h_col, floa
     if (m->nnz) {
         float* d_f = nullptr;
         int32_t* d_c = nullptr;
-        cudaError_t e = cudaMalloc(&d_f, m->nnz * sizeof(float));
-        if (e == cudaSuccess) e = cudaMalloc(&d_c, m->nnz * sizeof(int32_t));
+        cudaError_t e = mat_malloc(&d_f, m->nnz * sizeof(float), st);
+        if (e == cudaSuccess) e = mat_malloc(&d_c, m->nnz * sizeof(int32_t), st);
         if (e == cudaSuccess) {
             switch (m->value_type) {
                 case FD2_VALUES_F16:
@@ -1136,8 +1150,8 @@ int fd2_matrix_to_host(const fd2_matrix* m, int64_t* h_off, int32_t* h_col, floa
         if (e == cudaSuccess) e = cudaMemcpyAsync(h_val, d_f, m->nnz * sizeof(float), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(h_col, d_c, m->nnz * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (d_f) cudaFree(d_f);
-        if (d_c) cudaFree(d_c);
+        mat_free(d_f, st);
+        mat_free(d_c, st);
         FD2_CHECK_CUDA(e);
     }
     FD2_CHECK_CUDA(cudaStreamSynchronize(st));

@@ -264,10 +264,10 @@ int offsets_from_counts(const int64_t* d_count, int64_t n, int64_t* d_off, int64
         size_t tb = 0;
         FD2_CHECK_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tb, d_count, d_off + 1, n, st));
         void* tmp = nullptr;
-        FD2_CHECK_CUDA(cudaMalloc(&tmp, std::max<size_t>(tb, 16)));
+        FD2_CHECK_CUDA(mat_malloc(&tmp, std::max<size_t>(tb, 16), st));
         cudaError_t e = cub::DeviceScan::InclusiveSum(tmp, tb, d_count, d_off + 1, n, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        cudaFree(tmp);
+        mat_free(tmp, st);
         FD2_CHECK_CUDA(e);
     }
     FD2_CHECK_CUDA(cudaMemcpyAsync(total, d_off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -295,15 +295,16 @@ void voi_fill_dispatch(int dst_type, int64_t rows, const int64_t* off, const int
     }
 }
 
-struct Guard {  // frees device buffers on scope exit
+struct Guard {  // frees device buffers on scope exit, in the order of st
+    cudaStream_t st;
     std::vector<void*> p;
+    explicit Guard(cudaStream_t s) : st(s) {}
     ~Guard() {
-        for (void* q : p)
-            if (q) cudaFree(q);
+        for (void* q : p) mat_free(q, st);
     }
     template <typename T>
     cudaError_t alloc(T** ptr, size_t bytes) {
-        cudaError_t e = cudaMalloc((void**)ptr, std::max<size_t>(bytes, 16));
+        cudaError_t e = mat_malloc((void**)ptr, std::max<size_t>(bytes, 16), st);
         if (e == cudaSuccess) p.push_back((void*)*ptr);
         return e;
     }
@@ -346,7 +347,7 @@ int fd2_voi_matrices(const fd2_csr_ensemble* dose, const int32_t* h_voxel_row, i
     const int src_type = info.value_type;
     if (src_type == FD2_VALUES_F32) d_src_scale = nullptr;
 
-    Guard g;
+    Guard g(st);
     int32_t* d_map = nullptr;
     int64_t* d_count = nullptr;
     float* d_max = nullptr;
@@ -386,7 +387,7 @@ int fd2_voi_matrices(const fd2_csr_ensemble* dose, const int32_t* h_voxel_row, i
         }
         if (cudaGetLastError() != cudaSuccess) return fail(FD2_ERR_CUDA);
     }
-    if (cudaMalloc(&t->d_off, (rows + 1) * sizeof(int64_t)) != cudaSuccess) return fail(FD2_ERR_OUT_OF_MEMORY);
+    if (mat_malloc(&t->d_off, (rows + 1) * sizeof(int64_t), st) != cudaSuccess) return fail(FD2_ERR_OUT_OF_MEMORY);
     int64_t nnz = 0;
     int rc = offsets_from_counts(d_count, rows, t->d_off, &nnz, st);
     if (rc) return fail(rc);
@@ -464,7 +465,7 @@ int fd2_matrix_synthetic(fd2_context* ctx, int64_t rows, int64_t cols, int64_t w
         m[i]->scale_axis = !half ? FD2_SCALE_NONE : i == 0 ? FD2_SCALE_COLS : FD2_SCALE_ROWS;
         m[i]->index_format = index_format;
     }
-    Guard g;
+    Guard g(st);
     int64_t* d_count = nullptr;
     float* d_max = nullptr;
     if (g.alloc(&d_count, std::max(rows, cols) * sizeof(int64_t)) != cudaSuccess ||
@@ -474,7 +475,7 @@ int fd2_matrix_synthetic(fd2_context* ctx, int64_t rows, int64_t cols, int64_t w
     synth_t_count<<<(unsigned)cols, kThreads, 0, st>>>(sp, d_count, d_max);
     if (cudaGetLastError() != cudaSuccess) return fail(FD2_ERR_CUDA);
     fd2_matrix* t = m[1];
-    if (cudaMalloc(&t->d_off, (cols + 1) * sizeof(int64_t)) != cudaSuccess) return fail(FD2_ERR_OUT_OF_MEMORY);
+    if (mat_malloc(&t->d_off, (cols + 1) * sizeof(int64_t), st) != cudaSuccess) return fail(FD2_ERR_OUT_OF_MEMORY);
     int64_t nnz = 0;
     int rc = offsets_from_counts(d_count, cols, t->d_off, &nnz, st);
     if (rc) return fail(rc);
@@ -501,7 +502,7 @@ int fd2_matrix_synthetic(fd2_context* ctx, int64_t rows, int64_t cols, int64_t w
     const unsigned wblocks = (unsigned)((rows * 32 + 255) / 256);
     synth_count<<<wblocks, 256, 0, st>>>(sp, d_count);
     if (cudaGetLastError() != cudaSuccess) return fail(FD2_ERR_CUDA);
-    if (cudaMalloc(&a->d_off, (rows + 1) * sizeof(int64_t)) != cudaSuccess) return fail(FD2_ERR_OUT_OF_MEMORY);
+    if (mat_malloc(&a->d_off, (rows + 1) * sizeof(int64_t), st) != cudaSuccess) return fail(FD2_ERR_OUT_OF_MEMORY);
     int64_t nnz_a = 0;
     rc = offsets_from_counts(d_count, rows, a->d_off, &nnz_a, st);
     if (rc) return fail(rc);

@@ -48,3 +48,28 @@ def test_rows_of_one_length(ctx, cols, length):
         assert yt.shape == (cols,) and bool(torch.isfinite(yt).all())
         for a, b in zip(T.transpose().to_host(), (o, c, v)):
             np.testing.assert_array_equal(a, b)
+
+
+def test_matrix_memory_waits_for_products_and_outlives_the_context():
+    """A matrix is destroyed while its product runs on another stream, and after
+    its context; its memory is not handed to the next matrix before that."""
+    import torch
+
+    from fastdose_b200 import api
+
+    ctx = api.Context(0)
+    A, AT = optimize.Matrix.synthetic(ctx, 200_000, 4000, 8000, 0.5, seed=5)
+    x = torch.rand(4000, device="cuda")
+    ref = A.spmv(x).clone()
+    torch.cuda.synchronize()
+    y = torch.empty_like(ref)
+    s = torch.cuda.Stream()
+    for _ in range(20):
+        A.spmv(x, y, stream=s)
+    A.close()
+    B, BT = optimize.Matrix.synthetic(ctx, 200_000, 4000, 8000, 0.5, seed=6)
+    s.synchronize()
+    assert torch.equal(y, ref)
+    ctx.close()
+    for m in (AT, B, BT):
+        m.close()
