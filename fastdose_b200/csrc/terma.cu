@@ -33,11 +33,27 @@ __device__ __forceinline__ float trilinear(const float* __restrict__ vol, int nx
     float fi = floorf(xb), fj = floorf(yb), fk = floorf(zb);
     float ax = xb - fi, ay = yb - fj, az = zb - fk;
     int i = (int)fi, j = (int)fj, k = (int)fk;
-    float c00 = fetch(vol, nx, ny, nz, i, j, k) * (1.0f - ax) + fetch(vol, nx, ny, nz, i + 1, j, k) * ax;
-    float c10 = fetch(vol, nx, ny, nz, i, j + 1, k) * (1.0f - ax) + fetch(vol, nx, ny, nz, i + 1, j + 1, k) * ax;
-    float c01 = fetch(vol, nx, ny, nz, i, j, k + 1) * (1.0f - ax) + fetch(vol, nx, ny, nz, i + 1, j, k + 1) * ax;
-    float c11 =
-        fetch(vol, nx, ny, nz, i, j + 1, k + 1) * (1.0f - ax) + fetch(vol, nx, ny, nz, i + 1, j + 1, k + 1) * ax;
+    float t[8];  // corner (q & 1, q >> 1 & 1, q >> 2)
+    if ((unsigned)i < (unsigned)(nx - 1) && (unsigned)j < (unsigned)(ny - 1) && (unsigned)k < (unsigned)(nz - 1)) {
+        // inside: eight reads without a test between them
+        const float* p = vol + ((size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * (size_t)k));
+        const size_t plane = (size_t)nx * ny;
+        t[0] = __ldg(p);
+        t[1] = __ldg(p + 1);
+        t[2] = __ldg(p + nx);
+        t[3] = __ldg(p + nx + 1);
+        t[4] = __ldg(p + plane);
+        t[5] = __ldg(p + plane + 1);
+        t[6] = __ldg(p + plane + nx);
+        t[7] = __ldg(p + plane + nx + 1);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; q++) t[q] = fetch(vol, nx, ny, nz, i + (q & 1), j + (q >> 1 & 1), k + (q >> 2));
+    }
+    float c00 = t[0] * (1.0f - ax) + t[1] * ax;
+    float c10 = t[2] * (1.0f - ax) + t[3] * ax;
+    float c01 = t[4] * (1.0f - ax) + t[5] * ax;
+    float c11 = t[6] * (1.0f - ax) + t[7] * ax;
     float c0 = c00 * (1.0f - ay) + c10 * ay;
     float c1 = c01 * (1.0f - ay) + c11 * ay;
     return c0 * (1.0f - az) + c1 * az;
@@ -59,11 +75,16 @@ __device__ __forceinline__ float3 bev_to_pvcs(float3 v, float th, float ph, floa
                        k * cr + ct * t.z + st * (sr * t.y));
 }
 
-// 40 registers, 6 blocks per SM: the ray trace waits on density reads, and
-// the extra warps hide more of that latency (measured 66.6 against 68.7 ms per
-// 400-beam plan at 48 registers; 32 registers spilled and was slower).
-template <bool kSkipDark>
-__global__ void __launch_bounds__(256, 6) terma_kernel(const fd2_beam_t* __restrict__ beams,
+// The ray trace waits on density reads.  kThreads 256, 40 registers, 6 blocks per
+// SM: the extra warps hide more of that latency (measured 66.6 against 68.7 ms
+// per 400-beam plan at 48 registers; 32 registers spilled and was slower).
+// kThreads 64, for launches that leave SMs idle at 256: the rays spread over four
+// times the blocks, and without a register limit more of a slice's reads are in
+// flight together.  With the eight texel reads free of tests inside the volume:
+// 100-beam torso plan 16.85 -> 14.18 ms, one slab beam 142 -> 117 us, four 32 x 32
+// fields 480 -> 400 us.
+template <bool kSkipDark, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 6 : 4) terma_kernel(const fd2_beam_t* __restrict__ beams,
                                                     const float* const* __restrict__ fluence,
                                                     float* const* __restrict__ terma, float* const* __restrict__ dens,
                                                     const float* __restrict__ density, int nx, int ny, int nz,
@@ -128,16 +149,15 @@ int launch_terma(fd2_context* ctx, size_t fmap_npixels, size_t n_beams, const fd
         sp.mu[e] = spectrum->mu[e];
     }
     const fd2_volume_t& v = density->vol;
-    // blocks per beam cover up to 1024 pixels (the reference's bound: one block per beam)
-    dim3 grid((unsigned)n_beams, (unsigned)((fmap_npixels + 255) / 256)), block(256);
-    if (fluence_skip)
-        terma_kernel<true><<<grid, block, 0, stream>>>(d_beams, d_fluence, d_terma, d_dens, density->d_density,
-                                                       v.dim[0], v.dim[1], v.dim[2], v.voxel_size[0],
-                                                       v.voxel_size[1], v.voxel_size[2], sp);
-    else
-        terma_kernel<false><<<grid, block, 0, stream>>>(d_beams, d_fluence, d_terma, d_dens, density->d_density,
-                                                        v.dim[0], v.dim[1], v.dim[2], v.voxel_size[0],
-                                                        v.voxel_size[1], v.voxel_size[2], sp);
+    // blocks per beam cover up to 1024 pixels (the reference's bound: one block per
+    // beam); fewer than two blocks of 256 an SM go out as blocks of 64
+    const size_t blocks256 = n_beams * ((fmap_npixels + 255) / 256);
+    const unsigned threads = blocks256 < 2 * 148 ? 64 : 256;
+    dim3 grid((unsigned)n_beams, (unsigned)((fmap_npixels + threads - 1) / threads)), block(threads);
+    auto kernel = threads == 64 ? (fluence_skip ? terma_kernel<true, 64> : terma_kernel<false, 64>)
+                                : (fluence_skip ? terma_kernel<true, 256> : terma_kernel<false, 256>);
+    kernel<<<grid, block, 0, stream>>>(d_beams, d_fluence, d_terma, d_dens, density->d_density, v.dim[0], v.dim[1],
+                                       v.dim[2], v.voxel_size[0], v.voxel_size[1], v.voxel_size[2], sp);
     FD2_CHECK_CUDA(cudaGetLastError());
     if (ctx) ctx->launches += 1;
     return FD2_OK;
