@@ -217,9 +217,12 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
     namespace cg = cooperative_groups;
     const int n_cl = kWpa > 1 ? (int)cg::this_cluster().num_blocks() : 1;
     const int rank = kWpa > 1 ? (int)cg::this_cluster().block_rank() : 0;
+    // kept apart from blockIdx.x where kWpa is 1: with one expression for both
+    // the F = 20 instance spills 52 bytes instead of 44 and the F = 8 one 72
+    // instead of none (24 beams of 20 x 20 maps: 141.4 against 140.4 ms)
     const int unit = blockIdx.x / n_cl;
-    const int bi = split ? unit / n_tf : (order ? order[unit] : unit);
-    const int t0 = split ? unit % n_tf : 0;
+    const int bi = split ? (kWpa > 1 ? unit : blockIdx.x) / n_tf : (order ? order[blockIdx.x] : blockIdx.x);
+    const int t0 = split ? (kWpa > 1 ? unit : blockIdx.x) % n_tf : 0;
     const int t1 = split ? t0 + 1 : n_tf;
     const fd2_beam_t& b = beams[bi];
     RayGeom g;
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
             for (int v = threadIdx.x; v < g.P; v += blockDim.x)
                 tr[v] = s == st_s ? make_float2(s_stage[v], s_stage[kStageP + v])
                                   : make_float2(__ldg(T + (size_t)s * pitch + v), __ldg(R + (size_t)s * pitch + v));
-            for (int v = 32 * sub + lane; v < g.P; v += 32 * kWpa) mydp[v] = make_float2(0.0f, 0.0f);
+            for (int v = kWpa > 1 ? 32 * sub + lane : lane; v < g.P; v += 32 * kWpa) mydp[v] = make_float2(0.0f, 0.0f);
             __syncthreads();
             st_s = s + 1 < g.L ? s + 1 : (t + 1 < t1 ? 0 : -1);
             if (st_s >= 0)
@@ -326,106 +329,31 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
                 const bool flag = next_point(c, cd, np);
                 const float fe = (np.z * g.ls + g.lim_min) * g.inv_sad;
                 const float dzp = (np.z - c.z) * g.ls;
-                // the azimuth's warps in turn when two of its rays might meet in a voxel
-                const bool turns = kWpa > 1 && (may_meet(c.x, np.x, g.ffx) || may_meet(c.y, np.y, g.ffy));
-                for (int turn = turns ? 0 : sub;; turn++) {
-                    if (turn == sub) {
-                        if constexpr (kCols) {
-                            const float btx = __fadd_rn(c.x, fcol), ntx = __fadd_rn(np.x, fcol);
-                            const int cx = mid_index(btx, ntx, g.ffx, g.fx);
-                            const bool wrapx = crosses_edge(btx, ntx, g.ffx);
-                            const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
-                            const float dxz2 = dxp * dxp + dzp * dzp;
-                            const float bty = __fadd_rn(c.y, frow), nty = __fadd_rn(np.y, frow);
-                            const int ycode = mid_index(bty, nty, g.ffy, g.fy) | (crosses_edge(bty, nty, g.ffy) ? 64 : 0);
-                            const float dyq = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
-#pragma unroll
-                            for (int j = 0; j < RPL; j++) {
-                                const int y = cgrp + kgrp * (kWpa > 1 ? sub * RPL + j : j);
-                                const bool on = clane && y < g.fy;
-                                const int yc = __shfl_sync(0xffffffffu, ycode, on ? y : 0);
-                                const float dyp = __shfl_sync(0xffffffffu, dyq, on ? y : 0);
-                                const int mi = on ? cx + g.fx * (yc & 63) : 0;
-                                const bool wrap = wrapx || (yc & 64);
-                                const float l2 = dxz2 + dyp * dyp;
-                                const float len = seg_length(l2);
-                                const float2 trv = tr[mi];
-                                const float p = len * trv.y;
-                                const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
-                                const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
-                                if (on) {
-                                    float2 acc = mydp[mi];
-                                    acc.x += dep;
-                                    acc.y += p;
-                                    mydp[mi] = acc;
-                                }
-                                XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
-                                XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
-                            }
-                        } else if constexpr (kTab) {
-                            // F x F map, F <= 24: the rays of lane l are the cells l + 32 j,
-                            // so all 32 lanes carry rays whatever F.  The step's 2F halves
-                            // (x of each column, y of each row) are evaluated once, one per
-                            // lane and round, into the warp's half table {+-|offset|,
-                            // bytes into the slice}, the edge crossing as the sign bit;
-                            // each ray then reads its column's and its row's entry.
-                            float2* ht = s_htab + 64 * warp;
-                            for (int h = lane; h < 2 * g.fx; h += 32) {
-                                const bool yh = h >= g.fx;
-                                const float off = (float)(yh ? h - g.fx : h);
-                                const float hb = __fadd_rn(yh ? c.y : c.x, off), hn = __fadd_rn(yh ? np.y : np.x, off);
-                                const float ff = yh ? g.ffy : g.ffx, hh = yh ? g.hy : g.hx, bs = yh ? g.bsy : g.bsx;
-                                const int hi = mid_index(hb, hn, ff, yh ? g.fy : g.fx);
-                                const float hq = fabsf((hn - hh) * bs * fe - (hb - hh) * bs * fs);
-                                const float hs = crosses_edge(hb, hn, ff) ? -hq : hq;
-                                const int bytes = (int)sizeof(float2) * (yh ? hi * g.fx : hi);
-                                ht[h] = make_float2(hs, __int_as_float(bytes));
-                            }
-                            __syncwarp();
-                            const float dz2 = dzp * dzp;
-#pragma unroll
-                            for (int j = 0; j < RPL; j++) {
-                                const uint32_t pr = s_pairs[32 * (kWpa > 1 ? sub * RPL + j : j) + lane];
-                                const bool on = pr != 0xffffffffu;
-                                const float2 xe = ht[on ? (pr & 0xffffu) : 0], ye = ht[on ? (pr >> 16) : 0];
-                                const bool wrap = (__float_as_int(xe.x) | __float_as_int(ye.x)) < 0;
-                                const int mb = __float_as_int(xe.y) + __float_as_int(ye.y);
-                                const float dxz2 = xe.x * xe.x + dz2;
-                                const float l2 = dxz2 + ye.x * ye.x;
-                                const float len = seg_length(l2);
-                                const float2 trv = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(tr) + mb);
-                                const float p = len * trv.y;
-                                const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
-                                const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
-                                if (on) {
-                                    float2* acc_p = reinterpret_cast<float2*>(reinterpret_cast<char*>(mydp) + mb);
-                                    float2 acc = *acc_p;
-                                    acc.x += dep;
-                                    acc.y += p;
-                                    *acc_p = acc;
-                                }
-                                XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
-                                XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
-                            }
-                        } else {
+                auto rays = [&]() {
+                    if constexpr (kCols) {
+                        const float btx = __fadd_rn(c.x, fcol), ntx = __fadd_rn(np.x, fcol);
+                        const int cx = mid_index(btx, ntx, g.ffx, g.fx);
+                        const bool wrapx = crosses_edge(btx, ntx, g.ffx);
+                        const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
+                        const float dxz2 = dxp * dxp + dzp * dzp;
+                        const float bty = __fadd_rn(c.y, frow), nty = __fadd_rn(np.y, frow);
+                        const int ycode = mid_index(bty, nty, g.ffy, g.fy) | (crosses_edge(bty, nty, g.ffy) ? 64 : 0);
+                        const float dyq = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
 #pragma unroll
                         for (int j = 0; j < RPL; j++) {
-                            const float btx = __fadd_rn(c.x, fix[j]), ntx = __fadd_rn(np.x, fix[j]);
-                            const float bty = __fadd_rn(c.y, fiy[j]), nty = __fadd_rn(np.y, fiy[j]);
-                            const int cx = mid_index(btx, ntx, g.ffx, g.fx);
-                            const int cy = mid_index(bty, nty, g.ffy, g.fy);
-                            const int mi = cx + cy * g.fx;
-                            const bool wrap = crosses_edge(btx, ntx, g.ffx) || crosses_edge(bty, nty, g.ffy);
-                            // physical segment length (d_calcLineSeg, DoseComp.cu:114-144)
-                            const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
-                            const float dyp = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
-                            const float l2 = dxp * dxp + dyp * dyp + dzp * dzp;
+                            const int y = cgrp + kgrp * (kWpa > 1 ? sub * RPL + j : j);
+                            const bool on = clane && y < g.fy;
+                            const int yc = __shfl_sync(0xffffffffu, ycode, on ? y : 0);
+                            const float dyp = __shfl_sync(0xffffffffu, dyq, on ? y : 0);
+                            const int mi = on ? cx + g.fx * (yc & 63) : 0;
+                            const bool wrap = wrapx || (yc & 64);
+                            const float l2 = dxz2 + dyp * dyp;
                             const float len = seg_length(l2);
-                            const float2 trv = tr[act[j] ? mi : 0];
+                            const float2 trv = tr[mi];
                             const float p = len * trv.y;
                             const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
                             const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
-                            if (act[j]) {
+                            if (on) {
                                 float2 acc = mydp[mi];
                                 acc.x += dep;
                                 acc.y += p;
@@ -434,10 +362,90 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
                             XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
                             XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
                         }
+                    } else if constexpr (kTab) {
+                        // F x F map, F <= 24: the rays of lane l are the cells l + 32 j,
+                        // so all 32 lanes carry rays whatever F.  The step's 2F halves
+                        // (x of each column, y of each row) are evaluated once, one per
+                        // lane and round, into the warp's half table {+-|offset|,
+                        // bytes into the slice}, the edge crossing as the sign bit;
+                        // each ray then reads its column's and its row's entry.
+                        float2* ht = s_htab + 64 * warp;
+                        for (int h = lane; h < 2 * g.fx; h += 32) {
+                            const bool yh = h >= g.fx;
+                            const float off = (float)(yh ? h - g.fx : h);
+                            const float hb = __fadd_rn(yh ? c.y : c.x, off), hn = __fadd_rn(yh ? np.y : np.x, off);
+                            const float ff = yh ? g.ffy : g.ffx, hh = yh ? g.hy : g.hx, bs = yh ? g.bsy : g.bsx;
+                            const int hi = mid_index(hb, hn, ff, yh ? g.fy : g.fx);
+                            const float hq = fabsf((hn - hh) * bs * fe - (hb - hh) * bs * fs);
+                            const float hs = crosses_edge(hb, hn, ff) ? -hq : hq;
+                            const int bytes = (int)sizeof(float2) * (yh ? hi * g.fx : hi);
+                            ht[h] = make_float2(hs, __int_as_float(bytes));
                         }
+                        __syncwarp();
+                        const float dz2 = dzp * dzp;
+#pragma unroll
+                        for (int j = 0; j < RPL; j++) {
+                            const uint32_t pr = s_pairs[32 * (kWpa > 1 ? sub * RPL + j : j) + lane];
+                            const bool on = pr != 0xffffffffu;
+                            const float2 xe = ht[on ? (pr & 0xffffu) : 0], ye = ht[on ? (pr >> 16) : 0];
+                            const bool wrap = (__float_as_int(xe.x) | __float_as_int(ye.x)) < 0;
+                            const int mb = __float_as_int(xe.y) + __float_as_int(ye.y);
+                            const float dxz2 = xe.x * xe.x + dz2;
+                            const float l2 = dxz2 + ye.x * ye.x;
+                            const float len = seg_length(l2);
+                            const float2 trv = *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(tr) + mb);
+                            const float p = len * trv.y;
+                            const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
+                            const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
+                            if (on) {
+                                float2* acc_p = reinterpret_cast<float2*>(reinterpret_cast<char*>(mydp) + mb);
+                                float2 acc = *acc_p;
+                                acc.x += dep;
+                                acc.y += p;
+                                *acc_p = acc;
+                            }
+                            XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
+                            XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
+                        }
+                    } else {
+#pragma unroll
+                    for (int j = 0; j < RPL; j++) {
+                        const float btx = __fadd_rn(c.x, fix[j]), ntx = __fadd_rn(np.x, fix[j]);
+                        const float bty = __fadd_rn(c.y, fiy[j]), nty = __fadd_rn(np.y, fiy[j]);
+                        const int cx = mid_index(btx, ntx, g.ffx, g.fx);
+                        const int cy = mid_index(bty, nty, g.ffy, g.fy);
+                        const int mi = cx + cy * g.fx;
+                        const bool wrap = crosses_edge(btx, ntx, g.ffx) || crosses_edge(bty, nty, g.ffy);
+                        // physical segment length (d_calcLineSeg, DoseComp.cu:114-144)
+                        const float dxp = (ntx - g.hx) * g.bsx * fe - (btx - g.hx) * g.bsx * fs;
+                        const float dyp = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
+                        const float l2 = dxp * dxp + dyp * dyp + dzp * dzp;
+                        const float len = seg_length(l2);
+                        const float2 trv = tr[act[j] ? mi : 0];
+                        const float p = len * trv.y;
+                        const float ea = exp2_sfu(ka * p), eb = exp2_sfu(kb * p);
+                        const float dep = (Aa * XA[j] + Bb * XB[j]) * p;
+                        if (act[j]) {
+                            float2 acc = mydp[mi];
+                            acc.x += dep;
+                            acc.y += p;
+                            mydp[mi] = acc;
+                        }
+                        XA[j] = wrap ? 0.0f : __fmaf_rn(ea, XA[j] - trv.x, trv.x);
+                        XB[j] = wrap ? 0.0f : __fmaf_rn(eb, XB[j] - trv.x, trv.x);
                     }
-                    if constexpr (kWpa > 1) named_barrier(1 + az, 32 * kWpa);
-                    if (!turns || turn == kWpa - 1) break;
+                    }
+                };
+                if constexpr (kWpa > 1) {
+                    // the azimuth's warps in turn when two of its rays might meet in a voxel
+                    const bool turns = may_meet(c.x, np.x, g.ffx) || may_meet(c.y, np.y, g.ffy);
+                    for (int turn = turns ? 0 : sub;; turn++) {
+                        if (turn == sub) rays();
+                        named_barrier(1 + az, 32 * kWpa);
+                        if (!turns || turn == kWpa - 1) break;
+                    }
+                } else {
+                    rays();
                 }
                 c = np;
                 fs = fe;
@@ -454,16 +462,15 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
                     break;
                 }
             }
-            if (threadIdx.x == 0 && rank == 0) {
+            if (threadIdx.x == 0 && (kWpa == 1 || rank == 0)) {
                 // the first azimuth's plane after this slice; it always lies ahead
                 const int nxt = (int)roundf(c.z);
                 *s_next = nxt > s ? nxt : g.L;
             }
-            int s_new;
             if constexpr (kWpa > 1) {
                 cg::this_cluster().sync();
                 const int* ctrl = cg::this_cluster().map_shared_rank(s_ctrl, 0);
-                s_new = ctrl[1] ? g.L : ctrl[0];
+                const int s_new = ctrl[1] ? g.L : ctrl[0];
                 // this block's share of the pixels, over all blocks' azimuths in order
                 const float2* part[kMaxCluster];
 #pragma unroll
@@ -486,7 +493,7 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
                 continue;
             }
             __syncthreads();
-            s_new = *s_abort ? g.L : *s_next;
+            const int s_new = *s_abort ? g.L : *s_next;
             // reduce azimuths in order; normalise by the last azimuth's path sum
             for (int v = threadIdx.x; v < g.P; v += blockDim.x) {
                 float sum = 0.0f, last_sum_p;
@@ -494,7 +501,7 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
                 last_sum_p = dp[(size_t)(n_phi - 1) * g.P + v].y;
                 const float val = sum / (last_sum_p + 1e-4f);
                 if (split)
-                    split_out[(size_t)unit * split_stride + (size_t)s * g.P + v] = val;
+                    split_out[(size_t)(kWpa > 1 ? unit : (int)blockIdx.x) * split_stride + (size_t)s * g.P + v] = val;
                 else
                     // this block alone owns beam bi's dose and each (s, v) stays with
                     // one thread, so a fire-and-forget add gives D + val in pass order
