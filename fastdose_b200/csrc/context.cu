@@ -75,7 +75,7 @@ int density_pool(int device, cudaMemPool_t* out) {
 
 int matrix_pool(int device, cudaMemPool_t* out) {
     static cudaMemPool_t pools[kMaxDevices] = {};
-    return device_pool(pools, device, 1ull << 30, "matrix", out);
+    return device_pool(pools, device, 4ull << 30, "matrix", out);
 }
 
 int density_create_pooled(fd2_context* ctx, const float* host_density, const fd2_volume_t* volume,

@@ -92,7 +92,9 @@ namespace fd2 {
 // of a stream, from a pool the library keeps per device (as densities are): a
 // matrix makes some thirty allocations, and cudaMalloc and cudaFree, which wait
 // for the device, took most of the time of the orientation loop's phases.  The
-// pool keeps at most 1 GiB of freed memory; fd2_context_release empties it.
+// pool keeps at most 4 GiB of freed memory (with 1 GiB, the transpose of 5e7
+// nonzeros gave its buffers back and took them again: 15 % of the build);
+// fd2_context_release empties it.
 cudaError_t mat_malloc_bytes(void** p, size_t bytes, cudaStream_t stream);
 template <typename T>
 cudaError_t mat_malloc(T** p, size_t bytes, cudaStream_t stream) {
