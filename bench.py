@@ -35,11 +35,11 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "CCCS beamlets/s (dose-loading matrix, batched 4pi)"
-# From one ncu capture of the CCCS march on the 40-beam plan (6056 beamlets,
-# 8.2 waves; profiles/cccs_kernel_4pi_torso_40beams.md):
+# From one ncu capture of the CCCS march on the 40-beam plan (6056 beamlets;
+# profiles/cccs_march_4pi_torso_40beams.md):
 # dram__bytes_read.sum + dram__bytes_write.sum, and smsp__inst_executed.sum
-CCCS_DRAM_BYTES_PER_BEAMLET = (28.562879e9 + 9.447058e9) / 6056
-CCCS_WARP_INST_PER_BEAMLET = 124.063924973e9 / 6056
+CCCS_DRAM_BYTES_PER_BEAMLET = (28.421676e9 + 9.664041e9) / 6056
+CCCS_WARP_INST_PER_BEAMLET = 108.351843346e9 / 6056
 UNIT = "beamlets/s"
 
 
@@ -1088,7 +1088,7 @@ def run_fd2(args, rank, world):
     L = np.concatenate([b["long_dim"] for b in beamlets]).astype(np.float64)
     cccs_bytes = float(np.sum(4.0 * P * L * 3))  # Terma + density read, dose written, per beamlet
     # DRAM bytes the CCCS kernel moves per beamlet: dram__bytes_read.sum + dram__bytes_write.sum of one
-    # ncu capture of the march on the 40-beam plan (6056 beamlets, 38.0 GB),
+    # ncu capture of the march on the 40-beam plan (6056 beamlets, 38.1 GB),
     # scaled by the beamlets of this step (each zenith pass re-reads its slices: traffic grows with beamlets)
     cccs_traffic = CCCS_DRAM_BYTES_PER_BEAMLET * n_bl
     cccs_ms = stages["cccs"]
@@ -1132,15 +1132,15 @@ def run_fd2(args, rank, world):
         "gpu_launches": int(launches),
         "cccs_tuned": {"schedules": {str(k): v for k, v in ctx.tuned_schedules()[0].items()},
                        "tuning_runs": ctx.tuned_schedules()[1]},
-        "roofline": {"bound": "hbm", "kernel": "cccs_kernel", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": "hbm", "kernel": "cccs_march_kernel", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if achieved else None, "traffic": cccs_traffic,
                      "peak_source": peak_kind, "algorithmic_bytes_per_step": cccs_bytes},
-        "sfu_roofline": {"bound": "MUFU", "kernel": "cccs_kernel", "ops_per_step": sfu_ops, "ray_steps": ray_steps,
+        "sfu_roofline": {"bound": "MUFU", "kernel": "cccs_march_kernel", "ops_per_step": sfu_ops, "ray_steps": ray_steps,
                          "achieved_ops_per_s": sfu_achieved, "peak_ops_per_s": sfu_peak,
                          "frac": sfu_achieved / sfu_peak if sfu_achieved else None,
                          "basis": "3 MUFU per ray step; ray steps L (1 + (|dx|+|dy|)/dz) per cone pass from the "
                                   "device's cone directions; peak 16/clk/SM at the sampled SM clock"},
-        "issue_roofline": {"bound": "issue", "kernel": "cccs_kernel", "warp_instructions_per_step": issue_inst,
+        "issue_roofline": {"bound": "issue", "kernel": "cccs_march_kernel", "warp_instructions_per_step": issue_inst,
                            "achieved": issue_achieved, "peak": issue_peak, "unit": "warp instructions/s",
                            "frac": issue_achieved / issue_peak if issue_achieved else None,
                            "basis": "warp instructions per beamlet from one ncu capture of the 40-beam plan "
