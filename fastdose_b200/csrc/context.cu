@@ -78,6 +78,17 @@ int matrix_pool(int device, cudaMemPool_t* out) {
     return device_pool(pools, device, 4ull << 30, "matrix", out);
 }
 
+void device_free(int device, void* const* p, size_t n) {
+    int cur = -1;
+    cudaGetDevice(&cur);
+    if (cur != device) cudaSetDevice(device);
+    cudaDeviceSynchronize();
+    for (size_t i = 0; i < n; i++)
+        if (p[i]) cudaFreeAsync(p[i], cudaStreamLegacy);
+    cudaGetLastError();  // nothing a later launch check should see
+    if (cur >= 0 && cur != device) cudaSetDevice(cur);
+}
+
 int density_create_pooled(fd2_context* ctx, const float* host_density, const fd2_volume_t* volume,
                           fd2_density** out) {
     FD2_REQUIRE(ctx && host_density && volume && out, FD2_ERR_INVALID_ARGUMENT, "density_create: null argument");
@@ -269,17 +280,10 @@ int fd2_density_destroy(fd2_density* d) {
         if (d->pooled) {
             cudaFreeAsync(d->d_density, d->ctx->stream);
         } else {
-            // A density made by fd2_density_create may be read by work on any
-            // stream, and may outlive its context: like cudaFree, wait for the
-            // device, then return the memory to the library's density pool,
-            // which lives as long as the process, on the default stream.
-            int cur = -1;
-            cudaGetDevice(&cur);
-            if (cur != d->device) cudaSetDevice(d->device);
-            cudaDeviceSynchronize();
-            cudaFreeAsync(d->d_density, cudaStreamLegacy);
-            cudaGetLastError();  // nothing a later launch check should see
-            if (cur >= 0 && cur != d->device) cudaSetDevice(cur);
+            // a density made by fd2_density_create: the library's density pool
+            // lives as long as the process
+            void* const q = d->d_density;
+            fd2::device_free(d->device, &q, 1);
         }
     }
     delete d;

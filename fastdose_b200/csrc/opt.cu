@@ -313,6 +313,7 @@ unsigned vec_blocks(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<
 
 struct fd2_opt_problem {
     fd2_context* ctx = nullptr;
+    int device = fd2::current_device();  // where its memory is
     const fd2_matrix *A = nullptr, *AT = nullptr, *D = nullptr, *DT = nullptr;
     int64_t n_ptv = 0, n_oar = 0, nv = 0, n = 0, m = 0;
     float gamma = 1.0f, eta = 0.1f;
@@ -714,8 +715,7 @@ int fd2_opt_problem_create(fd2_context* ctx, const fd2_matrix* A, const fd2_matr
 int fd2_opt_problem_destroy(fd2_opt_problem* p) {
     if (!p) return FD2_OK;
     drop_graph(p);
-    cudaDeviceSynchronize();  // a caller may still read what the problem wrote
-    for (void* q : p->owned) mat_free(q, nullptr);
+    device_free(p->device, p->owned.data(), p->owned.size());  // a caller may still read what the problem wrote
     if (p->h_red) cudaFreeHost(p->h_red);
     if (p->h_nrm) cudaFreeHost(p->h_nrm);
     for (cudaEvent_t ev : {p->ev_fork, p->ev_join})

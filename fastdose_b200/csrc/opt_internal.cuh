@@ -45,11 +45,17 @@ struct ColView {
 
 inline size_t value_size(int vt) { return vt == FD2_VALUES_F32 ? 4 : 2; }
 inline int64_t round_chunk(int64_t n) { return (n + kChunk - 1) / kChunk * kChunk; }
+inline int current_device() {
+    int d = 0;
+    cudaGetDevice(&d);
+    return d;
+}
 
 }  // namespace fd2
 
 struct fd2_matrix {
     fd2_context* ctx = nullptr;
+    int device = fd2::current_device();  // where its memory is; it may outlive the context
     int64_t rows = 0, cols = 0, nnz = 0;
     int value_type = FD2_VALUES_F32;
     int scale_axis = FD2_SCALE_NONE;
@@ -112,8 +118,8 @@ int matrix_alloc_entries(fd2_matrix* m, cudaStream_t stream);
 // warp partition) from d_off, and packs the columns when m->index_format is
 // PACKED16.  Call once the offsets, columns and values are written.
 int matrix_finalize(fd2_matrix* m, cudaStream_t stream);
-// Frees what m holds, after all work of the device (a product may run on any
-// stream, and the matrix may outlive its context).
+// Frees what m holds, after all work of its device (a product may run on any
+// stream, the matrix may outlive its context, and another device may be current).
 void matrix_free(fd2_matrix* m);
 // Transpose into a matrix of the given index format.
 int matrix_transpose_fmt(const fd2_matrix* m, int index_format, fd2_matrix** out);

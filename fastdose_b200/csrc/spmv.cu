@@ -786,11 +786,10 @@ int matrix_alloc_entries(fd2_matrix* m, cudaStream_t st) {
 }
 
 void matrix_free(fd2_matrix* m) {
-    cudaDeviceSynchronize();
-    for (void* p : {(void*)m->d_off, (void*)m->d_col, (void*)m->d_col16, (void*)m->d_cbase, (void*)m->d_exc, m->d_val,
-                    (void*)m->d_scale, (void*)m->d_head, (void*)m->d_chunk_h, (void*)m->d_chunk_row0, (void*)m->d_nzrow,
-                    (void*)m->d_carry_row, (void*)m->d_carry_val, (void*)m->d_xs, (void*)m->d_zrow, (void*)m->d_nz})
-        mat_free(p, nullptr);
+    void* const held[] = {m->d_off,     m->d_col,    m->d_col16,      m->d_cbase, m->d_exc,       m->d_val,
+                          m->d_scale,   m->d_head,   m->d_chunk_h,    m->d_chunk_row0, m->d_nzrow, m->d_carry_row,
+                          m->d_carry_val, m->d_xs,   m->d_zrow,       m->d_nz};
+    device_free(m->device, held, sizeof(held) / sizeof(held[0]));
     m->d_off = nullptr;
     m->d_col = nullptr;
     m->d_col16 = nullptr;
