@@ -410,12 +410,14 @@ int join_side(fd2_opt_problem* p) {
 // d_o1 and d_o2; step: the line-search terms of d_x, d_y and d_g too.  The D
 // products and the line-search terms run beside the A products.  n_groups >= 0:
 // the results, with that many group norms, go to the host.
+// A matrix has one set of carries and scaled x, so a product of the same handle
+// follows on the work stream.
 int objective(fd2_opt_problem* p, const float* x, bool with_grad, int slot, int64_t n_groups, bool step = false) {
     cudaStream_t st = p->ctx->stream, side = st;
     const bool fork = p->m > 0 || step;
     if (fork) FD2_TRY(fork_side(p, &side));
     FD2_TRY(matrix_spmv(p->A, x, p->d_Ax, st));
-    if (p->m) FD2_TRY(matrix_spmv(p->D, x, p->d_Dx, side));
+    if (p->m) FD2_TRY(matrix_spmv(p->D, x, p->d_Dx, p->D == p->A ? st : side));
     if (step) {
         step_terms<<<red_blocks(p->n), kRedThreads, 0, side>>>(p->d_g, p->d_x, p->d_y, p->n, p->d_part2, p->d_done + 1,
                                                               p->d_red + S_DXY);
@@ -435,7 +437,7 @@ int objective(fd2_opt_problem* p, const float* x, bool with_grad, int slot, int6
         if (p->m) FD2_TRY(fork_side(p, &side));
         FD2_TRY(matrix_spmv(p->AT, p->d_g1, p->d_o1, st));
         if (p->m) {
-            FD2_TRY(matrix_spmv(p->DT, p->d_g2, p->d_o2, side));
+            FD2_TRY(matrix_spmv(p->DT, p->d_g2, p->d_o2, p->DT == p->AT ? st : side));
             FD2_TRY(join_side(p));
         } else {
             FD2_CHECK_CUDA(cudaMemsetAsync(p->d_o2, 0, p->n * sizeof(float), st));
