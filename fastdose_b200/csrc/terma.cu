@@ -26,37 +26,61 @@ __device__ __forceinline__ float fetch(const float* __restrict__ vol, int nx, in
     return __ldg(vol + (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * (size_t)k));
 }
 
-// Trilinear sample at unnormalised coordinates (u, v, w) in voxel units.
+// a (1 - w) + b w with its one fused multiply-add spelled out, so that every
+// instance of the kernel rounds alike: a beam's Terma does not depend on the batch.
+__device__ __forceinline__ float mix(float a, float b, float w) {
+    return __fmaf_rn(a, __fsub_rn(1.0f, w), __fmul_rn(b, w));
+}
+
+// Trilinear sample at unnormalised coordinates (u, v, w) in voxel units.  kAtOnce:
+// all eight texels are read before the first is used, else the upper four follow
+// the blend of the lower four.
+template <bool kAtOnce>
 __device__ __forceinline__ float trilinear(const float* __restrict__ vol, int nx, int ny, int nz, float u, float v,
                                            float w) {
     float xb = u - 0.5f, yb = v - 0.5f, zb = w - 0.5f;
     float fi = floorf(xb), fj = floorf(yb), fk = floorf(zb);
     float ax = xb - fi, ay = yb - fj, az = zb - fk;
     int i = (int)fi, j = (int)fj, k = (int)fk;
+    const bool inside = (unsigned)i < (unsigned)(nx - 1) && (unsigned)j < (unsigned)(ny - 1) && (unsigned)k < (unsigned)(nz - 1);
+    const float* p = vol + ((size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * (size_t)k));  // read inside only
+    const size_t plane = (size_t)nx * ny;
     float t[8];  // corner (q & 1, q >> 1 & 1, q >> 2)
-    if ((unsigned)i < (unsigned)(nx - 1) && (unsigned)j < (unsigned)(ny - 1) && (unsigned)k < (unsigned)(nz - 1)) {
-        // inside: eight reads without a test between them
-        const float* p = vol + ((size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * (size_t)k));
-        const size_t plane = (size_t)nx * ny;
-        t[0] = __ldg(p);
-        t[1] = __ldg(p + 1);
-        t[2] = __ldg(p + nx);
-        t[3] = __ldg(p + nx + 1);
-        t[4] = __ldg(p + plane);
-        t[5] = __ldg(p + plane + 1);
-        t[6] = __ldg(p + plane + nx);
-        t[7] = __ldg(p + plane + nx + 1);
-    } else {
+    float c00, c10, c01, c11;
+    auto read = [&](int q, const float* r) {  // inside: no test between the reads
+        t[q] = __ldg(r);
+        t[q + 1] = __ldg(r + 1);
+        t[q + 2] = __ldg(r + nx);
+        t[q + 3] = __ldg(r + nx + 1);
+    };
+    auto blend = [&](int q, float& low, float& high) {
+        low = mix(t[q], t[q + 1], ax);
+        high = mix(t[q + 2], t[q + 3], ax);
+    };
+    auto read_tested = [&]() {
 #pragma unroll
         for (int q = 0; q < 8; q++) t[q] = fetch(vol, nx, ny, nz, i + (q & 1), j + (q >> 1 & 1), k + (q >> 2));
+    };
+    if constexpr (kAtOnce) {
+        if (inside) {
+            read(0, p);
+            read(4, p + plane);
+        } else {
+            read_tested();
+        }
+        blend(0, c00, c10);
+        blend(4, c01, c11);
+    } else if (inside) {
+        read(0, p);
+        blend(0, c00, c10);
+        read(4, p + plane);
+        blend(4, c01, c11);
+    } else {
+        read_tested();
+        blend(0, c00, c10);
+        blend(4, c01, c11);
     }
-    float c00 = t[0] * (1.0f - ax) + t[1] * ax;
-    float c10 = t[2] * (1.0f - ax) + t[3] * ax;
-    float c01 = t[4] * (1.0f - ax) + t[5] * ax;
-    float c11 = t[6] * (1.0f - ax) + t[7] * ax;
-    float c0 = c00 * (1.0f - ay) + c10 * ay;
-    float c1 = c01 * (1.0f - ay) + c11 * ay;
-    return c0 * (1.0f - az) + c1 * az;
+    return mix(mix(c00, c10, ay), mix(c01, c11, ay), az);
 }
 
 // BEV -> PVCS rotation of v (inverse of the couch/gantry/collimator rotation).
@@ -76,13 +100,18 @@ __device__ __forceinline__ float3 bev_to_pvcs(float3 v, float th, float ph, floa
 }
 
 // The ray trace waits on density reads.  kThreads 256, 40 registers, 6 blocks per
-// SM: the extra warps hide more of that latency (measured 66.6 against 68.7 ms
-// per 400-beam plan at 48 registers; 32 registers spilled and was slower).
+// SM: the extra warps hide more of that latency (32 registers spilled and was
+// slower).  There the texels are read four at a time: eight at once spill at 40
+// registers, and with 48 registers and 5 blocks they are slower on 16 x 16 maps.
+// The stage, with the texels tested one by one / eight at once at 40 / at 48
+// registers / four at a time at 40: 100 beams of 16 x 16 maps 16.9 / 14.2 / 12.9 /
+// 12.4 ms; 24 beams of 20 x 20 (two blocks a map, the second half empty) 4.41 /
+// 4.81 / 4.15 / 4.13 ms; 8 beams of 24 x 24 2.23 / 2.47 / 2.22 / 2.14 ms; 12 beams
+// of 17 x 17 1.93 / 2.07 / 1.76 / 1.82 ms.
 // kThreads 64, for launches that leave SMs idle at 256: the rays spread over four
-// times the blocks, and without a register limit more of a slice's reads are in
-// flight together.  With the eight texel reads free of tests inside the volume:
-// 100-beam torso plan 16.85 -> 14.18 ms, one slab beam 142 -> 117 us, four 32 x 32
-// fields 480 -> 400 us.
+// times the blocks, and without a register limit a slice's reads are in flight
+// together.  One slab beam 140 -> 113 us, four 32 x 32 fields 408 -> 307 us (324
+// with four texels at a time).
 template <bool kSkipDark, int kThreads>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 6 : 4) terma_kernel(const fd2_beam_t* __restrict__ beams,
                                                     const float* const* __restrict__ fluence,
@@ -120,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 6 : 4) terma_kerne
             cn.x += sn.x;
             cn.y += sn.y;
             cn.z += sn.z;
-            float d = trilinear(density, nx, ny, nz, cn.x, cn.y, cn.z);
+            float d = trilinear<kThreads != 256>(density, nx, ny, nz, cn.x, cn.y, cn.z);
             rpl += d * stn;
             davg += d;
             sxd += k;
