@@ -1218,6 +1218,39 @@ int common_map(int side, const fd2_beam_t& b) {
 
 }  // namespace
 
+// Forward zenith bins of a kernel and its azimuths.
+static ConeAngles forward_angles(const fd2_cccs_kernel* k) {
+    ConeAngles ang{};
+    for (int t = 0; t < k->n_theta; t++)
+        if ((double)k->theta[t] <= 1.5707963267948966) ang.theta[ang.n_theta_fwd++] = k->theta[t];  // DoseComp.cu:265
+    ang.n_phi = k->n_phi;
+    for (int f = 0; f < k->n_phi; f++) ang.phi[f] = k->phi[f];
+    return ang;
+}
+
+// What of a batch selects its kernel beside the map's pixels and the cones.
+struct BatchForm {
+    int map = -1;        // common map side, else 0
+    bool reach = false;  // Reach::admits
+    int cluster = 0;     // spread_cluster under schedule 1
+};
+static BatchForm batch_form(const fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams, const ConeAngles& ang) {
+    BatchForm f;
+    Reach reach(ang);
+    for (size_t i = 0; i < n_beams; i++) {
+        if (f.map != 0) f.map = common_map(f.map, h_beams[i]);
+        reach.add(h_beams[i]);
+    }
+    f.reach = reach.admits();
+    f.cluster = spread_cluster(f.map, ang.n_phi, (unsigned)(n_beams * ang.n_theta_fwd), ctx->sm_count);
+    return f;
+}
+
+int cccs_form(const fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams, const fd2_cccs_kernel* k) {
+    const BatchForm f = batch_form(ctx, n_beams, h_beams, forward_angles(k));
+    return f.cluster | (f.map > 0 ? 0 : 8) | (f.reach ? 0 : 16);
+}
+
 int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams, const fd2_beam_t* d_beams,
                      const float* const* d_terma, const float* const* d_dens, float* const* d_dose,
                      const fd2_cccs_kernel* k, int schedule, cudaStream_t stream, const int* d_order) {
@@ -1245,11 +1278,7 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
     }
     FD2_REQUIRE(maxP > 0 && maxP <= 1024, FD2_ERR_INVALID_ARGUMENT, "dose_compute: fmap of %d pixels (1..1024)", maxP);
     // direction table [beam][theta_fwd][phi] as float4, evaluated on the device
-    ConeAngles ang{};
-    ang.n_theta_fwd = (int)fwd.size();
-    ang.n_phi = k->n_phi;
-    for (size_t t = 0; t < fwd.size(); t++) ang.theta[t] = k->theta[fwd[t]];
-    for (int f = 0; f < k->n_phi; f++) ang.phi[f] = k->phi[f];
+    const ConeAngles ang = forward_angles(k);
     size_t dir_bytes = n_beams * fwd.size() * k->n_phi * sizeof(float4);
     size_t plane_stride = (size_t)maxP * maxL;
     size_t plane_bytes = schedule == 1 ? n_beams * fwd.size() * plane_stride * sizeof(float) : 0;
@@ -1261,11 +1290,8 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
     // slices a zenith pass skips must contribute zero
     if (plane_bytes) FD2_CHECK_CUDA(cudaMemsetAsync(d_planes, 0, plane_bytes, stream));
     const unsigned blocks = (unsigned)(schedule == 1 ? n_beams * fwd.size() : n_beams);
-    int map = -1;
-    for (size_t i = 0; i < n_beams && map != 0; i++) map = common_map(map, h_beams[i]);
-    Reach reach(ang);
-    for (size_t i = 0; i < n_beams; i++) reach.add(h_beams[i]);
-    const int cluster = schedule == 1 ? spread_cluster(map, k->n_phi, blocks, ctx->sm_count) : 0;
+    const BatchForm form = batch_form(ctx, n_beams, h_beams, ang);
+    const int map = form.map, cluster = schedule == 1 ? form.cluster : 0;
     if (cluster && map <= 24)
         FD2_TRY((launch_spread<5, false, true, 4>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
                                                   d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
@@ -1276,8 +1302,8 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
         FD2_TRY((launch_spread<8, true, false, 4>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
                                                   d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
     else
-        FD2_TRY(launch_march(map, reach.admits(), maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp, schedule,
-                             d_planes, plane_stride, ctx->d_status, schedule == 1 ? nullptr : d_order));
+        FD2_TRY(launch_march(map, form.reach, maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp,
+                             schedule, d_planes, plane_stride, ctx->d_status, schedule == 1 ? nullptr : d_order));
     ctx->launches += 2;  // direction table + march
     if (schedule == 1) {
         dim3 grid(std::max(1, std::min(64, (int)((plane_stride + 255) / 256))), (unsigned)n_beams);
@@ -1339,11 +1365,7 @@ extern "C" int fd2_dose_compute(fd2_context* ctx, size_t fmap_npixels, size_t n_
 extern "C" int fd2_cccs_cone_directions(fd2_context* ctx, const fd2_cccs_kernel* k, size_t n_beams,
                                         const fd2_beam_t* h_beams, float* h_out, size_t n_out) {
     FD2_REQUIRE(ctx && k && h_beams && h_out, FD2_ERR_INVALID_ARGUMENT, "cone_directions: null argument");
-    fd2::ConeAngles ang{};
-    for (int t = 0; t < k->n_theta; t++)
-        if ((double)k->theta[t] <= 1.5707963267948966) ang.theta[ang.n_theta_fwd++] = k->theta[t];
-    ang.n_phi = k->n_phi;
-    for (int f = 0; f < k->n_phi; f++) ang.phi[f] = k->phi[f];
+    const fd2::ConeAngles ang = fd2::forward_angles(k);
     const size_t n = n_beams * ang.n_theta_fwd * ang.n_phi;
     FD2_REQUIRE(n_out >= 4 * n, FD2_ERR_CAPACITY, "cone_directions: need %zu floats", 4 * n);
     if (!n) return FD2_OK;

@@ -180,17 +180,20 @@ void make_column_info(const fd2_beam_t& b, const fd2_volume_t* vol, ColumnInfo& 
 }
 
 // The CCCS march of a batch under the context's tuned schedule.  Batches are
-// keyed by shape (beamlets to the nearest power of two, map pixels, cone
-// counts); the first batch of a shape runs both schedules -- one block per
+// keyed by shape (beamlets down to a power of two, map pixels, cone counts) and
+// by the kernel they take (the spread march is taken up to an exact count of
+// beamlets, inside a power of two); the first batch of a key runs both schedules -- one block per
 // beamlet over all zenith bins, and one block per (beamlet, zenith bin) -- and
-// keeps the faster for the shape.  The two give bitwise identical doses, so
+// keeps the faster for the key.  The two give bitwise identical doses, so
 // the batch keeps the second run's result (its dose buffer is cleared in
 // between).
-static int tuned_cccs(fd2_context* ctx, size_t nb, int P, const fd2_cccs_kernel* k, cudaStream_t st,
+static int tuned_cccs(fd2_context* ctx, size_t nb, const fd2_beam_t* h_beams, int P, const fd2_cccs_kernel* k,
+                      cudaStream_t st,
                       const std::function<int(int)>& run, float* dD, size_t n_dose) {
     int bucket = 0;
     while (((size_t)1 << (bucket + 1)) <= nb) bucket++;
-    const uint64_t key = (uint64_t)bucket | (uint64_t)P << 8 | (uint64_t)k->n_phi << 24 | (uint64_t)k->n_theta << 40;
+    const uint64_t key = (uint64_t)bucket | (uint64_t)P << 8 | (uint64_t)k->n_phi << 24 | (uint64_t)k->n_theta << 40 |
+                         (uint64_t)cccs_form(ctx, nb, h_beams, k) << 48;
     auto it = ctx->cccs_schedule.find(key);
     if (it != ctx->cccs_schedule.end()) return run(it->second);
     cudaEvent_t ev[3];
@@ -775,7 +778,7 @@ int fd2_dose_mat_construct(fd2_context* ctx, size_t n_beams, const uint32_t* n_p
                 } else if (params.cccs_schedule == -2) {
                     FD2_TRY(run(cccs_auto_schedule(ctx, nb)));
                 } else {
-                    FD2_TRY(tuned_cccs(ctx, nb, P, kernel, st, run, dD, off[nb]));
+                    FD2_TRY(tuned_cccs(ctx, nb, beams.data() + b0, P, kernel, st, run, dD, off[nb]));
                 }
                 t.stop();
             }

@@ -44,5 +44,9 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
 // march), ties in batch order, so a launch's last blocks are its short ones.
 void cccs_longest_first(size_t n_beams, const fd2_beam_t* h_beams, int* order);
 int cccs_auto_schedule(const fd2_context* ctx, size_t n_beams);
+// The march kernel a batch takes, as far as its map pixels and cones do not say:
+// blocks of a spread cluster (0, 2 or 4) | 8 where the maps are not one square
+// size | 16 where rays reach too far for the voxel-stationary march.
+int cccs_form(const fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams, const fd2_cccs_kernel* k);
 
 }  // namespace fd2

@@ -174,7 +174,9 @@ uint64_t fd2_context_launch_count(const fd2_context* ctx);
  * measured once per batch shape): up to cap (shape key, schedule) pairs and
  * their number in *n; *runs = batches on which both schedules were timed.
  * Key bits: 0-7 log2 of the batch's beamlets, 8-23 map pixels, 24-39 azimuths,
- * 40- zenith bins.
+ * 40-47 zenith bins, 48- what else selects the kernel (blocks of a spread
+ * cluster, | 8 where the maps are not one square size, | 16 where rays reach
+ * too far for the voxel-stationary march).
  */
 int fd2_context_tuned_schedules(const fd2_context* ctx, size_t cap, uint64_t* keys, int32_t* schedules, size_t* n,
                                 uint64_t* runs);

@@ -153,6 +153,35 @@ def test_tuned_cccs_schedule(ctx):
     c2.close()
 
 
+def test_tuned_schedule_is_kept_per_kernel(ctx):
+    """Batches of 16 and of 24 beamlets of 20 x 20 maps share a power of two, but
+    with 8 zenith bins and 6 azimuths only up to 18 take the spread march on 148
+    SMs: each kernel is timed for itself."""
+    import torch
+
+    from fastdose_b200 import phantoms
+    from fastdose_b200.types import make_bundle
+
+    c2 = api.Context(0)
+    ph = phantoms.torso_phantom(seed=2, dim=(40, 40, 32))
+    dens, sp = api.Density(c2, ph.density, ph.volume), api.Spectrum(c2, phantoms.synthetic_spectrum())
+    kn = api.Kernel(c2, phantoms.synthetic_kernel(n_theta=8, n_phi=6))
+    bund = make_bundle(ph.centre(), (0.4, 0.2, 0.1), fluence_dim=5, beamlet_size=0.5, sub_fluence_dim=20, sub_fluence_on=4)
+    limit = 2 * torch.cuda.get_device_properties(0).multi_processor_count // (2 * 8)
+    assert 16 <= limit - 2 and limit + 5 <= 25
+    for n, runs in ((limit - 2, 1), (limit - 1, 1), (limit + 4, 2), (limit + 5, 2)):
+        flags = np.zeros(25, np.uint8)
+        flags[:n] = 1
+        m = api.DoseMatConstruction(c2, [api.bundle_beamlets(bund, flags, ph.volume)], api.beamlet_fluence(bund), dens,
+                                    sp, kn)
+        m.close()
+        assert c2.tuned_schedules()[1] == runs
+    assert sorted(k >> 48 for k in c2.tuned_schedules()[0]) == [0, 2]
+    for h in (dens, sp, kn):
+        h.close()
+    c2.close()
+
+
 @pytest.mark.parametrize("vt,sched", [("f32", 0), ("f16", 1), ("f32", -1)])
 def test_graph_captured_construction_matches_direct(vt, sched):
     """Batches launched as captured CUDA graphs give the matrix of direct
