@@ -1176,11 +1176,13 @@ int launch_march(int map, bool reach_ok, int maxP, int n_phi, unsigned blocks, c
 
 // The spread march: 17 x 17 to 32 x 32 maps, where an azimuth's rays keep a warp
 // busy for hundreds of instructions a step, in a batch under schedule 1 whose
-// (beamlet, zenith bin) pairs leave SMs without a block.
+// (beamlet, zenith bin) pairs leave SMs without a block.  A device (or a slice of
+// one) that has no room for the clusters refuses the launch: *taken is false
+// then, and the plain march gives the same dose.
 template <int RPL, bool kCols, bool kTab, int kWpa>
 int launch_spread(unsigned blocks, int cluster, int n_phi, size_t maxP, cudaStream_t st, const fd2_beam_t* d_beams,
                   const float* const* T, const float* const* R, float* const* D, const float4* dirs,
-                  const ConeParams& cp, float* planes, size_t plane_stride, DeviceStatus* status) {
+                  const ConeParams& cp, float* planes, size_t plane_stride, DeviceStatus* status, bool* taken) {
     const size_t shm = (size_t)(1 + n_phi / cluster) * maxP * sizeof(float2);
     FD2_CHECK_CUDA(cudaFuncSetAttribute(cccs_kernel<RPL, kCols, kTab, kWpa>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)shm));
@@ -1195,8 +1197,9 @@ int launch_spread(unsigned blocks, int cluster, int n_phi, size_t maxP, cudaStre
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    FD2_CHECK_CUDA(cudaLaunchKernelEx(&cfg, cccs_kernel<RPL, kCols, kTab, kWpa>, d_beams, T, R, D, dirs, cp, 1, planes,
-                                      plane_stride, status, (const int*)nullptr));
+    *taken = cudaLaunchKernelEx(&cfg, cccs_kernel<RPL, kCols, kTab, kWpa>, d_beams, T, R, D, dirs, cp, 1, planes,
+                                plane_stride, status, (const int*)nullptr) == cudaSuccess;
+    if (!*taken) cudaGetLastError();
     return FD2_OK;
 }
 
@@ -1292,16 +1295,17 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
     const unsigned blocks = (unsigned)(schedule == 1 ? n_beams * fwd.size() : n_beams);
     const BatchForm form = batch_form(ctx, n_beams, h_beams, ang);
     const int map = form.map, cluster = schedule == 1 ? form.cluster : 0;
+    bool taken = false;
     if (cluster && map <= 24)
         FD2_TRY((launch_spread<5, false, true, 4>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
-                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
+                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status, &taken)));
     else if (cluster && k->n_phi / cluster <= 3)
         FD2_TRY((launch_spread<4, true, false, 8>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
-                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
+                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status, &taken)));
     else if (cluster)
         FD2_TRY((launch_spread<8, true, false, 4>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
-                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status)));
-    else
+                                                  d_dirs, cp, d_planes, plane_stride, ctx->d_status, &taken)));
+    if (!taken)
         FD2_TRY(launch_march(map, form.reach, maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp,
                              schedule, d_planes, plane_stride, ctx->d_status, schedule == 1 ? nullptr : d_order));
     ctx->launches += 2;  // direction table + march

@@ -3,7 +3,8 @@
 // preloaded before the library, it counts two devices, hands out host memory
 // and launches nothing.  It keeps each allocation's device and whether that
 // device was waited for since; fake_report() counts the frees that cudaFreeAsync
-// would get wrong.
+// would get wrong.  fake_launches() counts the launches, and fake_refuse() makes
+// those with attributes (clusters) fail.
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
@@ -18,6 +19,8 @@ struct Block {
 std::map<void*, Block> blocks;
 std::map<cudaMemPool_t, int> pools;
 int current = 0, wrong_device = 0, not_waited = 0;
+int plain = 0, extended = 0, refuse = 0;
+cudaError_t last = cudaSuccess;
 }  // namespace
 
 extern "C" {
@@ -29,6 +32,12 @@ void fake_report(int* live, int* wrong, int* early, int* cur) {
     *cur = current;
 }
 
+void fake_refuse(int on) { refuse = on; }
+void fake_launches(int* p, int* x) {
+    *p = plain;
+    *x = extended;
+}
+
 cudaError_t cudaGetDeviceCount(int* n) { return *n = 2, cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { return *d = current, cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { return current = d, cudaSuccess; }
@@ -37,8 +46,11 @@ cudaError_t cudaGetDeviceProperties_v2(cudaDeviceProp* p, int) {
     p->multiProcessorCount = 148;
     return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaPeekAtLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = last;
+    return last = cudaSuccess, e;
+}
+cudaError_t cudaPeekAtLastError() { return last; }
 
 cudaError_t cudaDeviceSynchronize() {
     for (auto& b : blocks)
@@ -93,6 +105,10 @@ cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return c
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) {
     return *n = 1, cudaSuccess;
 }
-unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void*) { return 1; }  // no launch
+unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void*) { return plain++, 1; }  // no launch
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) {
+    if (refuse) return last = cudaErrorInvalidClusterSize;
+    return extended++, cudaSuccess;
+}
 
 }  // extern "C"

@@ -1,7 +1,10 @@
-"""Matrices, problems and densities destroyed while another device is current:
+"""What a library on one healthy device does not meet, on the host against a
+stand-in for the CUDA runtime (fake_cudart.cpp).
+
+Matrices, problems and densities destroyed while another device is current:
 their memory goes back to its own device's pool, after a wait for that device,
-and the caller's device stays current.  Runs on the host against a stand-in for
-the CUDA runtime with two devices (fake_cudart.cpp)."""
+and the caller's device stays current.  And a device that refuses a cluster
+launch: the plain march is launched in its place."""
 import os
 import shutil
 import subprocess
@@ -70,6 +73,41 @@ assert cur == now, f"device {cur} is current, not {now}"
 print("HANDLES OK")
 """
 
+CLUSTER = """
+import ctypes as C, sys
+import numpy as np
+fake, refuse = C.CDLL(sys.argv[1]), int(sys.argv[2])
+from fastdose_b200 import _lib, phantoms
+from fastdose_b200.types import BEAM_DTYPE
+lib = _lib.get()
+ok = lambda rc: _lib.check(rc, "call")
+ctx, kern = C.c_void_p(), C.c_void_p()
+ok(lib.fd2_context_create(0, C.byref(ctx)))
+k = phantoms.synthetic_kernel(n_phi=8)
+p = lambda a: a.ctypes.data
+f = [np.ascontiguousarray(a, np.float32) for a in (k.theta, k.A, k.a, k.B, k.b, k.phi)]
+ok(lib.fd2_kernel_create(ctx, len(f[0]), *map(p, f[:5]), len(f[5]), p(f[5]), C.byref(kern)))
+b = np.zeros(1, BEAM_DTYPE)
+b["beamlet_size"] = 0.3
+b["fmap_size"] = int(sys.argv[3])
+b["sad"], b["long_spacing"], b["long_dim"] = 100.0, 0.25, 20
+b["TermaBEV_pitch"] = b["DensityBEV_pitch"] = 4 * int(sys.argv[3]) ** 2
+table = np.zeros(1, np.uint64)
+
+def launches():
+    v = [C.c_int(), C.c_int()]
+    fake.fake_launches(C.byref(v[0]), C.byref(v[1]))
+    return [i.value for i in v]
+
+was = launches()
+fake.fake_refuse(refuse)
+ok(lib.fd2_dose_compute(ctx, int(sys.argv[3]) ** 2, 1, p(b), p(table), p(table), p(table), kern, None))
+plain, cluster = (n - w for n, w in zip(launches(), was))
+# the direction table, the march, and the reduction of the zenith bins' planes
+assert (plain, cluster) == ((3, 0) if refuse else (2, 1)), (plain, cluster)
+print("CLUSTER OK")
+"""
+
 
 @pytest.fixture(scope="module")
 def fake(tmp_path_factory):
@@ -88,6 +126,15 @@ def test_handles_return_memory_to_their_own_device(fake, kind, own, now):
     p = subprocess.run([sys.executable, "-c", CHILD, fake, kind, str(own), str(now)], env=env, cwd=ROOT,
                        capture_output=True, text=True, timeout=300)
     assert p.returncode == 0 and "HANDLES OK" in p.stdout, p.stdout + p.stderr
+
+
+@pytest.mark.parametrize("side", [20, 32])
+@pytest.mark.parametrize("refuse", [0, 1])
+def test_a_refused_cluster_launch_becomes_a_plain_one(fake, refuse, side):
+    env = dict(os.environ, LD_PRELOAD=fake, PYTHONPATH=ROOT)
+    p = subprocess.run([sys.executable, "-c", CLUSTER, fake, str(refuse), str(side)], env=env, cwd=ROOT,
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and "CLUSTER OK" in p.stdout, p.stdout + p.stderr
 
 
 def test_the_library_uses_the_shared_runtime():
