@@ -181,7 +181,7 @@ int launch_terma(fd2_context* ctx, size_t fmap_npixels, size_t n_beams, const fd
     // blocks per beam cover up to 1024 pixels (the reference's bound: one block per
     // beam); fewer than two blocks of 256 an SM go out as blocks of 64
     const size_t blocks256 = n_beams * ((fmap_npixels + 255) / 256);
-    const unsigned threads = blocks256 < 2 * 148 ? 64 : 256;
+    const unsigned threads = blocks256 < 2 * (size_t)ctx->sm_count ? 64 : 256;
     dim3 grid((unsigned)n_beams, (unsigned)((fmap_npixels + threads - 1) / threads)), block(threads);
     auto kernel = threads == 64 ? (fluence_skip ? terma_kernel<true, 64> : terma_kernel<false, 64>)
                                 : (fluence_skip ? terma_kernel<true, 256> : terma_kernel<false, 256>);
