@@ -676,8 +676,24 @@ def _lat_stats(lat_s):
             "max_ms": float(lat.max()), "requests": int(lat.size)}
 
 
+def served_stats(stats, beamlets):
+    """A rate's figures: of a size that does not depend on the requests, so that
+    the bench line stays short."""
+    lat = np.array([s["end_ms"] - s["submit_ms"] for s in stats]) * 1e-3
+    span_s = (max(s["end_ms"] for s in stats) - min(s["submit_ms"] for s in stats)) * 1e-3
+    return dict(_lat_stats(lat), beamlets_per_s=beamlets / span_s,
+                queue_p50_ms=float(np.percentile([s["start_ms"] - s["submit_ms"] for s in stats], 50)))
+
+
+def served_timeline(stats):
+    """Per request (arrival order): beamlets, worker, submit ms (from the first
+    submit), queue ms, run ms."""
+    return [[int(s["beamlets"]), int(s["worker"]), round(s["submit_ms"] - stats[0]["submit_ms"], 1),
+             round(s["start_ms"] - s["submit_ms"], 1), round(s["end_ms"] - s["start_ms"], 1)] for s in stats]
+
+
 def served_leg(ctx, rates=(1.0, 5.0, 10.0, 20.0, 50.0), n_requests=200, seconds_per_rate=20.0, seed=11, workers=2,
-               plain_requests=30, graph_rate=10.0):
+               plain_requests=30, graph_rate=10.0, timeline_file=None):
     """p50/p99 plan latency (arrival -> dose-loading matrix on the device) and
     beamlets/s of the service under Poisson arrivals at each rate, over
     min(n_requests, max(30, rate * seconds_per_rate)) requests (seconds_per_rate
@@ -761,7 +777,7 @@ def served_leg(ctx, rates=(1.0, 5.0, 10.0, 20.0, 50.0), n_requests=200, seconds_
                    for r in reqs[:min(len(reqs), 48)]]
         for t in tickets:
             svc.wait(t)[0].close()
-    arrivals = {}
+    arrivals, timelines = {}, {}
 
     def run_rate(lam, n, graph):
         sub = reqs[:n]
@@ -787,16 +803,8 @@ def served_leg(ctx, rates=(1.0, 5.0, 10.0, 20.0, 50.0), n_requests=200, seconds_
                 m, s = svc.wait(t)
                 m.close()
                 stats.append(s)
-        lat = np.array([s["end_ms"] - s["submit_ms"] for s in stats]) * 1e-3
-        span_s = (max(s["end_ms"] for s in stats) - min(s["submit_ms"] for s in stats)) * 1e-3
-        return arr, dict(_lat_stats(lat), beamlets_per_s=sum(n_bl[:n]) / span_s, workers=workers, graph=graph,
-                         queue_p50_ms=float(np.percentile([s["start_ms"] - s["submit_ms"] for s in stats], 50)),
-                         # per request (arrival order): beamlets, worker, submit ms (from the first
-                         # submit), queue ms, run ms
-                         timeline=[[int(s["beamlets"]), int(s["worker"]), round(s["submit_ms"] - stats[0]["submit_ms"], 1),
-                                    round(s["start_ms"] - s["submit_ms"], 1), round(s["end_ms"] - s["start_ms"], 1)]
-                                   for s in stats],
-                         clocks=clk.summary())
+        timelines[f"rate_{lam:g}_per_s" + ("_graph" if graph else "")] = served_timeline(stats)
+        return arr, dict(served_stats(stats, sum(n_bl[:n])), workers=workers, graph=graph, clocks=clk.summary())
 
     for lam in rates:
         n = len(reqs) if seconds_per_rate <= 0 else min(len(reqs), max(30, int(lam * seconds_per_rate)))
@@ -821,9 +829,11 @@ def served_leg(ctx, rates=(1.0, 5.0, 10.0, 20.0, 50.0), n_requests=200, seconds_
     if graph_rate and f"rate_{graph_rate:g}_per_s" in out:
         n = min(len(reqs), max(30, int(graph_rate * seconds_per_rate))) if seconds_per_rate > 0 else len(reqs)
         _, on = run_rate(graph_rate, n, graph=True)  # the same arrivals, one graph per construction batch
-        on.pop("timeline")
         out[f"rate_{graph_rate:g}_per_s"]["service_with_graphs"] = on
     svc.close()
+    if timeline_file:
+        with open(timeline_file, "w") as f:
+            json.dump(timelines, f)
     return out
 
 
@@ -1178,7 +1188,7 @@ def run_fd2(args, rank, world):
         ctx.release()
         line["served"] = served_leg(ctx, rates=tuple(float(r) for r in args.served_rates.split(",")),
                                     n_requests=args.served_requests, seconds_per_rate=args.served_seconds,
-                                    workers=args.served_workers)
+                                    workers=args.served_workers, timeline_file=args.served_timeline)
     if rank == 0 and not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(cfg, beamlets, fluence, args.cpu_seconds, os.cpu_count() or 1)[0]
     if rank == 0:
@@ -1212,6 +1222,7 @@ def main():
                     help="beamlets per construction batch of the end-to-end leg (-1: a sixth of the plan, >= 4096)")
     ap.add_argument("--c4", action="store_true", help="run the multi-isocentre configuration alone")
     ap.add_argument("--only-served", action="store_true", help="run the served leg alone")
+    ap.add_argument("--served-timeline", default=None, help="file for every request's times of the served leg")
     args = ap.parse_args()
     if args.c4:
         import torch
@@ -1250,7 +1261,8 @@ def main():
             print(json.dumps({"served": served_leg(ctx, rates=tuple(float(r) for r in args.served_rates.split(",")),
                                                    n_requests=args.served_requests,
                                                    seconds_per_rate=args.served_seconds,
-                                                   workers=args.served_workers, plain_requests=args.plain_requests)}),
+                                                   workers=args.served_workers, plain_requests=args.plain_requests,
+                                                   timeline_file=args.served_timeline)}),
                   flush=True)
         return
     world = int(os.environ.get("WORLD_SIZE", "1"))
