@@ -88,6 +88,7 @@ struct fd2_matrix {
     float* d_xs = nullptr;           // [cols] x times the column scale
     int32_t* d_zrow = nullptr;       // rows the product itself does not write: empty, or only in carries
     int* d_nz = nullptr;             // number of those rows
+    int n_zrows = 0;                 // and on the host
 
     fd2::ColView cols_view() const { return fd2::ColView{d_col, d_col16, d_cbase, d_exc, interleaved}; }
 };

@@ -978,6 +978,8 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             }
         }
     }
+    if (!rc && cudaMemcpyAsync(&m->n_zrows, m->d_nz, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+        rc = FD2_ERR_CUDA;
     if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
     cleanup();
     if (rc && rc != FD2_ERR_OUT_OF_MEMORY) set_error("matrix_finalize: %s", cudaGetErrorString(cudaGetLastError()));
@@ -1113,7 +1115,7 @@ int fd2_matrix_info(const fd2_matrix* m, fd2_matrix_info_t* info) {
     const int64_t col_bytes =
         m->index_format == FD2_INDEX_PACKED16 ? pad * 2 + m->n_chunks * 4 + m->n_exc * kChunk * 4 : pad * 4;
     info->device_bytes = pad * (int64_t)value_size(m->value_type) + col_bytes + pad / 8 + m->n_chunks * 8 +
-                         m->n_nzrows * 4 + ns * (int64_t)sizeof(float);
+                         m->n_nzrows * 4 + m->n_zrows * (int64_t)4 + ns * (int64_t)sizeof(float);
     return FD2_OK;
 }
 

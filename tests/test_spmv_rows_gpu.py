@@ -50,6 +50,18 @@ def test_rows_of_one_length(ctx, cols, length):
             np.testing.assert_array_equal(a, b)
 
 
+def test_device_bytes_count_the_rows_a_product_clears(ctx):
+    """Empty rows are in the list each product reads: 4 bytes a row."""
+    rng = np.random.default_rng(2)
+    col = np.sort(rng.choice(900, 300, replace=False)).astype(np.int64)
+    val = np.ones(300, np.float32)
+    size = []
+    for empty in (0, 1000):
+        off = np.concatenate([[0, 300], np.full(empty, 300)]).astype(np.int64)
+        size.append(optimize.Matrix.from_csr(ctx, off, col, val, 900).info()["device_bytes"])
+    assert size[1] - size[0] == 4 * 1000
+
+
 def test_matrix_memory_waits_for_products_and_outlives_the_context():
     """A matrix is destroyed while its product runs on another stream, and after
     its context; its memory is not handed to the next matrix before that."""
