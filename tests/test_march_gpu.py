@@ -17,8 +17,8 @@ from fastdose_b200.types import make_bundle
 pytestmark = pytest.mark.gpu
 
 
-def _batch(ctx, ph, side, on, dens, spec, gantry, count=6):
-    bund = make_bundle(ph.centre(), (gantry, 0.3, 0.1), sad=100.0, fluence_dim=count, beamlet_size=0.5,
+def _batch(ctx, ph, side, on, dens, spec, gantry, count=6, beamlet_size=0.5):
+    bund = make_bundle(ph.centre(), (gantry, 0.3, 0.1), sad=100.0, fluence_dim=count, beamlet_size=beamlet_size,
                        sub_fluence_dim=side, sub_fluence_on=on, long_spacing=0.25)
     flags = np.zeros(count * count, np.uint8)
     flags[:: max(1, count * count // count)] = 1  # distinct beamlet sizes: distinct ray paths
@@ -37,8 +37,16 @@ def test_march_matches_the_per_ray_instance(ctx, side, on, n_phi):
     spec = api.Spectrum(ctx, phantoms.synthetic_spectrum())
     kern = api.Kernel(ctx, phantoms.synthetic_kernel(n_phi=n_phi))
     b = _batch(ctx, ph, side, on, dens, spec, 0.7)
-    api.DoseComputeCollective(ctx, b, kern)  # one map size: the march
-    # the same beams beside one of another map size: the general instance
+    got, ref = _march_and_general(ctx, ph, side, dens, spec, kern, b)
+    assert torch.all((got - ref).abs() <= 2e-5 * ref + 1e-6 * ref.max())
+
+
+def _march_and_general(ctx, ph, side, dens, spec, kern, b):
+    """The batch's dose, and that of the same beams beside one of another map size,
+    which the general instance marches."""
+    import torch
+
+    api.DoseComputeCollective(ctx, b, kern)
     other = _batch(ctx, ph, 10, 2, dens, spec, 1.9, count=1)
     dose = [torch.zeros_like(b.dose), torch.zeros_like(other.dose)]
     beams = torch.cat([b.d_beams, other.d_beams])
@@ -56,7 +64,61 @@ def test_march_matches_the_per_ray_instance(ctx, side, on, n_phi):
     got, ref = b.dose.double(), dose[0].double()
     assert float(ref.max()) > 0
     assert torch.all((got == 0) == (ref == 0))
-    assert torch.all((got - ref).abs() <= 2e-5 * ref + 1e-6 * ref.max())
+    return got, ref
+
+
+def _reach(kern_src, b):
+    """Voxels the widest cone moves sideways in a slice, and over the batch's longest beam."""
+    t = np.tan(np.float64(kern_src.theta)).max() * max(np.abs(np.cos(kern_src.phi)).max(), np.abs(np.sin(kern_src.phi)).max())
+    per = float((b.beams["long_spacing"] * t / b.beams["beamlet_size"].min(axis=1)).max())
+    return per, per * int(b.beams["long_dim"].max())
+
+
+# Coordinates of up to C voxels: a segment's lateral offset is the difference of two
+# products of that size, each of some three roundings, so a step's length is off by
+# 6 C 2^-24 voxels, and steps are half a voxel or longer on average
+def _far_bound(reach):
+    return 12 * reach * 2.0 ** -24 + 2e-5
+
+
+@pytest.mark.parametrize("side,on", [(8, 2), (12, 4), (16, 4)])
+def test_march_of_slices_with_several_rounds_of_path_records(ctx, side, on):
+    """Pixels of 0.05 cm: the widest bin takes more than 40 steps a slice (the
+    records of one round), up to some 200."""
+    import torch
+
+    ph = phantoms.torso_phantom(seed=side, dim=(40, 36, 32))
+    dens = api.Density(ctx, ph.density, ph.volume)
+    spec = api.Spectrum(ctx, phantoms.synthetic_spectrum())
+    src = phantoms.synthetic_kernel(n_theta=20, n_phi=6)
+    kern = api.Kernel(ctx, src)
+    b = _batch(ctx, ph, side, on, dens, spec, 0.7, beamlet_size=0.05 * on)
+    per, total = _reach(src, b)
+    assert per > 100 and per < 500 and total < 15000
+    got, ref = _march_and_general(ctx, ph, side, dens, spec, kern, b)
+    assert torch.all((got - ref).abs() <= _far_bound(total) * ref + 1e-6 * ref.max())
+
+
+@pytest.mark.parametrize("side,on", [(8, 2), (16, 4)])
+def test_batches_that_reach_too_far_take_the_other_march(ctx, side, on):
+    """Rays that move more than 15000 voxels sideways: the half-table instance, as
+    the tuned key tells, with the dose of the general one."""
+    import torch
+
+    ph = phantoms.torso_phantom(seed=side, dim=(72, 64, 56))
+    dens = api.Density(ctx, ph.density, ph.volume)
+    spec = api.Spectrum(ctx, phantoms.synthetic_spectrum())
+    src = phantoms.synthetic_kernel(n_theta=24, n_phi=6)
+    kern = api.Kernel(ctx, src)
+    b = _batch(ctx, ph, side, on, dens, spec, 0.7, count=3, beamlet_size=0.025 * on)
+    per, total = _reach(src, b)
+    assert 15000 < total < 28000, total  # beyond 2^15 voxels the reference's 1e-3 step slack is lost
+    got, ref = _march_and_general(ctx, ph, side, dens, spec, kern, b)
+    assert torch.all((got - ref).abs() <= _far_bound(total) * ref + 1e-6 * ref.max())
+    c2 = api.Context(0)
+    api.DoseMatConstruction(c2, [b.beams], np.ones(side * side, np.float32), dens, spec, kern).close()
+    assert [k >> 48 for k in c2.tuned_schedules()[0]] == [16]
+    c2.close()
 
 
 @pytest.mark.parametrize("n_phi", [4, 6, 8])
