@@ -554,7 +554,7 @@ int fd2_bev2pvcs(fd2_context* ctx, const fd2_beam_t* h_beam, const fd2_density* 
     ColumnInfo ci;
     make_column_info(*h_beam, nullptr, ci);
     return launch_bev2pvcs(ci, density->vol, d_bev, d_out, out_pitch_bytes / sizeof(float), 0, 0.0f,
-                           (cudaStream_t)stream);
+                           ctx->sm_count, (cudaStream_t)stream);
 }
 
 int fd2_bev2pvcs_supersampling(fd2_context* ctx, const fd2_beam_t* h_beam, const fd2_density* density,
@@ -567,7 +567,7 @@ int fd2_bev2pvcs_supersampling(fd2_context* ctx, const fd2_beam_t* h_beam, const
     ColumnInfo ci;
     make_column_info(*h_beam, nullptr, ci);
     return launch_bev2pvcs(ci, density->vol, d_bev, d_out, out_pitch_bytes / sizeof(float), ssfactor, extent,
-                           (cudaStream_t)stream);
+                           ctx->sm_count, (cudaStream_t)stream);
 }
 
 int fd2_dose_mat_construct(fd2_context* ctx, size_t n_beams, const uint32_t* n_per_beam, const fd2_beam_t* h_beamlets,

@@ -17,6 +17,7 @@
 // frustum, tests them against a cheap bound, and emits its nonzeros straight
 // into CSR order (voxel index ascending) with a block-wide scan.
 #include <algorithm>
+#include <cmath>
 
 #include <cub/block/block_reduce.cuh>
 #include <cub/block/block_scan.cuh>
@@ -100,24 +101,26 @@ __device__ __forceinline__ float3 to_bev_grid(const ColumnInfo& ci, float3 p) {
     return make_float3(v.x / (ci.bsx * k) + ci.hx, (v.y - ci.lim_min) * ci.inv_ls, v.z / (ci.bsy * k) + ci.hy);
 }
 
-// Dense volume: a warp takes 32 voxels of a row, a thread kDenseZ planes of
+// Dense volume: a warp takes 32 voxels of a row, a thread up to kDenseZ planes of
 // them.  Most of the volume lies outside the beam, so the pass is bound by
 // finding that out and writing zeros: a voxel more than half a texel off the map
 // or the depths, where the trilinear sample is zero, is told by four comparisons
 // without the two divisions (the margin of 0.01 texels is far more than they
 // round).
+// Fewer than kDenseZ planes where the volume would leave SMs without a block:
+// 64 x 64 x 51 12.3 us with 8 planes, 8.2 with one.
 constexpr int kDenseZ = 8;
 
 __global__ void __launch_bounds__(256) bev2pvcs_kernel(ColumnInfo ci, const float* __restrict__ bev,
                                                        float* __restrict__ out, size_t pitch, int nx, int ny, int nz,
-                                                       float vx, float vy, float vz) {
+                                                       float vx, float vy, float vz, int planes) {
     const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
     if (x >= nx || y >= ny) return;
     const float tx = (ci.hx + 0.51f) * fabsf(ci.bsx * ci.inv_sad), tz = (ci.hy + 0.51f) * fabsf(ci.bsy * ci.inv_sad);
     const float y0 = ci.lim_min - 0.51f * ci.ls, y1 = ci.lim_min + (ci.L + 0.51f) * ci.ls;
-    for (int z0 = blockIdx.z * kDenseZ; z0 < nz; z0 += gridDim.z * kDenseZ)
+    for (int z0 = blockIdx.z * planes; z0 < nz; z0 += gridDim.z * planes)
 #pragma unroll 4
-        for (int z = z0; z < min(z0 + kDenseZ, nz); z++) {
+        for (int z = z0; z < min(z0 + planes, nz); z++) {
             const float3 p = make_float3((x + 0.5f) * vx, (y + 0.5f) * vy, (z + 0.5f) * vz);
             const float3 v = rot(ci.R, make_float3(p.x - ci.src[0], p.y - ci.src[1], p.z - ci.src[2]));
             float val = 0.0f;
@@ -129,59 +132,135 @@ __global__ void __launch_bounds__(256) bev2pvcs_kernel(ColumnInfo ci, const floa
         }
 }
 
-// Supersampled volume.  Only the voxels within `extent` of the beam axis and
-// next to the BEV depths are sampled, about 0.5 % of a 200 x 200 x 160 volume for
-// 2 cm, so the work is found first: the volume is cut into tiles of 4 x 4 x 4
-// voxels, a block's first warp tests 32 tiles, and the block lists a hit tile's
-// voxels.
-// A warp then takes a voxel, its lanes the ss^3 samples: they fall into a few
-// texel cells, so that a load touches two or three cache lines, where 32 voxels
-// side by side touched up to sixteen and the pass was bound by their lookups.
-// The voxel's place in the beam frame is formed in double, the samples' offsets
-// from it in float.
+// Supersampled volume.  Only the voxels within `extent` of the beam axis that may
+// touch the map and the BEV depths are sampled, about 0.5 % of a 200 x 200 x 160
+// volume for 2 cm.  A voxel's place in the beam frame is formed in double, its
+// samples' offsets from it in float.  Leaving out what lies beside the map matters
+// where the extent is the larger: 200 x 200 x 160, 16 x 16 map of 0.25 cm, 5^3
+// samples, 8 cm 517 -> 96 us, 60 cm 5300 -> 92 us.
+struct SsFrame {
+    float vx, vy, vz, extent;
+    float mx, mz;      // lateral half width of the map per unit of depth, half a texel more (past which samples
+                       // are zero) and its rounding
+    float hv, slack;   // half diagonal of a voxel; allowance for rounding
+    float sx, sz;      // texels per unit of lateral distance over depth
+    SsFrame(const ColumnInfo& ci, const fd2_volume_t& v, float extent_)  // on the host, once a launch
+        : vx(v.voxel_size[0]), vy(v.voxel_size[1]), vz(v.voxel_size[2]), extent(extent_) {
+        mx = (ci.hx + 0.51f) * std::fabs(ci.bsx * ci.inv_sad);
+        mz = (ci.hy + 0.51f) * std::fabs(ci.bsy * ci.inv_sad);
+        hv = 0.5f * std::sqrt(vx * vx + vy * vy + vz * vz);
+        slack = 1e-3f + 1e-4f * (4.0f * hv + std::fabs(extent));
+        sx = 1.0f / (ci.bsx * ci.inv_sad);
+        sz = 1.0f / (ci.bsy * ci.inv_sad);
+    }
+    __device__ __forceinline__ float3 at(const ColumnInfo& ci, float x, float y, float z) const {  // voxels -> beam frame
+        return rot(ci.R, make_float3(x * vx - ci.src[0], y * vy - ci.src[1], z * vz - ci.src[2]));
+    }
+    // could a point within d of v lie on the map and the depths?
+    __device__ __forceinline__ bool near_map(const ColumnInfo& ci, float3 v, float d) const {
+        const float y = fabsf(v.y) + d;
+        return !(fabsf(v.x) > mx * y + d) && !(fabsf(v.z) > mz * y + d) && !(v.y < ci.lim_min - ci.ls - d) &&
+               !(v.y > ci.lim_min + (ci.L + 1) * ci.ls + d);
+    }
+    __device__ __forceinline__ bool sampled(const ColumnInfo& ci, int x, int y, int z) const {
+        const float3 v = at(ci, x + 0.5f, y + 0.5f, z + 0.5f);
+        return !(v.x * v.x + v.z * v.z > extent * extent) && near_map(ci, v, hv + slack);
+    }
+    // beam-frame offset of sample s of ss^3 from the voxel centre
+    __device__ __forceinline__ float3 offset(const ColumnInfo& ci, int ss, int s) const {
+        const float inv = 1.0f / ss;
+        const int jk = (int)((s + 0.5f) * inv), k = (int)((jk + 0.5f) * inv);  // s / ss and s / ss^2, s <= 4096
+        const float a = ((s - jk * ss + 0.5f) * inv - 0.5f) * vx, b = ((jk - k * ss + 0.5f) * inv - 0.5f) * vy,
+                    c = ((k + 0.5f) * inv - 0.5f) * vz;
+        return rot(ci.R, make_float3(a, b, c));
+    }
+};
+
+// A voxel's centre in the beam frame, and the BEV dose at an offset from it.
+struct SsVoxel {
+    float cx, cy, cw, cz;  // cw: depth behind the first slice
+    __device__ __forceinline__ SsVoxel(const ColumnInfo& ci, const SsFrame& f, int x, int y, int z) {
+        const double px = (x + 0.5) * f.vx - ci.src[0], py = (y + 0.5) * f.vy - ci.src[1], pz = (z + 0.5) * f.vz - ci.src[2];
+        cx = (float)(ci.R[0] * px + ci.R[1] * py + ci.R[2] * pz);
+        const double dy = ci.R[3] * px + ci.R[4] * py + ci.R[5] * pz;
+        cy = (float)dy;
+        cw = (float)(dy - ci.lim_min);
+        cz = (float)(ci.R[6] * px + ci.R[7] * py + ci.R[8] * pz);
+    }
+    template <typename Index>
+    __device__ __forceinline__ float sample(const ColumnInfo& ci, const SsFrame& f, const float* __restrict__ bev,
+                                            float3 o) const {
+        const float uy = cy + o.y;
+        float r = __fdividef(1.0f, uy);
+        r = fmaf(r, fmaf(-uy, r, 1.0f), r);
+        return bev_trilinear_near<Index>(bev, ci.fx, ci.fy, ci.L, fmaf((cx + o.x) * r, f.sx, ci.hx) - 0.5f,
+                                         fmaf((cz + o.z) * r, f.sz, ci.hy) - 0.5f, fmaf(cw + o.y, ci.inv_ls, -0.5f));
+    }
+};
+
+// Few samples a voxel: a thread takes a voxel.  A warp a voxel leaves most lanes
+// idle up to 2^3 samples, and the listing below costs a small volume more than 3^3
+// samples in turn.  2 cm, this form / the warps: 64 x 64 x 51, 1 sample 7 / 34 us,
+// 2^3 11 / 35, 3^3 19 / 33; 200 x 200 x 160, 1 sample 23 / 36, 2^3 27 / 37; 3^3 from
+// 2^19 voxels on is the warps' (100 x 100 x 80: 30 us, 200 x 200 x 160: 37).
+template <typename Index>
+__global__ void __launch_bounds__(256) bev2pvcs_ss_thread_kernel(ColumnInfo ci, const float* __restrict__ bev,
+                                                                 float* __restrict__ out, size_t pitch, int nx, int ny,
+                                                                 int nz, SsFrame f, int ss) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y,
+              z = blockIdx.z * blockDim.z + threadIdx.z;
+    if (x >= nx || y >= ny || z >= nz || !f.sampled(ci, x, y, z)) return;
+    const SsVoxel c(ci, f, x, y, z);
+    const float inv = 1.0f / ss;
+    float acc = 0.0f;
+    for (int k = 0; k < ss; k++)
+        for (int j = 0; j < ss; j++)
+#pragma unroll 3
+            for (int i = 0; i < ss; i++)
+                acc += c.sample<Index>(ci, f, bev, rot(ci.R, make_float3(((i + 0.5f) * inv - 0.5f) * f.vx,
+                                                                         ((j + 0.5f) * inv - 0.5f) * f.vy,
+                                                                         ((k + 0.5f) * inv - 0.5f) * f.vz)));
+    if (!(acc < 1e-4f)) out[(size_t)x + pitch * ((size_t)y + (size_t)ny * z)] = acc / (float)(ss * ss * ss);
+}
+
+// More samples: the work is found first.  The volume is cut into tiles of
+// 4 x 4 x 4 voxels, a block's first warp tests `per` tiles (32, fewer for small
+// volumes, whose tiles would else lie with a few blocks), and the block lists a
+// hit tile's voxels.  A warp then takes a voxel, its lanes the ss^3 samples: they
+// fall into a few texel cells, so that a load touches two or three cache lines,
+// where 32 voxels side by side touched up to sixteen and the pass was bound by
+// their lookups.  2 cm, 5^3 samples, a thread a voxel / 32 tiles a block / as now:
+// 200 x 200 x 160 111 / 56 / 56 us, 100 x 100 x 80 103 / 66 / 43, 64 x 64 x 51
+// 58 / 58 / 50.
 constexpr int kSsThreads = 256, kSsTile = 4, kSsTileVox = kSsTile * kSsTile * kSsTile;
 constexpr int kSsRounds = 4;  // samples per lane whose offsets are kept in registers (ss <= 5)
 
 template <typename Index>
 __global__ void __launch_bounds__(kSsThreads, 3) bev2pvcs_ss_kernel(ColumnInfo ci, const float* __restrict__ bev,
                                                                  float* __restrict__ out, size_t pitch, int nx, int ny,
-                                                                 int nz, float vx, float vy, float vz, int ss,
-                                                                 float extent) {
+                                                                 int nz, SsFrame f, int ss, int per) {
     __shared__ int s_vox[kSsTileVox];
     __shared__ int3 s_tile[32];
     __shared__ unsigned s_hits;
     __shared__ int s_n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tx = (nx + kSsTile - 1) / kSsTile, ty = (ny + kSsTile - 1) / kSsTile, tz = (nz + kSsTile - 1) / kSsTile;
-    const long long tiles = (long long)tx * ty * tz, groups = (tiles + 31) / 32;
+    const long long tiles = (long long)tx * ty * tz, groups = (tiles + per - 1) / per;
     const int n_s = ss * ss * ss;
-    // beam-frame offset of sample s from the voxel centre
-    auto offset = [&](int s) {
-        const float inv = 1.0f / ss;
-        const int jk = (int)((s + 0.5f) * inv), k = (int)((jk + 0.5f) * inv);  // s / ss and s / ss^2, s <= 4096
-        const float a = ((s - jk * ss + 0.5f) * inv - 0.5f) * vx, b = ((jk - k * ss + 0.5f) * inv - 0.5f) * vy,
-                    c = ((k + 0.5f) * inv - 0.5f) * vz;
-        return rot(ci.R, make_float3(a, b, c));
-    };
     float3 off[kSsRounds];
 #pragma unroll
-    for (int q = 0; q < kSsRounds; q++) off[q] = offset(lane + 32 * q);
-    const float sx = 1.0f / (ci.bsx * ci.inv_sad), sz = 1.0f / (ci.bsy * ci.inv_sad);
-    // half diagonals of a voxel and a tile, and slack for rounding
-    const float hv = 0.5f * sqrtf(vx * vx + vy * vy + vz * vz), ht = kSsTile * hv;
-    const float slack = 1e-3f + 1e-4f * (ht + fabsf(extent));
+    for (int q = 0; q < kSsRounds; q++) off[q] = f.offset(ci, ss, lane + 32 * q);
     for (long long g = blockIdx.x; g < groups; g += gridDim.x) {
         if (warp == 0) {
             // neighbouring tiles go to different blocks: tile numbers times a prime
             // beyond their count
-            const long long i = g * 32 + lane, tile = i * 2654435761LL % tiles;
+            const long long i = g * per + lane, tile = i * 2654435761LL % tiles;
             const int yz = (int)(tile / tx), x = ((int)(tile - (long long)yz * tx)) * kSsTile, z = yz / ty * kSsTile,
                       y = yz % ty * kSsTile;
-            const float3 v = rot(ci.R, make_float3((x + 0.5f * kSsTile) * vx - ci.src[0], (y + 0.5f * kSsTile) * vy - ci.src[1],
-                                                   (z + 0.5f * kSsTile) * vz - ci.src[2]));
-            const float r = fabsf(extent) + ht + slack, d = ht + hv + ci.ls + slack;
-            const unsigned hits = __ballot_sync(0xffffffffu, i < tiles && !(v.x * v.x + v.z * v.z > r * r) &&
-                                                                 v.y >= ci.lim_min - d && v.y <= ci.lim_min + ci.L * ci.ls + d);
+            const float3 v = f.at(ci, x + 0.5f * kSsTile, y + 0.5f * kSsTile, z + 0.5f * kSsTile);
+            const float ht = kSsTile * f.hv, r = fabsf(f.extent) + ht + f.slack;
+            const unsigned hits = __ballot_sync(0xffffffffu, lane < per && i < tiles && !(v.x * v.x + v.z * v.z > r * r) &&
+                                                                 f.near_map(ci, v, ht + f.slack));
             s_tile[lane] = make_int3(x, y, z);
             if (lane == 0) s_hits = hits;
         }
@@ -189,38 +268,25 @@ __global__ void __launch_bounds__(kSsThreads, 3) bev2pvcs_ss_kernel(ColumnInfo c
         const unsigned hits = s_hits;
         for (unsigned m = hits; m; m &= m - 1) {
             const int3 t0 = s_tile[__ffs(m) - 1];
-            const int x0 = t0.x, y0 = t0.y, z0 = t0.z;
             if (threadIdx.x == 0) s_n = 0;
             __syncthreads();
             if (threadIdx.x < kSsTileVox) {
-                const int q = threadIdx.x, x = x0 + q % kSsTile, y = y0 + q / kSsTile % kSsTile, z = z0 + q / (kSsTile * kSsTile);
-                const float3 c = make_float3((x + 0.5f) * vx, (y + 0.5f) * vy, (z + 0.5f) * vz);
-                const float3 v = rot(ci.R, make_float3(c.x - ci.src[0], c.y - ci.src[1], c.z - ci.src[2]));
-                if (x < nx && y < ny && z < nz && !(v.x * v.x + v.z * v.z > extent * extent))
+                const int q = threadIdx.x, x = t0.x + q % kSsTile, y = t0.y + q / kSsTile % kSsTile,
+                          z = t0.z + q / (kSsTile * kSsTile);
+                if (x < nx && y < ny && z < nz && f.sampled(ci, x, y, z))
                     s_vox[atomicAdd(&s_n, 1)] = q;  // any order: each voxel's sum is its own
             }
             __syncthreads();
             const int n = s_n;
             for (int w = warp; w < n; w += kSsThreads / 32) {
                 const int q = s_vox[w];
-                const int x = x0 + q % kSsTile, y = y0 + q / kSsTile % kSsTile, z = z0 + q / (kSsTile * kSsTile);
-                const double px = (x + 0.5) * vx - ci.src[0], py = (y + 0.5) * vy - ci.src[1], pz = (z + 0.5) * vz - ci.src[2];
-                const float cx = (float)(ci.R[0] * px + ci.R[1] * py + ci.R[2] * pz);
-                const double dy = ci.R[3] * px + ci.R[4] * py + ci.R[5] * pz;
-                const float cy = (float)dy, cw = (float)(dy - ci.lim_min);
-                const float cz = (float)(ci.R[6] * px + ci.R[7] * py + ci.R[8] * pz);
-                auto sample = [&](float3 o) {
-                    const float uy = cy + o.y;
-                    float r = __fdividef(1.0f, uy);
-                    r = fmaf(r, fmaf(-uy, r, 1.0f), r);
-                    return bev_trilinear_near<Index>(bev, ci.fx, ci.fy, ci.L, fmaf((cx + o.x) * r, sx, ci.hx) - 0.5f,
-                                              fmaf((cz + o.z) * r, sz, ci.hy) - 0.5f, fmaf(cw + o.y, ci.inv_ls, -0.5f));
-                };
+                const int x = t0.x + q % kSsTile, y = t0.y + q / kSsTile % kSsTile, z = t0.z + q / (kSsTile * kSsTile);
+                const SsVoxel c(ci, f, x, y, z);
                 float acc = 0.0f;
 #pragma unroll
                 for (int k = 0; k < kSsRounds; k++)
-                    if (lane + 32 * k < n_s) acc += sample(off[k]);
-                for (int k = lane + 32 * kSsRounds; k < n_s; k += 32) acc += sample(offset(k));
+                    if (lane + 32 * k < n_s) acc += c.sample<Index>(ci, f, bev, off[k]);
+                for (int k = lane + 32 * kSsRounds; k < n_s; k += 32) acc += c.sample<Index>(ci, f, bev, f.offset(ci, ss, k));
 #pragma unroll
                 for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                 if (lane == 0 && !(acc < 1e-4f))
@@ -549,19 +615,39 @@ int launch_column_rows(size_t n, const uint32_t* d_nnz, const float* d_max, int6
 }
 
 int launch_bev2pvcs(const ColumnInfo& ci, const fd2_volume_t& v, const float* d_bev, float* d_out, size_t pitch,
-                    int ss, float extent, cudaStream_t stream) {
+                    int ss, float extent, int sm_count, cudaStream_t stream) {
     if (ss <= 0) {
-        dim3 block(32, 8), grid((v.dim[0] + 31) / 32, (v.dim[1] + 7) / 8, std::min((v.dim[2] + kDenseZ - 1) / kDenseZ, 65535u));
+        dim3 block(32, 8), grid((v.dim[0] + 31) / 32, (v.dim[1] + 7) / 8);
+        const uint64_t columns = (uint64_t)grid.x * grid.y, want = (uint64_t)sm_count * 8;
+        const unsigned planes = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(kDenseZ, columns * v.dim[2] / want));
+        grid.z = std::min((v.dim[2] + planes - 1) / planes, 65535u);
         bev2pvcs_kernel<<<grid, block, 0, stream>>>(ci, d_bev, d_out, pitch, v.dim[0], v.dim[1], v.dim[2],
-                                                    v.voxel_size[0], v.voxel_size[1], v.voxel_size[2]);
+                                                    v.voxel_size[0], v.voxel_size[1], v.voxel_size[2], (int)planes);
     } else {
-        const uint64_t tiles = (uint64_t)((v.dim[0] + kSsTile - 1) / kSsTile) * ((v.dim[1] + kSsTile - 1) / kSsTile) *
-                               ((v.dim[2] + kSsTile - 1) / kSsTile);
-        const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((tiles + 31) / 32, 1 << 20));
         const bool small = (uint64_t)ci.fx * ci.fy * ci.L < (1ull << 30);
-        (small ? bev2pvcs_ss_kernel<int> : bev2pvcs_ss_kernel<size_t>)<<<blocks, kSsThreads, 0, stream>>>(
-            ci, d_bev, d_out, pitch, v.dim[0], v.dim[1], v.dim[2], v.voxel_size[0], v.voxel_size[1], v.voxel_size[2], ss,
-            extent);
+        const uint64_t voxels = (uint64_t)v.dim[0] * v.dim[1] * v.dim[2];
+        const SsFrame f(ci, v, extent);
+        if (ss <= 2 || (ss == 3 && voxels < (1u << 19))) {
+            dim3 block(8, 8, 4), grid((v.dim[0] + 7) / 8, (v.dim[1] + 7) / 8, (v.dim[2] + 3) / 4);
+            (small ? bev2pvcs_ss_thread_kernel<int> : bev2pvcs_ss_thread_kernel<size_t>)<<<grid, block, 0, stream>>>(
+                ci, d_bev, d_out, pitch, v.dim[0], v.dim[1], v.dim[2], f, ss);
+        } else {
+            const uint64_t tiles = (uint64_t)((v.dim[0] + kSsTile - 1) / kSsTile) * ((v.dim[1] + kSsTile - 1) / kSsTile) *
+                                   ((v.dim[2] + kSsTile - 1) / kSsTile);
+            // a block takes its hit tiles in turn: where the launch is little more than
+            // two waves, as many tiles as hold one hit, by the part of the volume that
+            // the sampled cylinder and its rim fill
+            const double rim = kSsTile * f.hv, ext = std::fabs(extent);
+            const double side_x = 2 * (std::min(ext, (double)f.mx / ci.inv_sad) + rim),
+                         side_z = 2 * (std::min(ext, (double)f.mz / ci.inv_sad) + rim);
+            const double part = 0.8 * side_x * side_z * ((double)ci.L * ci.ls + 2 * rim) /
+                                ((double)voxels * f.vx * f.vy * f.vz);
+            int per = 32;
+            while (per > 2 && tiles <= (uint64_t)per * 7 * sm_count && per * part > 1.0) per /= 2;
+            const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((tiles + per - 1) / per, 1 << 20));
+            (small ? bev2pvcs_ss_kernel<int> : bev2pvcs_ss_kernel<size_t>)<<<blocks, kSsThreads, 0, stream>>>(
+                ci, d_bev, d_out, pitch, v.dim[0], v.dim[1], v.dim[2], f, ss, per);
+        }
     }
     FD2_CHECK_CUDA(cudaGetLastError());
     return FD2_OK;

@@ -24,7 +24,7 @@ struct ColumnInfo {
 void make_column_info(const fd2_beam_t& b, const fd2_volume_t* vol, ColumnInfo& ci);
 
 int launch_bev2pvcs(const ColumnInfo& ci, const fd2_volume_t& v, const float* d_bev, float* d_out, size_t pitch,
-                    int ss, float extent, cudaStream_t stream);
+                    int ss, float extent, int sm_count, cudaStream_t stream);
 int launch_column_count(const ColumnInfo* d_infos, size_t n, uint32_t* d_counts, const fd2_volume_t& v, float extent,
                         cudaStream_t stream);
 int launch_column_values(const ColumnInfo* d_infos, size_t n, const float* const* d_dose, const uint64_t* d_cap_off,

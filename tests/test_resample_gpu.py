@@ -109,7 +109,7 @@ def test_dense(ctx, grid, pad):
 
 
 @pytest.mark.parametrize("extent", [0.6, 2.0, 50.0])
-@pytest.mark.parametrize("ss", [1, 2, 5, 6, 16])
+@pytest.mark.parametrize("ss", [1, 2, 3, 4, 5, 6, 16])
 @pytest.mark.parametrize("grid", list(GRIDS))
 def test_supersampled(ctx, grid, ss, extent):
     vol, b, bev = _case(grid)
