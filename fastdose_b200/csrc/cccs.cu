@@ -552,6 +552,15 @@ __global__ void cccs_split_reduce(const fd2_beam_t* __restrict__ beams, float* c
 // warp, and it runs while the other warps reduce the previous slice.  Two
 // barriers per slice.
 //
+// kOwnPath is for launches of few blocks, where the chain of one block is the
+// time: the other warps wait for those records, and a step's loads and votes are
+// not hidden by other blocks.  There every warp computes its azimuth's path as it
+// goes, beside the arithmetic of the rays, and the registers of a whole SM are
+// taken.  The same operations on the same floats: the dose is the same bit for bit.
+// One beam's zenith bins, rays in place / records / own path: 16 x 16, 6 azimuths,
+// 0.125 cm pixels 1.81 / 2.11 / 1.65 ms; 12 x 12 2.12 / 1.82 / 1.42; 8 x 8 1.38 /
+// 1.37 / 1.11.
+//
 // The lateral offset and the edge crossing of a column or row are the
 // reference's own roundings, evaluated once per column and row (only the rays on
 // the first and last column and row can cross an edge).  Where rounding
@@ -645,21 +654,21 @@ enum : int {
 // Shared memory of a march block.  A map's cell (column v, row r) is at
 // v * S + r: a lane's rows are consecutive, and with S = F + 4 (F a multiple of
 // 8) eight neighbouring lanes' 16-byte accesses hit distinct banks.
-template <int F>
+template <int F, int kW>
 struct MarchShared {
     static constexpr int S = F + 4;
-    float4 rec[kMarchWarps][kMarchSteps];  // next point x, y; divergence factor there; (depth of the step)^2
-    int code[kMarchWarps][kMarchSteps];
+    float4 rec[kW][kMarchSteps];  // next point x, y; divergence factor there; (depth of the step)^2
+    int code[kW][kMarchSteps];
     alignas(16) float T[2][F * S];         // this slice and the one staged behind it
     alignas(16) float R[2][F * S];
-    alignas(16) float dose[kMarchWarps][F * S];  // each azimuth's sums of the slice
+    alignas(16) float dose[kW][F * S];  // each azimuth's sums of the slice
     alignas(16) float path[F * S];               // the last azimuth's path sums
-    alignas(16) float xa[kMarchWarps][F * S], xb[kMarchWarps][F * S];  // ray states in march_exact_step
-    alignas(16) float row[kMarchWarps][2][F];    // the step's lateral offset of each row
-    float3 c[kMarchWarps];                 // chain state: point, voxel shift,
-    int2 k[kMarchWarps];
-    ConeDir dir[kMarchWarps];              // direction,
-    int count[kMarchWarps];                // records of this round,
+    alignas(16) float xa[kW][F * S], xb[kW][F * S];  // ray states in march_exact_step
+    alignas(16) float row[kW][2][F];    // the step's lateral offset of each row
+    float3 c[kW];                 // chain state: point, voxel shift,
+    int2 k[kW];
+    ConeDir dir[kW];              // direction,
+    int count[kW];                // records of this round,
     int next, more, abort;                 // next slice; some azimuth has more rounds; step cap hit
 };
 
@@ -687,10 +696,28 @@ __device__ __forceinline__ int path_axis(float c, float n, bool& exact) {
     return biased_int(fl);
 }
 
+// The record of the step c..n of a base ray at voxel shift k0, and the shift kn
+// along it; whether it asks for march_exact_step.
+template <int F>
+__device__ __forceinline__ bool path_record(const MarchRay& g, float3 c, float3 n, int2 k0, int2& kn, float4& rec) {
+    bool exact = false;
+    kn = make_int2(path_axis<F>(c.x, n.x, exact), 0);
+    kn.y = path_axis<F>(c.y, n.y, exact);
+    const float dz = (n.z - c.z) * g.ls;
+    rec = make_float4(n.x, n.y, (n.z * g.ls + g.lim_min) * g.inv_sad, __fmul_rn(dz, dz));
+    return exact || abs(kn.x - k0.x) > 1 || abs(kn.y - k0.y) > 1;
+}
+
+// The first azimuth's plane after slice s; it always lies ahead.
+__device__ __forceinline__ int plane_after(float z, int s, int L) {
+    const int nxt = (int)roundf(z);
+    return nxt > s ? nxt : L;
+}
+
 // One round of every azimuth's path (lane = azimuth) from the chain state in
 // shared memory.  `open`: the lane's slice is not finished.
-template <int F>
-__device__ __forceinline__ void march_paths(MarchShared<F>& sm, const MarchRay& g, int n_phi, int s, int L, bool open) {
+template <int F, int kW>
+__device__ __forceinline__ void march_paths(MarchShared<F, kW>& sm, const MarchRay& g, int n_phi, int s, int L, bool open) {
     const int w = threadIdx.x & 31;
     int n = 0;
     if (w < n_phi && open) {
@@ -700,25 +727,19 @@ __device__ __forceinline__ void march_paths(MarchShared<F>& sm, const MarchRay& 
         bool flag = false;
         while (!flag && n < kMarchSteps) {
             float3 np;
+            int2 kn;
             flag = next_point_biased(c, k, np);
-            bool exact = false;
-            const int kx = path_axis<F>(c.x, np.x, exact), ky = path_axis<F>(c.y, np.y, exact);
-            exact = exact || abs(kx - k0.x) > 1 || abs(ky - k0.y) > 1;
-            const float fe = (np.z * g.ls + g.lim_min) * g.inv_sad;
-            const float dz = (np.z - c.z) * g.ls;
-            sm.rec[w][n] = make_float4(np.x, np.y, fe, dz * dz);
-            sm.code[w][n++] = (flag ? kRecEnd : 0) | (exact ? kRecExact : 0) | (kx != k0.x ? kRecMoveX : 0) |
-                              (ky != k0.y ? kRecMoveY : 0);
+            const bool exact = path_record<F>(g, c, np, k0, kn, sm.rec[w][n]);
+            sm.code[w][n++] = (flag ? kRecEnd : 0) | (exact ? kRecExact : 0) | (kn.x != k0.x ? kRecMoveX : 0) |
+                              (kn.y != k0.y ? kRecMoveY : 0);
             c = np;
-            k0 = make_int2(kx, ky);
+            k0 = kn;
         }
         sm.k[w] = k0;
         sm.c[w] = c;
         open = !flag;
         if (w == 0 && flag) {
-            // the first azimuth's plane after this slice; it always lies ahead
-            const int nxt = (int)roundf(c.z);
-            sm.next = nxt > s ? nxt : L;
+            sm.next = plane_after(c.z, s, L);
         }
     }
     if (w < n_phi) sm.count[w] = n;
@@ -733,10 +754,10 @@ __device__ __forceinline__ void march_paths(MarchShared<F>& sm, const MarchRay& 
 // which is returned.  Rays of one step can only meet in a voxel next to their
 // own, so four passes, one per parity of column and row, keep the additions
 // apart and their order fixed.
-template <int F, int G, int R>
-__device__ __noinline__ int2 march_exact_step(MarchShared<F>& sm, int buf, const MarchRay& g, float2 b, float2 n,
+template <int F, int G, int R, int kW>
+__device__ __noinline__ int2 march_exact_step(MarchShared<F, kW>& sm, int buf, const MarchRay& g, float2 b, float2 n,
                                               float fs, float fe, float dz2, int ox, int oy, bool last) {
-    constexpr int S = MarchShared<F>::S;
+    constexpr int S = MarchShared<F, kW>::S;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, v = lane % F, grp = lane / F;
     const bool on = grp < G;
     const float ff = (float)F, hh = 0.5f * F;
@@ -811,9 +832,11 @@ __device__ __forceinline__ void store_cells(float* p, const F2 (&o)[R / 2]) {
     }
 }
 
-// 80 registers: four blocks of 6 azimuths an SM.
-template <int F, int G, int R>
-__global__ void __launch_bounds__(32 * kMarchWarps, 3)
+// kW: azimuths the shared memory is for.  80 registers: four blocks of 6 azimuths
+// an SM, six of up to 4 (with the shared memory of 8 azimuths only five fit: 1800
+// beams of 16 x 16, 4 azimuths 14.7 ms, 12.0 so, 12.1 with the rays in place).
+template <int F, int G, int R, int kW, bool kOwnPath>
+__global__ void __launch_bounds__(32 * kW, kOwnPath ? 1 : (kW <= 4 ? 6 : 3))
     cccs_march_kernel(const fd2_beam_t* __restrict__ beams, const float* const* __restrict__ terma,
                       const float* const* __restrict__ dens, float* const* __restrict__ dose,
                       const float4* __restrict__ dirs,  // [beam][n_tf][n_phi]
@@ -821,8 +844,8 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3)
                       const int* __restrict__ order) {
     static_assert(F == G * R && G > 1 && R % 2 == 0 && F * G <= 32, "a lane holds R rows of a column in pairs");
     constexpr unsigned kAll = 0xffffffffu;
-    constexpr int P = F * F, S = MarchShared<F>::S;
-    __shared__ MarchShared<F> sm;
+    constexpr int P = F * F, S = MarchShared<F, kW>::S;
+    __shared__ MarchShared<F, kW> sm;
     const int n_tf = cp.n_theta_fwd, n_phi = cp.n_phi;
     // split: one block per (zenith bin, beamlet), the widest bin (most steps per
     // slice) first; else one block per beamlet in `order` (longest first)
@@ -861,7 +884,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3)
     };
     // the azimuths of slice s in order, normalised by the last one's path sum;
     // done by the warps that compute no path (the first does)
-    const int rt0 = n_phi > 1 ? 32 : 0;
+    const int rt0 = n_phi > 1 && !kOwnPath ? 32 : 0;
     auto reduce = [&](int t, int s) {
         for (int i = threadIdx.x - rt0; i < P; i += blockDim.x - rt0) {
             const int q = i % F * S + i / F;
@@ -878,7 +901,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3)
         }
     };
 
-    int buf = 0;
+    int buf = 0, staged = 0;
     stage(0, 0);
     int prev_s = -1, prev_t = 0;  // the slice whose sums wait to be reduced
     for (int t = t0; t < t1; t++) {
@@ -897,7 +920,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3)
         // a move in x takes a state from lane ux, one in y the row carried over
         // from another group's lane uy; the ray on this lane's column (group 0) or
         // row `v` (group 1) changes by -step
-        const bool xp = d4.x >= 0.0f, yp = d4.y >= 0.0f;
+        const bool xp = d4.x >= 0.0f, yp = d4.y >= 0.0f, yp_all = __any_sync(kAll, yp);
         const int ux = (xp ? (v == 0 ? F - 1 : v - 1) : (v == F - 1 ? 0 : v + 1)) + grp * F;
         const int uy = (yp ? (grp == 0 ? G - 1 : grp - 1) : (grp + 1 >= G ? 0 : grp + 1)) * F + v;
         const float step = (yl ? yp : xp) ? 1.0f : -1.0f;
@@ -914,164 +937,252 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 3)
         // for this zenith bin; the other azimuths keep marching from wherever
         // they stopped.
         int s = 0, par = 0;
+        // kOwnPath: the azimuth's own path state
+        const ConeDir cd = make_cone_dir(make_float3(d4.x, d4.y, d4.z));
+        float3 c = make_float3(0.5f, 0.5f, 0.0f);
+        int2 k0 = make_int2(0, 0);
         while (s < L) {
             F2 Tv[R / 2], Rv[R / 2], Dv[R / 2], Pv[R / 2];
             int s_next = L;
-            for (int round = 0;; round++) {
-                if (warp == 0) {
-                    bool open = true;
-                    if (round > 0) {  // azimuths still inside the slice: their last record does not end it
-                        open = lane < n_phi && sm.count[lane] > 0 && !(sm.code[lane][sm.count[lane] - 1] & kRecEnd);
-                        if ((long long)round * kMarchSteps >= kStepCap) {
-                            open = false;
-                            if (lane == 0) {
-                                atomicExch(&status->code, (int)FD2_ERR_WATCHDOG);
-                                sm.abort = 1;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                    march_paths<F>(sm, g, n_phi, s, L, open);
+            auto load_slice = [&]() {
+                load_cells<R>(&sm.T[buf][cell], Tv);
+                load_cells<R>(&sm.R[buf][cell], Rv);
+#pragma unroll
+                for (int q = 0; q < R / 2; q++) {
+                    if (!on) Tv[q] = Rv[q] = pk(0.0f, 0.0f);
+                    Dv[q] = Pv[q] = pk(0.0f, 0.0f);
                 }
-                if (round == 0) {
-                    if (prev_s >= 0 && (warp > 0 || n_phi == 1)) reduce(prev_t, prev_s);
-                    cp_async_wait_all();  // this thread's pixels of the slice have landed
+            };
+            auto store_sums = [&]() {
+                if (on) {
+                    store_cells<R>(&sm.dose[warp][cell], Dv);
+                    if (last) store_cells<R>(&sm.path[cell], Pv);
                 }
-                __syncthreads();
-                if (sm.abort) return;  // the same for all: written before the barrier only
-                if (round == 0) {
-                    load_cells<R>(&sm.T[buf][cell], Tv);
-                    load_cells<R>(&sm.R[buf][cell], Rv);
+            };
+            // the states to the shift of the coming step
+            auto move = [&](bool move_x, bool move_y) {
+                if (move_x) {
 #pragma unroll
                     for (int q = 0; q < R / 2; q++) {
-                        if (!on) Tv[q] = Rv[q] = pk(0.0f, 0.0f);
-                        Dv[q] = Pv[q] = pk(0.0f, 0.0f);
+                        const float2 a = up(XA[q]), b = up(XB[q]);
+                        XA[q] = pk(__shfl_sync(kAll, a.x, ux), __shfl_sync(kAll, a.y, ux));
+                        XB[q] = pk(__shfl_sync(kAll, b.x, ux), __shfl_sync(kAll, b.y, ux));
                     }
                 }
-                const bool more = sm.more;
-                if (!more) {
-                    s_next = sm.next;
-                    // the next slice to come (or slice 0 of the next zenith pass)
-                    const int st = s_next < L ? s_next : (t + 1 < t1 ? 0 : -1);
-                    if (st >= 0) stage(st, buf ^ 1);
-                }
-                const int n = sm.count[warp];
-                for (int i = 0; i < n; i++) {
-                    for (; i < n; i++) {
-                        const int code = sm.code[warp][i];
-                        if (__any_sync(kAll, code & kRecExact)) break;
-                        const float4 rec = sm.rec[warp][i];
-                        const float cn = yl ? rec.y : rec.x;
-                        if (__any_sync(kAll, code & kRecMoveX)) {
+                if (move_y) {
+                    if (R == 2 || kOwnPath ? yp_all : __any_sync(kAll, yp)) {
+                        const float ea = __shfl_sync(kAll, up(XA[R / 2 - 1]).y, uy);
+                        const float eb = __shfl_sync(kAll, up(XB[R / 2 - 1]).y, uy);
 #pragma unroll
-                            for (int q = 0; q < R / 2; q++) {
-                                const float2 a = up(XA[q]), b = up(XB[q]);
-                                XA[q] = pk(__shfl_sync(kAll, a.x, ux), __shfl_sync(kAll, a.y, ux));
-                                XB[q] = pk(__shfl_sync(kAll, b.x, ux), __shfl_sync(kAll, b.y, ux));
-                            }
-                            if (!yl) lf -= step;
+                        for (int q = R / 2 - 1; q >= 0; q--) {
+                            XA[q] = pk(q ? up(XA[q ? q - 1 : 0]).y : ea, up(XA[q]).x);
+                            XB[q] = pk(q ? up(XB[q ? q - 1 : 0]).y : eb, up(XB[q]).x);
                         }
-                        if (__any_sync(kAll, code & kRecMoveY)) {
-                            if (__any_sync(kAll, yp)) {
-                                const float ea = __shfl_sync(kAll, up(XA[R / 2 - 1]).y, uy);
-                                const float eb = __shfl_sync(kAll, up(XB[R / 2 - 1]).y, uy);
-#pragma unroll
-                                for (int q = R / 2 - 1; q >= 0; q--) {
-                                    XA[q] = pk(q ? up(XA[q ? q - 1 : 0]).y : ea, up(XA[q]).x);
-                                    XB[q] = pk(q ? up(XB[q ? q - 1 : 0]).y : eb, up(XB[q]).x);
-                                }
-                            } else {
-                                const float ea = __shfl_sync(kAll, up(XA[0]).x, uy);
-                                const float eb = __shfl_sync(kAll, up(XB[0]).x, uy);
-#pragma unroll
-                                for (int q = 0; q < R / 2; q++) {
-                                    const bool e = q == R / 2 - 1;
-                                    XA[q] = pk(up(XA[q]).y, e ? ea : up(XA[e ? q : q + 1]).x);
-                                    XB[q] = pk(up(XB[q]).y, e ? eb : up(XB[e ? q : q + 1]).x);
-                                }
-                            }
-                            if (yl) lf -= step;
-                        }
-                        lf = lf < 0.0f ? lf + F : (lf >= F ? lf - F : lf);
-                        // lateral offset of the ray on this lane's column or row, its edge
-                        // crossing as the sign (the offset enters the length squared)
-                        const float b = __fadd_rn(cb, lf), e = __fadd_rn(cn, lf);
-                        float d = fabsf((e - 0.5f * F) * bs * rec.z - (b - 0.5f * F) * bs * fs);
-                        d = floor_biased(__fdividef(b, (float)F)) != floor_biased(__fdividef(e, (float)F)) ? -d : d;
-                        if (yl) sm.row[warp][par][v] = d;
-                        const float dx = __shfl_sync(kAll, d, v);
-                        const float dxz2 = dx * dx + rec.w;
-                        cb = cn;
-                        fs = rec.z;
-                        __syncwarp();
-                        F2 dy[R / 2];
-                        load_cells<R>(&sm.row[warp][par][on ? grp * R : 0], dy);
-                        par ^= 1;
-                        const F2 dxz = pk(dxz2, dxz2);
+                    } else {
+                        const float ea = __shfl_sync(kAll, up(XA[0]).x, uy);
+                        const float eb = __shfl_sync(kAll, up(XB[0]).x, uy);
 #pragma unroll
                         for (int q = 0; q < R / 2; q++) {
-                            const F2 l2 = fma2(dy[q], dy[q], dxz);
-                            const float2 l2s = up(l2);
-                            const F2 p = mul2(mul2(l2, pk(rsqrt_sfu(l2s.x), rsqrt_sfu(l2s.y))), Rv[q]);
-                            const float2 xa = up(mul2(p, ka2)), xb = up(mul2(p, kb2));
-                            Dv[q] = fma2(fma2(Bb2, XB[q], mul2(Aa2, XA[q])), p, Dv[q]);
-                            if (last) Pv[q] = add2(Pv[q], p);
-                            XA[q] = fma2(pk(exp2_sfu(xa.x), exp2_sfu(xa.y)), sub2(XA[q], Tv[q]), Tv[q]);
-                            XB[q] = fma2(pk(exp2_sfu(xb.x), exp2_sfu(xb.y)), sub2(XB[q], Tv[q]), Tv[q]);
+                            const bool e = q == R / 2 - 1;
+                            XA[q] = pk(up(XA[q]).y, e ? ea : up(XA[e ? q : q + 1]).x);
+                            XB[q] = pk(up(XB[q]).y, e ? eb : up(XB[e ? q : q + 1]).x);
                         }
-                        // rays that crossed an edge start anew
-                        const bool wx = __float_as_int(dx) < 0;
-                        if (__any_sync(kAll, wx)) {
+                    }
+                }
+            };
+            // lateral offset over the step of the ray on this lane's column or row, its
+            // edge crossing as the sign (the offset enters the length squared); rows'
+            // offsets go to the warp's table, columns' come by shuffle
+            auto offset = [&](float cn, float fe) {
+                const float b = __fadd_rn(cb, lf), e = __fadd_rn(cn, lf);
+                float d = fabsf((e - 0.5f * F) * bs * fe - (b - 0.5f * F) * bs * fs);
+                d = floor_biased(__fdividef(b, (float)F)) != floor_biased(__fdividef(e, (float)F)) ? -d : d;
+                if (yl) sm.row[warp][par][v] = d;
+                return __shfl_sync(kAll, d, v);
+            };
+            // the rays of a step, at the offsets of the column and of the table
+            auto rays = [&](float dx, float dz2) {
+                const float dxz2 = dx * dx + dz2;
+                F2 dy[R / 2];
+                load_cells<R>(&sm.row[warp][par][on ? grp * R : 0], dy);
+                const F2 dxz = pk(dxz2, dxz2);
 #pragma unroll
-                            for (int q = 0; q < R / 2; q++) {
-                                XA[q].v = wx ? 0ull : XA[q].v;
-                                XB[q].v = wx ? 0ull : XB[q].v;
+                for (int q = 0; q < R / 2; q++) {
+                    const F2 l2 = fma2(dy[q], dy[q], dxz);
+                    const float2 l2s = up(l2);
+                    const F2 p = mul2(mul2(l2, pk(rsqrt_sfu(l2s.x), rsqrt_sfu(l2s.y))), Rv[q]);
+                    const float2 xa = up(mul2(p, ka2)), xb = up(mul2(p, kb2));
+                    Dv[q] = fma2(fma2(Bb2, XB[q], mul2(Aa2, XA[q])), p, Dv[q]);
+                    if (last) Pv[q] = add2(Pv[q], p);
+                    XA[q] = fma2(pk(exp2_sfu(xa.x), exp2_sfu(xa.y)), sub2(XA[q], Tv[q]), Tv[q]);
+                    XB[q] = fma2(pk(exp2_sfu(xb.x), exp2_sfu(xb.y)), sub2(XB[q], Tv[q]), Tv[q]);
+                }
+                // rays that crossed an edge start anew
+                const bool wx = __float_as_int(dx) < 0;
+                if (__any_sync(kAll, wx)) {
+#pragma unroll
+                    for (int q = 0; q < R / 2; q++) {
+                        XA[q].v = wx ? 0ull : XA[q].v;
+                        XB[q].v = wx ? 0ull : XB[q].v;
+                    }
+                }
+                const bool w0 = __float_as_int(up(dy[0]).x) < 0, w1 = __float_as_int(up(dy[R / 2 - 1]).y) < 0;
+                XA[0] = pk(w0 ? 0.0f : up(XA[0]).x, up(XA[0]).y);
+                XB[0] = pk(w0 ? 0.0f : up(XB[0]).x, up(XB[0]).y);
+                XA[R / 2 - 1] = pk(up(XA[R / 2 - 1]).x, w1 ? 0.0f : up(XA[R / 2 - 1]).y);
+                XB[R / 2 - 1] = pk(up(XB[R / 2 - 1]).x, w1 ? 0.0f : up(XB[R / 2 - 1]).y);
+            };
+            // one step, whose shift changed by a column and a row
+            auto ray_step = [&](const float4& rec, bool move_x, bool move_y) {
+                move(move_x, move_y);
+                if (yl ? move_y : move_x) lf -= step;
+                lf = lf < 0.0f ? lf + F : (lf >= F ? lf - F : lf);
+                const float cn = yl ? rec.y : rec.x;
+                const float dx = offset(cn, rec.z);
+                cb = cn;
+                fs = rec.z;
+                __syncwarp();
+                rays(dx, rec.w);
+                par ^= 1;
+            };
+            // a step from b to n in which some ray's voxel may not be the shifted one;
+            // the states come at shift o and leave at the one returned
+            auto exact_step = [&](float2 b, float2 n, float f0, float f1, float dz2, int ox, int oy) {
+                if (on) {
+                    store_cells<R>(&sm.dose[warp][cell], Dv);
+                    store_cells<R>(&sm.xa[warp][cell], XA);
+                    store_cells<R>(&sm.xb[warp][cell], XB);
+                    if (last) store_cells<R>(&sm.path[cell], Pv);
+                }
+                const int2 k = march_exact_step<F, G, R, kW>(sm, buf, g, b, n, f0, f1, dz2, ox, oy, last);
+                if (on) {
+                    load_cells<R>(&sm.dose[warp][cell], Dv);
+                    load_cells<R>(&sm.xa[warp][cell], XA);
+                    load_cells<R>(&sm.xb[warp][cell], XB);
+                    if (last) load_cells<R>(&sm.path[cell], Pv);
+                }
+                __syncwarp();
+                return k;
+            };
+            if constexpr (kOwnPath) {
+                if (s != staged) {  // the slice after the last one was skipped
+                    cp_async_wait_all();
+                    stage(s, buf);
+                }
+                cp_async_wait_all();
+                __syncthreads();  // the slice stands, the last one's sums are used
+                load_slice();
+                staged = s + 1 < L ? s + 1 : (t + 1 < t1 ? 0 : -1);
+                if (staged >= 0) stage(staged, buf ^ 1);
+                bool flag = false;
+                for (int guard = 0; !flag; guard++) {
+                    if (guard >= kStepCap) {
+                        if (lane == 0) {
+                            atomicExch(&status->code, (int)FD2_ERR_WATCHDOG);
+                            sm.abort = 1;
+                        }
+                        break;
+                    }
+                    float3 np;
+                    int2 kn;
+                    float4 rec;
+                    flag = next_point_biased(c, cd, np);
+                    if (path_record<F>(g, c, np, k0, kn, rec)) {
+                        const int2 k = exact_step(make_float2(c.x, c.y), make_float2(np.x, np.y), fs, rec.z, rec.w,
+                                                  pos_mod(k0.x, F), pos_mod(k0.y, F));
+                        lf = (float)pos_mod(v - (yl ? k.y : k.x), F);
+                        cb = yl ? rec.y : rec.x;
+                        fs = rec.z;
+                    } else {
+                        ray_step(rec, kn.x != k0.x, kn.y != k0.y);
+                    }
+                    c = np;
+                    k0 = kn;
+                }
+                store_sums();
+                if (threadIdx.x == 0) sm.next = plane_after(c.z, s, L);
+                __syncthreads();  // the slice's sums stand
+                if (sm.abort) {
+                    cp_async_wait_all();
+                    return;
+                }
+                s_next = sm.next;
+                reduce(t, s);
+            } else {
+                for (int round = 0;; round++) {
+                    if (warp == 0) {
+                        bool open = true;
+                        if (round > 0) {  // azimuths still inside the slice: their last record does not end it
+                            open = lane < n_phi && sm.count[lane] > 0 && !(sm.code[lane][sm.count[lane] - 1] & kRecEnd);
+                            if ((long long)round * kMarchSteps >= kStepCap) {
+                                open = false;
+                                if (lane == 0) {
+                                    atomicExch(&status->code, (int)FD2_ERR_WATCHDOG);
+                                    sm.abort = 1;
+                                }
                             }
                         }
-                        const bool w0 = __float_as_int(up(dy[0]).x) < 0, w1 = __float_as_int(up(dy[R / 2 - 1]).y) < 0;
-                        XA[0] = pk(w0 ? 0.0f : up(XA[0]).x, up(XA[0]).y);
-                        XB[0] = pk(w0 ? 0.0f : up(XB[0]).x, up(XB[0]).y);
-                        XA[R / 2 - 1] = pk(up(XA[R / 2 - 1]).x, w1 ? 0.0f : up(XA[R / 2 - 1]).y);
-                        XB[R / 2 - 1] = pk(up(XB[R / 2 - 1]).x, w1 ? 0.0f : up(XB[R / 2 - 1]).y);
+                        __syncwarp();
+                        march_paths<F, kW>(sm, g, n_phi, s, L, open);
                     }
-                    if (i >= n) break;
-                    const float4 rec = sm.rec[warp][i];
-                    if (on) {
-                        store_cells<R>(&sm.dose[warp][cell], Dv);
-                        store_cells<R>(&sm.xa[warp][cell], XA);
-                        store_cells<R>(&sm.xb[warp][cell], XB);
-                        if (last) store_cells<R>(&sm.path[cell], Pv);
+                    if (round == 0) {
+                        if (prev_s >= 0 && (warp > 0 || n_phi == 1)) reduce(prev_t, prev_s);
+                        cp_async_wait_all();  // this thread's pixels of the slice have landed
                     }
-                    const int o = pos_mod(v - (int)lf, F);  // the shift: of x in group 0, of y in group 1
-                    const int2 k = march_exact_step<F, G, R>(
-                        sm, buf, g, make_float2(__shfl_sync(kAll, cb, 0), __shfl_sync(kAll, cb, F)),
-                        make_float2(rec.x, rec.y), fs, rec.z, rec.w, __shfl_sync(kAll, o, 0), __shfl_sync(kAll, o, F), last);
-                    if (on) {
-                        load_cells<R>(&sm.dose[warp][cell], Dv);
-                        load_cells<R>(&sm.xa[warp][cell], XA);
-                        load_cells<R>(&sm.xb[warp][cell], XB);
-                        if (last) load_cells<R>(&sm.path[cell], Pv);
+                    __syncthreads();
+                    if (sm.abort) return;  // the same for all: written before the barrier only
+                    if (round == 0) load_slice();
+                    const bool more = sm.more;
+                    if (!more) {
+                        s_next = sm.next;
+                        // the next slice to come (or slice 0 of the next zenith pass)
+                        const int st = s_next < L ? s_next : (t + 1 < t1 ? 0 : -1);
+                        if (st >= 0) stage(st, buf ^ 1);
                     }
-                    __syncwarp();
-                    lf = (float)pos_mod(v - (yl ? k.y : k.x), F);
-                    cb = yl ? rec.y : rec.x;
-                    fs = rec.z;
+                    const int n = sm.count[warp];
+                    for (int i = 0; i < n; i++) {
+                        for (; i < n; i++) {
+                            const int code = sm.code[warp][i];
+                            if (__any_sync(kAll, code & kRecExact)) break;
+                            const float4 rec = sm.rec[warp][i];
+                            const bool mx = __any_sync(kAll, code & kRecMoveX), my = __any_sync(kAll, code & kRecMoveY);
+                            move(mx, my);
+                            if (yl ? my : mx) lf -= step;
+                            lf = lf < 0.0f ? lf + F : (lf >= F ? lf - F : lf);
+                            const float cn = yl ? rec.y : rec.x;
+                            const float dx = offset(cn, rec.z);
+                            cb = cn;
+                            fs = rec.z;
+                            __syncwarp();
+                            rays(dx, rec.w);
+                            par ^= 1;
+                        }
+                        if (i >= n) break;
+                        const float4 rec = sm.rec[warp][i];
+                        const int o = pos_mod(v - (int)lf, F);  // the shift: of x in group 0, of y in group 1
+                        const int2 k = exact_step(make_float2(__shfl_sync(kAll, cb, 0), __shfl_sync(kAll, cb, F)),
+                                                  make_float2(rec.x, rec.y), fs, rec.z, rec.w, __shfl_sync(kAll, o, 0),
+                                                  __shfl_sync(kAll, o, F));
+                        lf = (float)pos_mod(v - (yl ? k.y : k.x), F);
+                        cb = yl ? rec.y : rec.x;
+                        fs = rec.z;
+                    }
+                    if (!more) break;
+                    __syncthreads();  // the round's records are used
                 }
-                if (!more) break;
-                __syncthreads();  // the round's records are used
+                store_sums();
+                __syncthreads();  // the slice's sums stand, its records and data are used
+                prev_s = s;
+                prev_t = t;
             }
-            if (on) {
-                store_cells<R>(&sm.dose[warp][cell], Dv);
-                if (last) store_cells<R>(&sm.path[cell], Pv);
-            }
-            __syncthreads();  // the slice's sums stand, its records and data are used
-            prev_s = s;
-            prev_t = t;
             buf ^= 1;
             s = s_next;
         }
     }
-    if (prev_s >= 0 && (warp > 0 || n_phi == 1)) reduce(prev_t, prev_s);
+    if constexpr (kOwnPath)
+        cp_async_wait_all();  // a slice staged and not taken
+    else if (prev_s >= 0 && (warp > 0 || n_phi == 1))
+        reduce(prev_t, prev_s);
 }
 
 template <int RPL, bool kCols, bool kTab = false>
@@ -1091,9 +1202,18 @@ template <int F, int G, int R>
 int launch_voxel_march(unsigned blocks, int n_phi, cudaStream_t st, const fd2_beam_t* d_beams,
                        const float* const* T, const float* const* Rho, float* const* D, const float4* dirs,
                        const ConeParams& cp, int split, float* planes, size_t plane_stride, DeviceStatus* status,
-                       const int* order) {
-    cccs_march_kernel<F, G, R><<<blocks, 32 * n_phi, 0, st>>>(d_beams, T, Rho, D, dirs, cp, split, planes,
-                                                              plane_stride, status, order);
+                       const int* order, int sm_count) {
+    // kOwnPath up to some 20 warps an SM: later its blocks, one of more than 4
+    // azimuths an SM, run one after the other (16 x 16, 6 azimuths, own path / records:
+    // 2.2 blocks an SM 2.09 / 2.52 ms at 0.125 cm and 0.69 / 0.81 at 0.5; 3.8 blocks
+    // 2.10 / 2.62 and 1.05 / 0.85).  8 x 8 maps leave room for two blocks.  Blocks of
+    // whole beamlets are all long: only as many as run at once.
+    const uint64_t half_blocks = split ? (F == 8 ? 12 : (n_phi <= 4 ? 10 : 5)) : (F == 8 || n_phi <= 4 ? 4 : 2);  // per SM
+    const bool own_path = 2 * (uint64_t)blocks <= half_blocks * sm_count;
+    (own_path ? cccs_march_kernel<F, G, R, kMarchWarps, true>
+     : n_phi <= 4 ? cccs_march_kernel<F, G, R, 4, false>
+                  : cccs_march_kernel<F, G, R, kMarchWarps, false>)<<<blocks, 32 * n_phi, 0, st>>>(
+        d_beams, T, Rho, D, dirs, cp, split, planes, plane_stride, status, order);
     FD2_CHECK_CUDA(cudaGetLastError());
     return FD2_OK;
 }
@@ -1129,9 +1249,9 @@ struct Reach {
 // 16 take the voxel-stationary march (1..8 azimuth warps); other common sides
 // up to 24 the half-table instance and up to 32 the shared-column instance
 // (4..8 azimuth warps); anything else the general per-ray instance.
-int launch_march(int map, bool reach_ok, int maxP, int n_phi, unsigned blocks, cudaStream_t st, const fd2_beam_t* d_beams,
-                 const float* const* T, const float* const* R, float* const* D, const float4* dirs,
-                 const ConeParams& cp, int split, float* planes, size_t plane_stride, DeviceStatus* status,
+int launch_march(int map, bool reach_ok, int sm_count, int maxP, int n_phi, unsigned blocks, cudaStream_t st,
+                 const fd2_beam_t* d_beams, const float* const* T, const float* const* R, float* const* D,
+                 const float4* dirs, const ConeParams& cp, int split, float* planes, size_t plane_stride, DeviceStatus* status,
                  const int* order = nullptr) {
     const int threads = 32 * n_phi;
     const size_t shm = (size_t)(1 + n_phi) * maxP * sizeof(float2);
@@ -1139,13 +1259,13 @@ int launch_march(int map, bool reach_ok, int maxP, int n_phi, unsigned blocks, c
     if (reach_ok && n_phi <= kMarchWarps) {
         if (map == 16)
             return launch_voxel_march<16, 2, 8>(blocks, n_phi, st, d_beams, T, R, D, dirs, cp, split, planes,
-                                                plane_stride, status, order);
+                                                plane_stride, status, order, sm_count);
         if (map == 12)
             return launch_voxel_march<12, 2, 6>(blocks, n_phi, st, d_beams, T, R, D, dirs, cp, split, planes,
-                                                plane_stride, status, order);
+                                                plane_stride, status, order, sm_count);
         if (map == 8)
             return launch_voxel_march<8, 4, 2>(blocks, n_phi, st, d_beams, T, R, D, dirs, cp, split, planes,
-                                               plane_stride, status, order);
+                                               plane_stride, status, order, sm_count);
     }
     if (map > 0 && map <= 24 && warps_ok) {  // half-table instance: rays per lane = ceil(F^2 / 32)
         const int P = map * map;
@@ -1306,7 +1426,7 @@ int launch_cccs_host(fd2_context* ctx, size_t n_beams, const fd2_beam_t* h_beams
         FD2_TRY((launch_spread<8, true, false, 4>(blocks, cluster, k->n_phi, maxP, stream, d_beams, d_terma, d_dens, d_dose,
                                                   d_dirs, cp, d_planes, plane_stride, ctx->d_status, &taken)));
     if (!taken)
-        FD2_TRY(launch_march(map, form.reach, maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp,
+        FD2_TRY(launch_march(map, form.reach, ctx->sm_count, maxP, k->n_phi, blocks, stream, d_beams, d_terma, d_dens, d_dose, d_dirs, cp,
                              schedule, d_planes, plane_stride, ctx->d_status, schedule == 1 ? nullptr : d_order));
     ctx->launches += 2;  // direction table + march
     if (schedule == 1) {
@@ -1548,6 +1668,9 @@ extern "C" int fd2_dose_compute_static(size_t fmap_npixels, size_t n_beams, cons
     FD2_REQUIRE(maxP > 0 && maxP <= 1024, FD2_ERR_INVALID_ARGUMENT,
                 "dose_compute_static: fmap of %d pixels (1..1024)", maxP);
 
+    int device = 0, sm_count = 0;
+    FD2_CHECK_CUDA(cudaGetDevice(&device));
+    FD2_CHECK_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
     unsigned char* base = nullptr;
     FD2_TRY(static_scratch_address(&base));
     DeviceStatus* d_status = (DeviceStatus*)base;
@@ -1556,8 +1679,8 @@ extern "C" int fd2_dose_compute_static(size_t fmap_npixels, size_t n_beams, cons
     FD2_TRY(launch_cone_dirs(d_beams, n_beams, ang, d_dirs, st));
     const float* const* T = (const float* const*)d_terma;
     const float* const* R = (const float* const*)d_density_bev;
-    FD2_TRY(launch_march(map, reach.admits(), maxP, cp.n_phi, (unsigned)n_beams, st, d_beams, T, R, d_dose, d_dirs, cp, 0, nullptr, 0,
-                         d_status));
+    FD2_TRY(launch_march(map, reach.admits(), sm_count, maxP, cp.n_phi, (unsigned)n_beams, st, d_beams, T, R, d_dose,
+                         d_dirs, cp, 0, nullptr, 0, d_status));
     if (status_out)
         FD2_CHECK_CUDA(cudaMemcpyAsync(status_out, &d_status->code, sizeof(int), cudaMemcpyDefault, st));
     return FD2_OK;

@@ -74,6 +74,34 @@ def _reach(kern_src, b):
     return per, per * int(b.beams["long_dim"].max())
 
 
+@pytest.mark.parametrize("n_phi", [1, 4, 6, 8])
+@pytest.mark.parametrize("side,on,size", [(8, 2, 0.5), (8, 2, 0.1), (12, 4, 0.5), (12, 4, 0.2), (16, 4, 0.5), (16, 4, 0.2)])
+def test_march_of_few_and_of_many_beamlets(ctx, side, on, size, n_phi):
+    """Few blocks compute their paths warp by warp, many take them from one warp's
+    records; the zenith bins go to blocks of their own up to 4 beamlets an SM and
+    to one block above.  The same dose, bit for bit."""
+    import torch
+
+    ph = phantoms.torso_phantom(seed=side, dim=(48, 44, 40))
+    dens = api.Density(ctx, ph.density, ph.volume)
+    spec = api.Spectrum(ctx, phantoms.synthetic_spectrum())
+    kern = api.Kernel(ctx, phantoms.synthetic_kernel(n_theta=9, n_phi=n_phi))
+    few = _batch(ctx, ph, side, on, dens, spec, 0.7, count=3, beamlet_size=size)
+    n, total = len(few.beams), int(few.offsets[-1])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    doses = []
+    for copies in (1, 8 * sms // (9 * n) + 1, 4 * sms // n + 1):  # blocks an SM: under 1, 8, and 4 of whole beamlets
+        b = api.BEVBatch(np.concatenate([few.beams] * copies))
+        b.terma.copy_(few.terma.repeat(copies))
+        b.dens.copy_(few.dens.repeat(copies))
+        api.DoseComputeCollective(ctx, b, kern)
+        doses += [b.dose[:total].clone(), b.dose[-total:].clone()]
+    torch.cuda.synchronize()
+    assert float(doses[0].max()) > 0
+    for d in doses[1:]:
+        assert torch.equal(doses[0], d)
+
+
 # Coordinates of up to C voxels: a segment's lateral offset is the difference of two
 # products of that size, each of some three roundings, so a step's length is off by
 # 6 C 2^-24 voxels, and steps are half a voxel or longer on average
