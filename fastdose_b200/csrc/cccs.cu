@@ -1324,11 +1324,18 @@ int launch_spread(unsigned blocks, int cluster, int n_phi, size_t maxP, cudaStre
 }
 
 // Blocks per cluster of the spread march: the azimuths are divided evenly and
-// the clusters stay within two blocks an SM; 0 when it is not taken.
+// the clusters stay within two blocks an SM; 0 when it is not taken.  Blocks of 512
+// threads run one an SM, the rest of two in a second wave: that stays the faster
+// where a plain block has more rays a lane than registers for them (maps over 20:
+// 24 x 24, 8 azimuths, 18 beams 2.9 / 4.7 ms), below only while the second wave is
+// short (20 x 20, 0.3 cm: 13 beams 2.42 / 2.56 ms, 18 beams 2.79 / 2.55, 30 beams of
+// 4 bins 1.87 / 1.46; 0.1 cm: 13 beams 5.98 / 7.06, 18 beams 6.2 / 7.05).
 int spread_cluster(int map, int n_phi, unsigned blocks, int sm_count) {
     if (map < 17 || map > 32 || n_phi < 4 || n_phi > 8) return 0;
-    for (int c : {kMaxCluster, 2})
-        if (n_phi % c == 0 && blocks * (unsigned)c <= 2u * (unsigned)sm_count) return c;
+    for (int c : {kMaxCluster, 2}) {
+        const unsigned quarters = map <= 20 && 32 * 4 * (n_phi / c) > 384 ? 6 : 8;  // blocks per 4 SMs
+        if (n_phi % c == 0 && 4 * blocks * (unsigned)c <= quarters * (unsigned)sm_count) return c;
+    }
     return 0;
 }
 
