@@ -15,7 +15,8 @@ constexpr int kChunk = 256;           // nonzeros per SpMV chunk (32 lanes x 8)
 constexpr int kChunkWords = kChunk / 32;
 
 // Storage position of logical nonzero k.  A matrix of long rows whose x is
-// gathered from global memory is interleaved inside a chunk: logical element
+// gathered from global memory, or whose values are 16 bits and x is large, is
+// interleaved inside a chunk: logical element
 // 32 i + l is stored at 8 l + i, so that lane l's two 16-byte loads bring it
 // elements l, l + 32, ..., l + 224, and each of the warp's x-gathers covers 32
 // consecutive nonzeros of the row instead of 32 elements 8 apart.  In the other
@@ -85,7 +86,7 @@ struct fd2_matrix {
     bool interleaved = true;       // storage order inside a chunk (slot())
     int64_t* d_carry_row = nullptr;  // [n_ranges] row open at each range's end
     float* d_carry_val = nullptr;    // [n_ranges] its partial sum
-    float* d_xs = nullptr;           // [cols] x times the column scale
+    float* d_xs = nullptr;           // [cols] x times the column scale, where the product does not scale x itself
     int32_t* d_zrow = nullptr;       // rows the product itself does not write: empty, or only in carries
     int* d_nz = nullptr;             // number of those rows
     int n_zrows = 0;                 // and on the host

@@ -14,13 +14,14 @@
 //  * rows are found from a row-start bitmap (1 bit per nonzero) and a per-chunk
 //    count of row starts; a chunk without row starts is one FMA per lane and
 //    element into the open row;
-//  * storage order and summation come in two forms.  Where x is in shared
-//    memory, and for short rows, a lane's elements are consecutive: a chunk
-//    with row starts is summed per lane up to and after its row start, and one
-//    segmented warp scan over the lanes closes all its rows.  For long rows
-//    with x in global memory the chunk is interleaved (slot()), so that each
-//    x-gather of the warp covers 32 consecutive nonzeros, and the rare slices
-//    of 32 elements with row starts are scanned one by one;
+//  * storage order and summation come in two forms.  Mostly where x is in
+//    shared memory, and for short rows, a lane's elements are consecutive: a
+//    chunk with row starts is summed per lane up to and after its row start,
+//    and one segmented warp scan over the lanes closes all its rows.  For long
+//    rows with x in global memory (and with 16-bit values and a large x in
+//    shared memory) the chunk is interleaved (slot()), so that each x-gather of
+//    the warp covers 32 consecutive nonzeros, and the rare slices of 32 elements
+//    with row starts are scanned one by one;
 //  * the row open at the end of a range is carried; a second kernel adds the
 //    carries in range order.  The rows that no range closes are listed with the
 //    matrix and set to zero by the product itself.
@@ -52,6 +53,10 @@ constexpr int kSmemThreads = 1024;          // x-in-shared-memory variant: one b
 // with 8; long interleaved rows only lose prefetch (54 us with one, 58 with 4).
 constexpr int kRangesPerWarp = 4, kMinRange = 8;
 constexpr int64_t kSmemXMaxBytes = 200 * 1024, kSmemXSmall = 32 * 1024;
+// x of up to kSmemXScaled bytes is scaled as every SM copies it; a larger one by a
+// launch of its own, since reading the scales too doubles the copies (50k columns,
+// 8e6 nonzeros in 16 bits: 46 us scaled in the copies, 38 before them).
+constexpr int64_t kSmemXScaled = 64 * 1024;
 
 struct StreamArgs {
     const void* val;
@@ -668,16 +673,26 @@ __global__ void gather_transposed(const int64_t* __restrict__ off, int64_t rows,
 // The x-in-shared-memory instance of the stream kernel, allowed the largest x.
 template <typename T, bool kPacked>
 cudaError_t allow_smem_x() {
-    return cudaFuncSetAttribute(spmv_stream_kernel<T, kPacked, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kSmemXMaxBytes);
+    const cudaError_t e = cudaFuncSetAttribute(spmv_stream_kernel<T, kPacked, true, true>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemXMaxBytes);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(spmv_stream_kernel<T, kPacked, true, false>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemXMaxBytes);
+}
+
+// Whether the stream kernel scales x as it copies it to shared memory.
+bool scales_in_copy(const fd2_matrix* m) {
+    return m->x_in_smem && m->cols * (int64_t)sizeof(float) <= kSmemXScaled;
 }
 
 template <typename T, bool kPacked>
 int launch_stream_fmt(const fd2_matrix* m, const StreamArgs& a, const float* x, float* y, cudaStream_t st) {
     if (m->x_in_smem) {  // the shared-memory limit was raised when the matrix was finalized
         const unsigned blocks = (unsigned)(((int64_t)m->n_warps * 32 + kSmemThreads - 1) / kSmemThreads);
-        spmv_stream_kernel<T, kPacked, true, false>
-            <<<blocks, kSmemThreads, (size_t)m->cols * sizeof(float), st>>>(a, x, y);
+        if (m->interleaved)
+            spmv_stream_kernel<T, kPacked, true, true><<<blocks, kSmemThreads, (size_t)m->cols * sizeof(float), st>>>(a, x, y);
+        else
+            spmv_stream_kernel<T, kPacked, true, false><<<blocks, kSmemThreads, (size_t)m->cols * sizeof(float), st>>>(a, x, y);
     } else {
         const unsigned blocks = (unsigned)(((int64_t)m->n_warps * 32 + kStreamThreads - 1) / kStreamThreads);
         if (m->interleaved)
@@ -695,7 +710,7 @@ int launch_stream(const fd2_matrix* m, const float* x, float* y, cudaStream_t st
                  m->scale_axis == FD2_SCALE_ROWS ? m->d_scale : nullptr, m->n_chunks, m->n_warps,
                  m->n_ranges, m->rows,
                  m->d_carry_row, m->d_carry_val, (int)m->cols,
-                 m->scale_axis == FD2_SCALE_COLS && m->x_in_smem ? m->d_scale : nullptr, m->d_zrow, m->d_nz};
+                 m->scale_axis == FD2_SCALE_COLS && scales_in_copy(m) ? m->d_scale : nullptr, m->d_zrow, m->d_nz};
     if (m->index_format == FD2_INDEX_PACKED16)
         FD2_TRY((launch_stream_fmt<T, true>(m, a, x, y, st)));
     else
@@ -823,7 +838,12 @@ int resident_warps(fd2_matrix* m, int sm_count) {
                                                       (size_t)xb) == cudaSuccess &&
         per_sm >= 1) {
         m->x_in_smem = true;
-        m->interleaved = false;
+        // 16-bit values over a large x, where a product is short of issue slots for the
+        // gathers: the interleaved form spends fewer on a chunk without row starts.
+        // 4e7 nonzeros, 50k columns, lanes / interleaved: packed 300 a row 75.8 / 70.7
+        // us, 2000 66.6 / 64.3, but 100 78.9 / 85.0; int32 columns 100 a row 101 / 85,
+        // 2000 85 / 75.  Up to 16k columns the lanes are as fast (52 to 69 us).
+        m->interleaved = sizeof(T) == 2 && xb > kSmemXScaled && m->nnz >= (kPacked ? kChunk : kChunk * 3 / 8) * m->rows;
         return per_sm * sm_count * (kSmemThreads / 32);
     }
     cudaGetLastError();  // a refused attribute or query leaves the global-gather instance
@@ -866,7 +886,7 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     FD2_CHECK_CUDA(mat_malloc(&m->d_zrow, std::max<int64_t>(m->rows, 1) * sizeof(int32_t), st));
     FD2_CHECK_CUDA(mat_malloc(&m->d_nz, sizeof(int), st));
     FD2_CHECK_CUDA(cudaMemsetAsync(m->d_nz, 0, sizeof(int), st));
-    if (m->scale_axis == FD2_SCALE_COLS && !m->x_in_smem)
+    if (m->scale_axis == FD2_SCALE_COLS && !scales_in_copy(m))
         FD2_CHECK_CUDA(mat_malloc(&m->d_xs, std::max<int64_t>(m->cols, 1) * sizeof(float), st));
     FD2_CHECK_CUDA(cudaMemsetAsync(m->d_head, 0, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t),
                                    st));
@@ -992,7 +1012,7 @@ int matrix_spmv(const fd2_matrix* m, const float* x, float* y, cudaStream_t st) 
         FD2_CHECK_CUDA(cudaMemsetAsync(y, 0, m->rows * sizeof(float), st));
         return FD2_OK;
     }
-    if (m->scale_axis == FD2_SCALE_COLS && !m->x_in_smem) {
+    if (m->scale_axis == FD2_SCALE_COLS && !scales_in_copy(m)) {
         scale_vector_kernel<<<grid_for(m->cols), 256, 0, st>>>(m->d_scale, x, m->d_xs, m->cols);
         FD2_CHECK_CUDA(cudaGetLastError());
         x = m->d_xs;

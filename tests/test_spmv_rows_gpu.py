@@ -1,7 +1,9 @@
 """Products over rows of a constant length around the lane (8), slice (32) and
 chunk (256 nonzeros) sizes of the stream kernel, with runs of empty rows, in the
 forms a matrix is stored in: x in shared memory, and x in global memory with
-short rows (a lane's elements consecutive) or long ones (interleaved).
+short rows (a lane's elements consecutive) or long ones (interleaved).  A large x in
+shared memory (scaled by a launch of its own, and interleaved with 16-bit values and
+long rows) has a test of its own: it takes a matrix of more bytes than its copies.
 
 Tolerance: a row of n nonzeros is a sum in FP32 of n products in some order, so
 it is within (n + 2) 2^-24 of its |A||x| sum."""
@@ -52,6 +54,31 @@ def test_rows_of_one_length(ctx, cols, length):
         assert np.all(np.abs(yt - np.bincount(col, q, cols)) <= (n_col + 5) * 2.0 ** -24 * np.bincount(col, np.abs(q), cols))
         for a, b in zip(T.transpose().to_host(), (o, c, v)):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("per", [20, 95, 120, 255, 260, 900])
+@pytest.mark.parametrize("vt,fmt", [("f16", "packed16"), ("bf16", "i32"), ("f32", "packed16")])
+def test_large_x_in_shared_memory(ctx, vt, fmt, per):
+    import torch
+
+    rng = np.random.default_rng(per)
+    cols, rows = 20000, 3_200_000 // per
+    counts = np.minimum(rng.poisson(per, rows), cols)
+    counts[rng.random(rows) < 0.05] = 0
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    row = np.repeat(np.arange(rows), counts)
+    gap = (cols // (counts + 1))[row]  # one column in each of the row's gaps
+    col = (np.arange(off[-1]) - off[row]) * gap + rng.integers(0, 1 << 30, off[-1]) % gap
+    val = (rng.random(off[-1]) - 0.3).astype(np.float32)
+    M = optimize.Matrix.from_csr(ctx, off, col, val, cols, value_type=vt, index_format=fmt)
+    assert M.info()["x_in_shared"]
+    x = rng.standard_normal(cols).astype(np.float32)
+    _, c, v = M.to_host()
+    np.testing.assert_array_equal(c, col)
+    y = M.spmv(torch.from_numpy(x).cuda()).cpu().numpy()
+    p = v.astype(np.float64) * x[col]
+    assert np.all(np.abs(y - np.bincount(row, p, rows)) <= (counts + 4) * 2.0 ** -24 * np.bincount(row, np.abs(p), rows))
+    np.testing.assert_array_equal(M.spmv(torch.from_numpy(x).cuda()).cpu().numpy(), y)
 
 
 def test_device_bytes_count_the_rows_a_product_clears(ctx):
