@@ -88,8 +88,8 @@ struct fd2_matrix {
     float* d_carry_val = nullptr;    // [n_ranges] its partial sum
     float* d_xs = nullptr;           // [cols] x times the column scale, where the product does not scale x itself
     int32_t* d_zrow = nullptr;       // rows the product itself does not write: empty, or only in carries
-    int* d_nz = nullptr;             // number of those rows
-    int n_zrows = 0;                 // and on the host
+    int* d_nz = nullptr;             // [2] number of those rows, and n_nzrows
+    int n_zrows = 0;                 // the first on the host
 
     fd2::ColView cols_view() const { return fd2::ColView{d_col, d_col16, d_cbase, d_exc, interleaved}; }
 };

@@ -536,9 +536,12 @@ __global__ void pack_columns(const int32_t* __restrict__ col, int64_t nnz, int64
 
 // Rows that the product's ranges do not write: empty ones, and those that end
 // where a range does (the next row starts the next range, or the matrix ends),
-// whose sum is only in carries.  In any order: they are set to zero.
+// whose sum is only in carries.  In any order: they are set to zero.  count: their
+// number (zero before), and that of the rows with nonzeros, from their scan.
 __global__ void list_unwritten_rows(const int64_t* __restrict__ off, int64_t rows, int64_t nnz, int64_t n_chunks,
-                                    int64_t n_ranges, int32_t* __restrict__ zrow, int* __restrict__ count) {
+                                    int64_t n_ranges, const int32_t* __restrict__ ne, const int32_t* __restrict__ pos,
+                                    int32_t* __restrict__ zrow, int* __restrict__ count) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) count[1] = pos[rows - 1] + ne[rows - 1];
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
         const int64_t end = off[r + 1];
         bool un = off[r] == end || end == nnz;
@@ -884,8 +887,8 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     FD2_CHECK_CUDA(mat_malloc(&m->d_carry_row, m->n_ranges * sizeof(int64_t), st));
     FD2_CHECK_CUDA(mat_malloc(&m->d_carry_val, m->n_ranges * sizeof(float), st));
     FD2_CHECK_CUDA(mat_malloc(&m->d_zrow, std::max<int64_t>(m->rows, 1) * sizeof(int32_t), st));
-    FD2_CHECK_CUDA(mat_malloc(&m->d_nz, sizeof(int), st));
-    FD2_CHECK_CUDA(cudaMemsetAsync(m->d_nz, 0, sizeof(int), st));
+    FD2_CHECK_CUDA(mat_malloc(&m->d_nz, 2 * sizeof(int), st));
+    FD2_CHECK_CUDA(cudaMemsetAsync(m->d_nz, 0, 2 * sizeof(int), st));
     if (m->scale_axis == FD2_SCALE_COLS && !scales_in_copy(m))
         FD2_CHECK_CUDA(mat_malloc(&m->d_xs, std::max<int64_t>(m->cols, 1) * sizeof(float), st));
     FD2_CHECK_CUDA(cudaMemsetAsync(m->d_head, 0, std::max<int64_t>(m->n_chunks * kChunkWords, 1) * sizeof(uint32_t),
@@ -907,18 +910,18 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
     int rc = FD2_OK;
     if (m->rows) mark_row_starts<<<grid_for(m->rows), 256, 0, st>>>(m->d_off, m->rows, m->interleaved, m->d_head, ne);
     if (m->rows) rc = exclusive_scan(ne, pos, m->rows, st);
-    int32_t last_ne = 0, last_pos = 0;
-    if (!rc && m->rows) {
-        if (cudaMemcpy(&last_ne, ne + m->rows - 1, 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(&last_pos, pos + m->rows - 1, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+    int32_t counts[2] = {0, 0};
+    if (!rc && m->rows && m->n_chunks) {
+        list_unwritten_rows<<<grid_for(m->rows), 256, 0, st>>>(m->d_off, m->rows, m->nnz, m->n_chunks, m->n_ranges, ne, pos,
+                                                              m->d_zrow, m->d_nz);
+        if (cudaMemcpyAsync(counts, m->d_nz, sizeof(counts), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
             rc = FD2_ERR_CUDA;
     }
-    m->n_nzrows = (int64_t)last_pos + last_ne;
+    m->n_zrows = counts[0];
+    m->n_nzrows = counts[1];
     if (!rc && mat_malloc(&m->d_nzrow, std::max<int64_t>(m->n_nzrows, 1) * sizeof(int32_t), st) != cudaSuccess)
         rc = FD2_ERR_OUT_OF_MEMORY;
-    if (!rc && m->rows && m->n_chunks)
-        list_unwritten_rows<<<grid_for(m->rows), 256, 0, st>>>(m->d_off, m->rows, m->nnz, m->n_chunks, m->n_ranges, m->d_zrow,
-                                                              m->d_nz);
     if (!rc && m->rows) scatter_rows<<<grid_for(m->rows), 256, 0, st>>>(ne, pos, m->rows, m->d_nzrow);
     if (!rc && m->n_chunks) {
         chunk_head_counts<<<grid_for(m->n_chunks), 256, 0, st>>>(m->d_head, m->n_chunks, cnt);
@@ -998,8 +1001,6 @@ int matrix_finalize(fd2_matrix* m, cudaStream_t st) {
             }
         }
     }
-    if (!rc && cudaMemcpyAsync(&m->n_zrows, m->d_nz, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-        rc = FD2_ERR_CUDA;
     if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = FD2_ERR_CUDA;
     cleanup();
     if (rc && rc != FD2_ERR_OUT_OF_MEMORY) set_error("matrix_finalize: %s", cudaGetErrorString(cudaGetLastError()));
