@@ -179,13 +179,14 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// Block: n_phi warps (kWpa per azimuth of the block).  Dynamic shared memory: float2 tr[P] (Terma, density of
-// the current slice) followed by float2 dp[n_phi][P] (per-azimuth dose and path
-// sums).  RPL = rays per lane (P <= 32 * RPL).
-// kCols: every map of the batch is F x F with F <= 32 -- each lane owns one
-// column (lane % F) and the rows lane / F + k j (k = 32 / F lanes per column),
-// so the x half of the voxel work is done once per lane and the y half once per
-// row and shared by shuffles; RPL >= ceil(F / k).
+// Block: n_phi warps (kWpa per azimuth of the block).  Dynamic shared memory:
+// float2 tr[P] (Terma, density of the current slice) followed by float2
+// dp[n_phi][P] (per-azimuth dose and path sums).  RPL = rays per lane (P <= 32 * RPL).
+// kCols: every map of the batch is F x F with 25 <= F <= 32 -- lane l owns column
+// l, so the x half of the voxel work is done once per lane and the y half once per
+// row and shared by shuffles; RPL * kWpa >= F.  (With the arithmetic for several
+// lanes a column, of narrower maps, it spilled 300 bytes instead of 156: 30 beams of
+// 32 x 32, 8 azimuths 12.4 ms, 8.9 without.)
 //
 // kWpa > 1 spreads a (beamlet, zenith bin) that would leave most of the device
 // idle: kWpa warps share an azimuth's rays, RPL each, and the azimuths are
@@ -274,12 +275,9 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
             fiy[j] = (float)(r / g.fx);
         }
     }
-    // kCols: this lane's column and first row, the lanes per column, and the
-    // row whose y half this lane computes for the others
-    const int kgrp = kCols ? 32 / g.fx : 1;
-    const int ccol = kCols ? lane % g.fx : 0, cgrp = kCols ? lane / g.fx : 0;
-    const bool clane = kCols && lane < kgrp * g.fx;
-    const float fcol = (float)ccol, frow = (float)(kCols && lane < g.fy ? lane : 0);
+    // kCols: this lane's column, and the row whose y half it computes for the others
+    const bool clane = kCols && lane < g.fx;
+    const float fcol = clane ? (float)lane : 0.0f, frow = fcol;
 
     // The slice most likely to come next (s + 1, or slice 0 of the next zenith
     // pass), copied by cp.async into s_stage (Terma, then density) during the
@@ -339,9 +337,14 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
                         const float bty = __fadd_rn(c.y, frow), nty = __fadd_rn(np.y, frow);
                         const int ycode = mid_index(bty, nty, g.ffy, g.fy) | (crosses_edge(bty, nty, g.ffy) ? 64 : 0);
                         const float dyq = (nty - g.hy) * g.bsy * fe - (bty - g.hy) * g.bsy * fs;
+                        // kWpa: formed at every step, or the rows' numbers and predicates are
+                        // kept over the steps and spill (32 x 32, one beam of 8 azimuths 1.77
+                        // ms, 1.74 so)
+                        int y0 = 0;
+                        if constexpr (kWpa > 1) asm volatile("mov.b32 %0, %1;" : "=r"(y0) : "r"(sub * RPL));
 #pragma unroll
                         for (int j = 0; j < RPL; j++) {
-                            const int y = cgrp + kgrp * (kWpa > 1 ? sub * RPL + j : j);
+                            const int y = y0 + j;
                             const bool on = clane && y < g.fy;
                             const int yc = __shfl_sync(0xffffffffu, ycode, on ? y : 0);
                             const float dyp = __shfl_sync(0xffffffffu, dyq, on ? y : 0);
@@ -501,7 +504,7 @@ __global__ void __launch_bounds__(kWpa > 1 ? kSpreadThreads : (kCols || kTab ? k
                 last_sum_p = dp[(size_t)(n_phi - 1) * g.P + v].y;
                 const float val = sum / (last_sum_p + 1e-4f);
                 if (split)
-                    split_out[(size_t)(kWpa > 1 ? unit : (int)blockIdx.x) * split_stride + (size_t)s * g.P + v] = val;
+                    split_out[(size_t)blockIdx.x * split_stride + (size_t)s * g.P + v] = val;
                 else
                     // this block alone owns beam bi's dose and each (s, v) stays with
                     // one thread, so a fire-and-forget add gives D + val in pass order
