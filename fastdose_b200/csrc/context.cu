@@ -1,6 +1,7 @@
 // context.cu -- context, density, spectrum and CCCS-kernel handles.
 #include <cstring>
 #include <mutex>
+#include <unordered_set>
 
 #include "fd2_internal.cuh"
 
@@ -78,13 +79,32 @@ int matrix_pool(int device, cudaMemPool_t* out) {
     return device_pool(pools, device, 4ull << 30, "matrix", out);
 }
 
+static std::mutex plain_mu;
+static std::unordered_set<void*>& plain_blocks() {  // never destroyed: handles may be freed while the process ends
+    static auto* s = new std::unordered_set<void*>();
+    return *s;
+}
+void plain_block_add(void* p) {
+    std::lock_guard<std::mutex> lock(plain_mu);
+    plain_blocks().insert(p);
+}
+bool plain_block_remove(void* p) {
+    std::lock_guard<std::mutex> lock(plain_mu);
+    return plain_blocks().erase(p) != 0;
+}
+
 void device_free(int device, void* const* p, size_t n) {
     int cur = -1;
     cudaGetDevice(&cur);
     if (cur != device) cudaSetDevice(device);
     cudaDeviceSynchronize();
-    for (size_t i = 0; i < n; i++)
-        if (p[i]) cudaFreeAsync(p[i], cudaStreamLegacy);
+    for (size_t i = 0; i < n; i++) {
+        if (!p[i]) continue;
+        if (plain_block_remove(p[i]))
+            cudaFree(p[i]);
+        else
+            cudaFreeAsync(p[i], cudaStreamLegacy);
+    }
     cudaGetLastError();  // nothing a later launch check should see
     if (cur >= 0 && cur != device) cudaSetDevice(cur);
 }

@@ -164,11 +164,15 @@ inline int ctx_scratch(fd2_context* ctx, size_t bytes, cudaStream_t st, void** o
 constexpr int kMaxDevices = 64;
 int density_pool(int device, cudaMemPool_t* out);
 int matrix_pool(int device, cudaMemPool_t* out);  // optimizer matrices and problems
-// Like cudaFree, for memory of those pools that work on any stream may still
-// use and that may outlive its context: waits for `device`, whichever device is
-// current, and returns the n pointers (null ones are skipped) to their pool.  The
-// current device and the last error are left as they were found.
+// Like cudaFree, for memory of those pools (and the plain blocks below) that work
+// on any stream may still use and that may outlive its context: waits for
+// `device`, whichever device is current, and returns the n pointers (null ones are
+// skipped).  The current device and the last error are left as they were found.
 void device_free(int device, void* const* p, size_t n);
+// The blocks of the optimizer that are plain allocations: noted when made, and
+// true once when given back.
+void plain_block_add(void* p);
+bool plain_block_remove(void* p);
 int density_create_pooled(fd2_context* ctx, const float* host_density, const fd2_volume_t* volume,
                           fd2_density** out);
 

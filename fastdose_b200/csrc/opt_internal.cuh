@@ -102,7 +102,12 @@ namespace fd2 {
 // for the device, took most of the time of the orientation loop's phases.  The
 // pool keeps at most 4 GiB of freed memory (with 1 GiB, the transpose of 5e7
 // nonzeros gave its buffers back and took them again: 15 % of the build);
-// fd2_context_release empties it.
+// fd2_context_release empties it.  Blocks of kPlainBlock and more are plain
+// allocations: past what it keeps, a pool maps and unmaps 3 to 11 ms a GiB, where
+// cudaMalloc and cudaFree take 0.6 and 1.2.  Transpose of 2e8 nonzeros in 16 bits,
+// all from cudaMalloc / from the pool / as now: 24.6 / 98 / 22 ms, of 8e8 91 / 590 /
+// 84, of 5e7 10.1 / 2.7 / 3.8; the VOI matrices of 2.7e8: 0.11 / 0.6 to 1 / 0.10 s.
+constexpr size_t kPlainBlock = (size_t)512 << 20;
 cudaError_t mat_malloc_bytes(void** p, size_t bytes, cudaStream_t stream);
 template <typename T>
 cudaError_t mat_malloc(T** p, size_t bytes, cudaStream_t stream) {

@@ -775,11 +775,27 @@ cudaError_t mat_malloc_bytes(void** p, size_t bytes, cudaStream_t stream) {
     cudaError_t e = cudaGetDevice(&device);
     cudaMemPool_t pool = nullptr;
     if (e == cudaSuccess && matrix_pool(device, &pool) != FD2_OK) e = cudaErrorMemoryAllocation;
-    return e == cudaSuccess ? cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, stream) : e;
+    if (e != cudaSuccess) return e;
+    auto take = [&]() {
+        return bytes >= kPlainBlock ? cudaMalloc(p, bytes)
+                                    : cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, stream);
+    };
+    e = take();
+    if (e == cudaErrorMemoryAllocation) {  // what the pool keeps may be what is missing
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool, 0);
+        e = take();
+    }
+    if (e == cudaSuccess && bytes >= kPlainBlock) plain_block_add(*p);
+    return e;
 }
 
 void mat_free(void* p, cudaStream_t stream) {
-    if (p) cudaFreeAsync(p, stream);
+    if (!p) return;
+    if (plain_block_remove(p))
+        cudaFree(p);  // waits for the device
+    else
+        cudaFreeAsync(p, stream);
 }
 
 int matrix_alloc(fd2_matrix* m, cudaStream_t st) {

@@ -19,7 +19,7 @@ struct Block {
 std::map<void*, Block> blocks;
 std::map<cudaMemPool_t, int> pools;
 int current = 0, wrong_device = 0, not_waited = 0;
-int plain = 0, extended = 0, refuse = 0;
+int plain = 0, extended = 0, refuse = 0, plain_blocks = 0;
 cudaError_t last = cudaSuccess;
 }  // namespace
 
@@ -32,6 +32,7 @@ void fake_report(int* live, int* wrong, int* early, int* cur) {
     *cur = current;
 }
 
+int fake_plain_blocks() { return plain_blocks; }
 void fake_refuse(int on) { refuse = on; }
 void fake_launches(int* p, int* x) {
     *p = plain;
@@ -63,8 +64,16 @@ cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return *e = (cudaEvent_t)malloc(8), cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { return free(e), cudaSuccess; }
 
-cudaError_t cudaMalloc(void** p, size_t n) { return *p = calloc(1, n), cudaSuccess; }
-cudaError_t cudaFree(void* p) { return free(p), cudaSuccess; }
+// plain allocations of 64 MiB and more are counted with the pools' blocks
+cudaError_t cudaMalloc(void** p, size_t n) {
+    *p = calloc(1, n);
+    if (n >= (size_t)64 << 20) {
+        blocks[*p] = Block{current, false};
+        plain_blocks++;
+    }
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) { return blocks.erase(p), free(p), cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return *p = calloc(1, n), cudaSuccess; }
 cudaError_t cudaMallocHost(void** p, size_t n) { return *p = calloc(1, n), cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return free(p), cudaSuccess; }

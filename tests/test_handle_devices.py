@@ -3,7 +3,8 @@ stand-in for the CUDA runtime (fake_cudart.cpp).
 
 Matrices, problems and densities destroyed while another device is current:
 their memory goes back to its own device's pool, after a wait for that device,
-and the caller's device stays current.  And a device that refuses a cluster
+and the caller's device stays current.  Blocks of 512 MiB and more are plain
+allocations, given back as such.  And a device that refuses a cluster
 launch: the plain march is launched in its place."""
 import os
 import shutil
@@ -53,6 +54,9 @@ if kind == "density":
     handles.append((lib.fd2_density_destroy, h))
 else:
     ms = [matrix(5), matrix(7, 1)]
+    if kind == "large":  # its column scales and what finds them are blocks of 560 MB
+        ms.append(matrix(140_000_000, 1))
+        assert fake.fake_plain_blocks() >= 1, "a large block came from the pool"
     if kind == "problem":
         A, AT = matrix(0), matrix(0)
         f = (C.c_float * 1)()
@@ -120,7 +124,7 @@ def fake(tmp_path_factory):
 
 
 @pytest.mark.parametrize("own,now", [(0, 0), (0, 1), (1, 0)])
-@pytest.mark.parametrize("kind", ["matrix", "problem", "density"])
+@pytest.mark.parametrize("kind", ["matrix", "large", "problem", "density"])
 def test_handles_return_memory_to_their_own_device(fake, kind, own, now):
     env = dict(os.environ, LD_PRELOAD=fake, PYTHONPATH=ROOT)
     p = subprocess.run([sys.executable, "-c", CHILD, fake, kind, str(own), str(now)], env=env, cwd=ROOT,
