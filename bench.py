@@ -38,8 +38,8 @@ METRIC = "CCCS beamlets/s (dose-loading matrix, batched 4pi)"
 # From one ncu capture of the CCCS march on the 40-beam plan (6056 beamlets;
 # profiles/cccs_march_4pi_torso_40beams.md):
 # dram__bytes_read.sum + dram__bytes_write.sum, and smsp__inst_executed.sum
-CCCS_DRAM_BYTES_PER_BEAMLET = (28.421676e9 + 9.664041e9) / 6056
-CCCS_WARP_INST_PER_BEAMLET = 108.351843346e9 / 6056
+CCCS_DRAM_BYTES_PER_BEAMLET = (28.469368e9 + 9.680342e9) / 6056
+CCCS_WARP_INST_PER_BEAMLET = 109.818948260e9 / 6056
 UNIT = "beamlets/s"
 
 

@@ -475,8 +475,9 @@ int ensure_groups(fd2_opt_problem* p, int64_t n_groups) {
 // nonzeros a trial is a chain of short kernels, so their number counts: the
 // products are one launch each, every sum is finished by the last block of the
 // kernel that starts it, the gradient's parts are added where they are used, and
-// the D products run beside the A products.  20 steps on 48k x 1944 in 16 bits:
-// 3.8 ms with some 34 graph nodes a trial in a row, 2.5 ms with 14.
+// the D products run beside the A products.  20 steps on 48k x 1944 in 16 bits,
+// with the same products: 3.8 ms with some 34 graph nodes a trial in a row, 2.5 ms
+// with 14.
 int trial_enqueue(fd2_opt_problem* p, const fd2_opt_state_t* st, int64_t n_groups) {
     cudaStream_t s = p->ctx->stream;
     const int64_t n = p->n;
