@@ -108,10 +108,14 @@ __device__ __forceinline__ float3 bev_to_pvcs(float3 v, float th, float ph, floa
 // 12.4 ms; 24 beams of 20 x 20 (two blocks a map, the second half empty) 4.41 /
 // 4.81 / 4.15 / 4.13 ms; 8 beams of 24 x 24 2.23 / 2.47 / 2.22 / 2.14 ms; 12 beams
 // of 17 x 17 1.93 / 2.07 / 1.76 / 1.82 ms.
-// kThreads 64, for launches that leave SMs idle at 256: the rays spread over four
-// times the blocks, and without a register limit a slice's reads are in flight
-// together.  One slab beam 140 -> 113 us, four 32 x 32 fields 408 -> 307 us (324
-// with four texels at a time).
+// kThreads 64, for launches of up to 24 blocks of 256 an SM: the rays spread over
+// four times the blocks, which fill the SMs to the end, and without a register
+// limit a slice's reads are in flight together.  One slab beam 140 -> 113 us, four
+// 32 x 32 fields 408 -> 307 us (324 with four texels at a time); 1000 beams of 8 x 8
+// maps 1.4 times as fast as with 256, 600 of 16 x 16 1.3 times, 2500 1.05.  Above
+// that line the two are within 5 % of each other on repeated beams (3600 blocks of
+// 20 x 20: 256 by 2 %, 4000 of 8 x 8: 64 by 5 %), but the 100-beam plan of 16 x 16
+// maps takes 12.4 ms with 256 and 15.2 with 64.
 template <bool kSkipDark, int kThreads>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 6 : 4) terma_kernel(const fd2_beam_t* __restrict__ beams,
                                                     const float* const* __restrict__ fluence,
@@ -178,10 +182,9 @@ int launch_terma(fd2_context* ctx, size_t fmap_npixels, size_t n_beams, const fd
         sp.mu[e] = spectrum->mu[e];
     }
     const fd2_volume_t& v = density->vol;
-    // blocks per beam cover up to 1024 pixels (the reference's bound: one block per
-    // beam); fewer than two blocks of 256 an SM go out as blocks of 64
+    // blocks per beam cover up to 1024 pixels (the reference's bound: one block per beam)
     const size_t blocks256 = n_beams * ((fmap_npixels + 255) / 256);
-    const unsigned threads = blocks256 < 2 * (size_t)ctx->sm_count ? 64 : 256;
+    const unsigned threads = blocks256 < 24 * (size_t)ctx->sm_count ? 64 : 256;
     dim3 grid((unsigned)n_beams, (unsigned)((fmap_npixels + threads - 1) / threads)), block(threads);
     auto kernel = threads == 64 ? (fluence_skip ? terma_kernel<true, 64> : terma_kernel<false, 64>)
                                 : (fluence_skip ? terma_kernel<true, 256> : terma_kernel<false, 256>);

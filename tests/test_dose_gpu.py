@@ -52,6 +52,33 @@ def test_terma_matches_oracle(ctx, case_fn, idx):
         assert np.abs(R - Ro).max() <= 1e-4 * np.abs(Ro).max()
 
 
+@pytest.mark.parametrize("side,below", [(8, 1), (8, 0), (15, 0), (16, 0), (17, 1), (17, 0), (20, 0)])
+def test_terma_block_sizes_agree_bitwise(ctx, side, below):
+    """Launches of 24 and more blocks of 256 rays an SM keep blocks of 256; smaller
+    ones, the four beams alone among them, go out as blocks of 64.  A beam's rays are
+    the same arithmetic in both, so the bits do not depend on the launch: on both sides
+    of the line, with maps of less than, exactly and just over one block of 256."""
+    import torch
+
+    case = small_case()
+    dens, sp = _setup(ctx, case)[:2]
+    beams = case["beams"][[0, 5, 10, 15]].copy()
+    beams["fmap_size"] = side
+    for i in range(4):
+        beams[i] = api.calc_range(beams[i], case["phantom"].volume)
+    per_beam = (side * side + 255) // 256
+    n = -(-24 * torch.cuda.get_device_properties(0).multi_processor_count // per_beam) - below
+    fluence = np.random.default_rng(side).random((4, side * side), dtype=np.float32)
+    few, many = api.BEVBatch(beams), api.BEVBatch(beams[np.arange(n) % 4])
+    api.TermaComputeCollective(ctx, few, torch.from_numpy(fluence).cuda(), dens, sp)
+    api.TermaComputeCollective(ctx, many, torch.from_numpy(fluence[np.arange(n) % 4]).cuda(), dens, sp)
+    torch.cuda.synchronize()
+    for i in (0, 1, 2, 3, n - 4, n - 3, n - 2, n - 1):
+        assert few.get("terma", i % 4).max() > 0
+        for what in ("terma", "dens"):
+            assert torch.equal(many.get(what, i), few.get(what, i % 4))
+
+
 @pytest.mark.parametrize("case_fn,idx", [(small_case, [0, 5, 10, 15]), (c1_case, [0, 44, 93])])
 def test_cccs_matches_oracle(ctx, case_fn, idx):
     """The oracle marches with the device's cone directions; its boundary
